@@ -1,0 +1,103 @@
+"""FP16 stacks on the tensor cores (the FBP's default FP16 form and stacked-backproject's half mode):
+edges of the 11 x 20 pixel tiles, of the slice shares of a CTA, of the angle stages, and rows with
+non-finite values.
+
+Tolerance: filtered sinograms round to 11 bits (2^-12 relative) and weights to 2^-12; on random
+data, where neighbouring bins are independent, both add up to a few 1e-4 relative L2."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+import oracle
+import ufob
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-3
+
+
+def _raw(nz, P, W, seed):
+    return np.random.default_rng(seed).standard_normal((nz, P, W)).astype(np.float32)
+
+
+def _ref(raw, N, **bp):
+    nz, P, W = raw.shape
+    filt = oracle.fft_filter_ifft(raw.reshape(-1, W), size_x=N, crop_width=W).reshape(nz, P, W)
+    return np.stack([oracle.backproject(filt[z].astype(np.float32), **bp) for z in range(nz)])
+
+
+def _fbp(raw, N, **bp):
+    f = ufob.FBP(filter_props={"size_x": N, "crop_width": raw.shape[-1]}, bp_props=bp, storage=ufob.F16)
+    out = f.process(torch.from_numpy(raw).cuda()).cpu().numpy()
+    ufob.device_status()
+    return out
+
+
+# tiles: one pixel short of, at and past the 11-wide and 20-high tile; odd and tiny widths
+@pytest.mark.parametrize("W", [5, 10, 11, 12, 19, 20, 21, 45, 121])
+def test_tile_edges(cuda, W):
+    raw, N = _raw(17, 37, W, W), 1 << (W - 1).bit_length()
+    assert oracle.rel_l2(_fbp(raw, N), _ref(raw, N)) < TOL
+
+
+# slices: partly filled octets and 16-slice products, each share size and two shares
+@pytest.mark.parametrize("nz", [17, 23, 33, 64, 70, 96, 113, 128, 131, 200, 257])
+def test_slice_shares(cuda, nz):
+    raw = _raw(nz, 40, 60, nz)
+    got, ref = _fbp(raw, 64), _ref(raw, 64)
+    for z in (0, 7, nz // 2, nz - 1):
+        assert oracle.rel_l2(got[z], ref[z]) < TOL, z
+
+
+# angles: fewer than a stage, partly filled stages and groups of 32, for each stage length
+@pytest.mark.parametrize("nz", [20, 50, 120])
+@pytest.mark.parametrize("P", [1, 2, 3, 7, 9, 31, 33, 70])
+def test_angle_counts(cuda, nz, P):
+    raw = _raw(nz, P, 48, P)
+    assert oracle.rel_l2(_fbp(raw, 64), _ref(raw, 64)) < TOL
+
+
+def test_roi_axis_offset(cuda):
+    raw = _raw(18, 60, 100, 4)
+    bp = dict(axis_pos=43.3, angle_step=math.pi / 50, angle_offset=0.7, roi_x=70, roi_y=5, roi_width=61,
+              roi_height=90)  # part of the region sees no detector
+    assert oracle.rel_l2(_fbp(raw, 128, **bp), _ref(raw, 128, **bp)) < TOL
+
+
+@pytest.mark.parametrize("nz", [17, 45])
+def test_stacked_half(cuda, nz):
+    raw = _raw(nz, 50, 77, nz)
+    t = ufob.StackedBackprojectTask(precision_mode="half", axis_pos=36.5)
+    got = t.process(torch.from_numpy(raw).cuda()).cpu().numpy()
+    ref = np.stack([oracle.stacked_backproject(raw[z:z + 1], "single", axis_pos=36.5)[0] for z in range(nz)])
+    assert oracle.rel_l2(got, ref) < TOL
+
+
+# one infinite bin, FP16 overflow and a NaN row: only the pixels that interpolate them may change.
+# stacked-backproject takes the rows as they are, so the affected pixels are known exactly.
+@pytest.mark.parametrize("bad", [math.inf, -math.inf, math.nan, 1.0e6])
+def test_nonfinite_bins_stay_local(cuda, bad):
+    nz, P, W, axis = 20, 33, 90, 44.6
+    raw = _raw(nz, P, W, 9)
+    dirty = raw.copy()
+    hits = [(3, 5, 41), (3, 32, 0), (17, 11, W - 1)]
+    for z, p, j in hits:
+        dirty[z, p, j] = bad
+    t = ufob.StackedBackprojectTask(precision_mode="half", axis_pos=axis)
+    clean = t.process(torch.from_numpy(raw).cuda()).cpu().numpy()
+    got = t.process(torch.from_numpy(dirty).cuda()).cpu().numpy()
+    ufob.device_status()
+    x = np.arange(W) + 0.5 - np.float32(axis)
+    touched = np.zeros((nz, W, W), bool)
+    near = np.zeros((nz, W, W), bool)
+    for z, p, j in hits:
+        a = p * math.pi / P
+        h = x[None, :] * math.cos(a) - x[:, None] * math.sin(a) + np.float32(axis) - 0.5
+        touched[z] |= np.abs(h - j) < 0.999
+        near[z] |= np.abs(h - j) < 1.001
+    assert not np.isfinite(got[touched]).any()
+    assert np.isfinite(got[~near]).all()
+    # the flagged rows are sampled with FP32 weights, the others with 11-bit ones
+    assert oracle.rel_l2(got[~near], clean[~near]) < TOL

@@ -1,0 +1,533 @@
+// Parallel-beam backprojection of a stack on the 5th-gen tensor cores: FP16 filtered sinograms,
+// fixed-point interpolation weights, FP32 accumulation (the FP16 form of the FBP for stacks, and
+// stacked-backproject's half mode).  Same image as backproject.cu's kernels (src/kernels/
+// backproject.cl:50-94): slice[y][x] = pi / P * sum_p lerp(sino[p], h_p), zero outside the detector.
+//
+// For one angle, the interpolation of a few pixels that share a short detector window is a matrix
+// product: D[pixel][slice] += A[pixel][tap] * B[tap][slice], where a row of A holds 1 - f and f at
+// the pixel's two taps and zeros elsewhere, and B is the staged window.  11 x 10 pixels reach at
+// most 16 bins at any angle (projected diagonal sqrt(10^2 + 9^2) = 13.5), so the product has
+// K = 16, one tcgen05.mma of M = 128 (110 rows used) and N = all slices of the CTA.  7 of 8
+// products are with zeros, but the slice-quad kernel (backproject.cu) is bound by shared-memory
+// gathers and FP32 issue at 22.7 updates per clock and SM, where a product of 128 slices makes
+// 110 * 128 updates in 64 tensor-core clocks.
+//
+//   Sinograms: slice octets [ceil(nz/8)][P][W] of 16-byte cells, cell j = bin j of eight slices.
+//     A window is one TMA box of KW cells x 1 angle x ns/8 groups, which lies in shared memory as
+//     an N-major operand without swizzle (core matrix = 8 bins x 8 slices), readable from any
+//     first bin: the accumulators of a CTA take their own 16 bins of one staged window.
+//     (FP16 rows as a K-major operand: 64-byte TMA rows, 6.4 clocks each, 11.7 against 19.8 TGUPS
+//     for 128 slices with the first version of this kernel.)
+//   Weights: built by CUDA cores, a row of two accumulators per thread, and stored to tensor memory
+//     (tcgen05.st), where the product reads A.  (Scattered 4-byte stores to shared memory and A
+//     read from there bound the SM's shared memory: 440 of 481 clocks per angle.)  A row is
+//     hat(u - k) = max(min(1 + u - k, 1 + k - u), 0) for the taps k = 0..15 in fixed point with 11
+//     fractional bits, two taps per 32-bit word (a packed add-min-relu each).  The integers
+//     0..2048 read as FP16 are n * 2^-24 exactly (subnormals and the first normals), so the
+//     accumulators count in 2^-13 of the sum.  Errors of the weights are at most 2^-12 (the
+//     slice-quad kernel: 10 fractional bits).
+//   Accumulators: FP32 in tensor memory over all angles, MT * ns columns.
+//
+// Roles of a CTA: four builder warps, a producer warp (one TMA per angle), an MMA warp per
+// accumulator (the issuing lane's instructions, not the tensor pipe, limit one warp for both: 29
+// against 24 ms).  Stages of KA angles; SA stages of weights, SB of windows; a stage's products
+// arrive on one barrier that frees its weights and its windows.  What bounds it is the fixed cost
+// of a stage (barriers, issue latencies), so small CTAs (KA = 2, four per SM) run up to 32 slices
+// and larger stages (KA = 4, 8) the cases that leave room for fewer CTAs.  2048^2 x 1500 angles, ms per
+// pass: ns <= 32 15.5, 64 16.6, 96 24.2, 128 29.0 (13.0, 24.3, 25.0, 27.8 TGUPS; slice quads 6.6).
+//
+// A non-finite value of a window would reach every pixel of its tile (0 * inf), so the filter
+// flags the angles that hold one; their products are skipped and the epilogue adds them by direct
+// sampling, which touches the pixels whose taps they are.
+#include <cuda.h>
+#include <cuda_fp16.h>
+#include <cudaTypedefs.h>
+
+#include <algorithm>
+
+#include "tma.cuh"
+#include "ufob_internal.h"
+
+namespace ufob {
+
+namespace {
+
+constexpr int MX = 11, MY = 10;  // pixels of one accumulator
+constexpr int MT = 2;            // accumulators of a CTA, one above the other
+constexpr int KT = 16;           // taps of one product
+constexpr int KW = 28;           // staged bins: KT + 10 |sin| + 1, rounded up
+constexpr int SA = 2;            // stages of weights
+constexpr int kBuildWarps = 4;
+constexpr int kThreads = 32 * (kBuildWarps + 1 + MT);
+constexpr uint32_t kSkip = 0xffffffffu;
+constexpr int kErrUmmaTimeout = 0x1003;
+
+// KA angles per stage.
+template <int KA>
+struct UmmaShape {
+    static constexpr int SB = 16 / KA;  // stages of windows
+    static constexpr uint32_t kACols = SA * KA * MT * (KT / 2);  // tensor-memory columns of the weights
+    static constexpr uint32_t window_bytes(uint32_t ns) { return ns * KW * 2; }  // one angle, all slices
+    static constexpr uint32_t smem(uint32_t ns) { return SB * KA * window_bytes(ns) + 128; }
+};
+
+__device__ __forceinline__ void tmem_alloc(uint32_t *slot, uint32_t ncols)
+{
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(ncols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols)
+{
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+
+// Shared-memory matrix descriptor (version 1), no swizzle.
+__device__ __forceinline__ uint64_t desc_plain(uint32_t saddr, uint32_t lbo, uint32_t sbo)
+{
+    return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)((lbo >> 4) & 0x3FFF) << 16) |
+           ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | ((uint64_t)1 << 46);
+}
+
+// A from tensor memory, B from shared memory
+__device__ __forceinline__ void mma_f16(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t acc)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
+        "r"(a), "l"(b), "r"(idesc), "r"(acc)
+        : "memory");
+}
+
+__device__ __forceinline__ void mma_commit(uint64_t *bar)
+{
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+                 : "memory");
+}
+
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16])
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+        "%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr),
+                 "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+
+// Bounded wait that also gives up once another role raised the abort flag.
+__device__ __forceinline__ bool wait_or_abort(uint64_t *bar, uint32_t parity, volatile int *abort_flag)
+{
+    uint64_t t0 = 0;
+    for (uint32_t i = 1;; i++) {
+        if (mbar_try_wait(bar, parity)) return true;
+        if ((i & 255u) == 0) {
+            if (*abort_flag) return false;
+            const uint64_t t = global_timer_ns();
+            if (!t0) {
+                t0 = t;
+            } else if (t - t0 > kWaitLimitNs) {
+                *abort_flag = 1;
+                return false;
+            }
+        }
+    }
+}
+
+struct UmmaArgs {
+    uint32_t P, nz, ns;  // angles, slices, slices per CTA (multiple of 16)
+    uint32_t roi_x, roi_y, roi_w, roi_h;
+    float axis, norm;
+    const float2 *sincos;
+    const uint4 *sino;     // slice octets, for the flagged angles
+    uint32_t W, pitch;     // bins, cells per row
+    uint64_t group_pitch;  // cells per octet
+    const uint8_t *flags;  // [P] angles with a non-finite value in some slice
+    float *out;
+    int *err;
+    uint32_t tiles_x, tiles_y, tmem_cols;
+    uint32_t one;  // 1, not known to the compiler: keeps the weights' sums off the busier ALU pipe
+};
+
+// First detector bin reached by the accumulator centred at (cx, cy).  Every role computes it with
+// the same operations, so they agree to the bit.
+__device__ __forceinline__ int window_start(float cx, float cy, float2 sc, float axis)
+{
+    const float hc = fmaf(cy, sc.x, fmaf(cx, sc.y, axis));
+    const float ext = fmaf(0.5f * (MX - 1), fabsf(sc.y), __fmul_rn(0.5f * (MY - 1), fabsf(sc.x)));
+    float e = floorf(__fsub_rn(__fsub_rn(hc, ext), 0.51f));
+    e = fminf(fmaxf(e, -16777216.f), 16777216.f);
+    return (int)e;
+}
+
+// v[0..15] += samples of the flagged angles at one pixel, slices z .. z + 15 (not weighted by norm)
+__device__ __noinline__ void add_flagged(const UmmaArgs &a, float bx, float by, uint32_t z, float (&v)[16])
+{
+    for (uint32_t p = 0; p < a.P; p++) {
+        if (!__ldg(a.flags + p)) continue;
+        const float2 sc = __ldg(&a.sincos[p]);
+        const float h = fmaf(by, sc.x, fmaf(bx, sc.y, a.axis)) - 0.5f;
+        const float e = floorf(h), f = h - e;
+        if (!(e >= -1.0f && e < (float)a.W)) continue;
+        const int j = (int)e;
+        for (uint32_t q = 0; q < 2; q++) {
+            const uint32_t g = z / 8 + q;
+            if (g * 8 >= a.nz) break;
+            const uint4 *row = a.sino + (size_t)g * a.group_pitch + (size_t)p * a.pitch;
+            const uint4 zero = make_uint4(0, 0, 0, 0);
+            const uint4 lo = j >= 0 ? __ldg(row + j) : zero, hi = j + 1 < (int)a.W ? __ldg(row + j + 1) : zero;
+            const uint32_t l[4] = {lo.x, lo.y, lo.z, lo.w}, u[4] = {hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float2 s0 = __half22float2(*reinterpret_cast<const __half2 *>(&l[i]));
+                const float2 s1 = __half22float2(*reinterpret_cast<const __half2 *>(&u[i]));
+                v[8 * q + 2 * i] += (1.0f - f) * s0.x + f * s1.x;
+                v[8 * q + 2 * i + 1] += (1.0f - f) * s0.y + f * s1.y;
+            }
+        }
+    }
+}
+
+template <int KA>
+__global__ void __launch_bounds__(kThreads, KA <= 2 ? 4 : 2)
+    k_bp_umma(const __grid_constant__ CUtensorMap map, const __grid_constant__ UmmaArgs args)
+{
+    using Sh = UmmaShape<KA>;
+    constexpr int SB = Sh::SB;
+    static_assert(32 % KA == 0 && SB >= SA, "whole stages per 32 angles; one barrier ring serves both slots");
+    extern __shared__ unsigned char smem_dyn[];
+    __shared__ uint64_t full_a[SA], full_b[SB], empty[SB], done;
+    __shared__ float4 s_tab[kBuildWarps][32];
+    __shared__ int s_win[32];
+    __shared__ uint32_t s_off[MT][32];
+    __shared__ uint32_t tslot;
+    __shared__ int s_abort, s_flagged, s_live;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t bbytes = Sh::window_bytes(args.ns);
+    const uint32_t base = (smem_u32(smem_dyn) + 127u) & ~127u;
+    unsigned char *gbase = smem_dyn + (base - smem_u32(smem_dyn));
+
+    // tiles in bands about 200 pixels wide, walked top to bottom: the CTAs resident at one time
+    // cover a compact region, whose windows the L2 serves to all of them
+    constexpr uint32_t GW = 18;
+    const uint32_t id = blockIdx.x, band_tiles = GW * args.tiles_y;
+    const uint32_t band = id / band_tiles, rr = id - band * band_tiles;
+    const uint32_t bw = min(GW, args.tiles_x - band * GW);
+    const int x0 = (int)(band * GW + rr % bw) * MX, y0 = (int)(rr / bw) * (MT * MY);
+    const uint32_t z0 = blockIdx.y * args.ns;
+
+    if (warp == kBuildWarps) tmem_alloc(&tslot, args.tmem_cols);
+    if (tid == 0) {
+        for (int s = 0; s < SA; s++) mbar_init(&full_a[s], kBuildWarps);
+        for (int s = 0; s < SB; s++) {
+            mbar_init(&full_b[s], 1);
+            mbar_init(&empty[s], MT);
+        }
+        mbar_init(&done, MT);
+        s_abort = s_flagged = s_live = 0;
+        fence_barrier_init();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tslot;
+    volatile int *abort_flag = &s_abort;
+
+    const uint32_t P = args.P;
+    const float axis = args.axis;
+    // centre of the upper accumulator
+    const float cx = (float)(args.roi_x + x0) - axis + 0.5f + 0.5f * (MX - 1);
+    const float cy = (float)(args.roi_y + y0) - axis + 0.5f + 0.5f * (MY - 1);
+    // row of both accumulators of a builder thread and its pixel in the upper one (rows past
+    // MX * MY repeat pixel 0 and are not stored)
+    const int row = (warp & 3) * 32 + lane;
+    const int pix = row < MX * MY ? row : 0;
+    const int px = x0 + pix % MX, py = y0 + pix / MX;
+    const float bx = (float)(args.roi_x + px) - axis + 0.5f;
+    const float by = (float)(args.roi_y + py) - axis + 0.5f;
+
+    if (warp < kBuildWarps) {
+        const float kFix = 6144.0f;  // 1.5 * 2^12: 11 fractional bits left in the mantissa
+        const uint32_t ta = tmem + MT * args.ns + ((uint32_t)warp << 21);
+        const uint32_t one = args.one;
+        float4 *tab = s_tab[warp];
+        bool ok = true;
+        for (uint32_t p0 = 0; p0 < P && ok; p0 += 32) {
+            {
+                const float2 sc = __ldg(&args.sincos[min(p0 + lane, P - 1)]);
+                __syncwarp();
+                tab[lane] = make_float4(sc.x, sc.y, axis - 0.5f - (float)window_start(cx, cy, sc, axis),
+                                        axis - 0.5f - (float)window_start(cx, cy + MY, sc, axis));
+                __syncwarp();
+            }
+            const uint32_t n = min(32u, P - p0);
+            for (uint32_t j = 0; j < n; j += KA) {
+                const uint32_t it = (p0 + j) / KA, s = it % SA;
+                // slot s is free when the products of stage it - SA are done
+                ok = it < SA || wait_or_abort(&empty[(it - SA) % SB], ((it - SA) / SB) & 1u, abort_flag);
+                if (!__all_sync(0xffffffffu, ok)) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+#pragma unroll
+                for (int a = 0; a < KA; a++) {
+                    const float4 t = tab[(j + a) & 31];
+#pragma unroll
+                    for (int h = 0; h < MT; h++) {
+                        // tap coordinate, then +-u in units of 2^-11 in both 16-bit halves
+                        const float u = fmaf(by + (float)(h * MY), t.x, fmaf(bx, t.y, h ? t.w : t.z));
+                        const uint32_t up = __float_as_uint(kFix + u), un = __float_as_uint(kFix - u);
+                        const uint32_t up2 = __byte_perm(up, up, 0x1010), un2 = __byte_perm(un, un, 0x1010);
+                        uint32_t w[KT / 2];
+#pragma unroll
+                        for (int k = 0; k < KT / 2; k++) {
+                            // taps 2k and 2k + 1.  The second operand is one 32-bit sum: its lower
+                            // half carries into the upper one only where it is not negative
+                            // (u <= 2k + 1), where the upper half is not the smaller operand
+                            constexpr uint32_t c1 = 2048u;
+                            const uint32_t lo = ((c1 - (2 * k) * c1) & 0xffffu) | ((c1 - (2 * k + 1) * c1) << 16);
+                            const uint32_t hi = (c1 + (2 * k) * c1) + ((c1 + (2 * k + 1) * c1) << 16);
+                            w[k] = __viaddmin_s16x2_relu(up2, lo, un2 * one + hi);
+                        }
+                        tmem_st8(ta + ((s * KA + a) * MT + h) * (KT / 2), w);
+                    }
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full_a[s]);
+            }
+        }
+    } else {
+        const bool produce = warp == kBuildWarps;
+        const int m = warp - kBuildWarps - 1;  // accumulator of an MMA warp
+        // D = F32, A = B = F16, B N-major
+        const uint32_t idesc = (1u << 4) | (1u << 16) | ((args.ns >> 3) << 17) | ((128u >> 4) << 24);
+        const uint64_t desc0 = desc_plain(base, 128, KW * 16);
+        const uint32_t dcol = tmem + (uint32_t)m * args.ns;
+        const uint32_t acol = tmem + MT * args.ns + (uint32_t)m * (KT / 2);
+        uint32_t acc = 0;
+        bool ok = true, skips = false;
+        for (uint32_t p0 = 0; p0 < P; p0 += 32) {
+            {
+                // windows of the next 32 angles, and where in them the accumulators' taps start
+                const uint32_t p = min(p0 + lane, P - 1);
+                const float2 sc = __ldg(&args.sincos[p]);
+                const int w0 = window_start(cx, cy, sc, axis), w1 = window_start(cx, cy + MY, sc, axis);
+                const int wm = min(w0, w1);
+                const bool skip = !produce && __ldg(args.flags + p) != 0;
+                __syncwarp();
+                if (produce) {
+                    s_win[lane] = wm;
+                } else {
+                    s_off[m][lane] = skip ? kSkip : (uint32_t)min((m ? w1 : w0) - wm, KW - KT);
+                    if (skip) s_flagged = 1;
+                }
+                skips = __any_sync(0xffffffffu, skip);
+            }
+            const uint32_t n = min(32u, P - p0);
+            if (lane == 0) {
+                for (uint32_t j = 0; j < n; j += KA) {
+                    const uint32_t it = (p0 + j) / KA, sb = it % SB, sa = it % SA;
+                    const uint32_t nval = min((uint32_t)KA, n - j);
+                    if (produce) {
+                        ok = it < SB || wait_or_abort(&empty[sb], ((it / SB) - 1) & 1u, abort_flag);
+                        if (!ok) break;
+                        mbar_arrive_expect_tx(&full_b[sb], nval * bbytes);
+#pragma unroll
+                        for (uint32_t a = 0; a < KA; a++)
+                            if (a < nval)
+                                tma_load_3d(gbase + (sb * KA + a) * bbytes, &map, &full_b[sb], s_win[j + a] * 8,
+                                            (int)(p0 + j + a), (int)(z0 / 8));
+                    } else {
+                        uint32_t off[KA];
+#pragma unroll
+                        for (int a = 0; a < KA; a++) off[a] = s_off[m][j + a];
+                        ok = wait_or_abort(&full_b[sb], (it / SB) & 1u, abort_flag) &&
+                             wait_or_abort(&full_a[sa], (it / SA) & 1u, abort_flag);
+                        if (!ok) break;
+                        tc_fence_after();
+                        if (!skips && nval == KA) {
+#pragma unroll
+                            for (int a = 0; a < KA; a++)
+                                mma_f16(dcol, acol + (sa * KA + a) * (MT * (KT / 2)),
+                                        desc0 + (uint64_t)((sb * KA + a) * (bbytes >> 4) + off[a]), idesc,
+                                        a > 0 ? 1u : acc);
+                            acc = 1;
+                        } else {
+#pragma unroll 1
+                            for (uint32_t a = 0; a < nval; a++) {
+                                const uint32_t o = s_off[m][j + a];
+                                if (o == kSkip) continue;
+                                mma_f16(dcol, acol + (sa * KA + a) * (MT * (KT / 2)),
+                                        desc0 + (uint64_t)((sb * KA + a) * (bbytes >> 4) + o), idesc, acc);
+                                acc = 1;
+                            }
+                        }
+                        mma_commit(&empty[sb]);
+                    }
+                }
+            }
+            ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+            if (!ok) break;
+        }
+        if (!produce && lane == 0) {
+            if (m == 0) s_live = (int)acc;  // read after the CTA barrier below
+            mma_commit(&done);
+        }
+    }
+    __syncwarp();
+    bool ok = true;
+    if (warp < kBuildWarps) ok = wait_or_abort(&done, 0, abort_flag);
+    __syncthreads();
+    if (warp < kBuildWarps) {
+        // results: a pixel of each accumulator per thread, slices along its columns
+        tc_fence_after();
+        if (__all_sync(0xffffffffu, ok)) {
+            const size_t plane = (size_t)args.roi_w * args.roi_h;
+            const bool live = s_live != 0, flagged = s_flagged != 0;
+            const uint32_t nz = min(args.ns, args.nz - z0);
+            for (int h = 0; h < MT; h++) {
+                const int y = py + h * MY;
+                const bool in = row < MX * MY && px < (int)args.roi_w && y < (int)args.roi_h;
+                const uint32_t taddr = tmem + (uint32_t)h * args.ns + ((uint32_t)warp << 21);
+                float *o = args.out + (size_t)z0 * plane + (size_t)y * args.roi_w + px;
+                for (uint32_t c = 0; c < nz; c += 16) {
+                    uint32_t r[16];
+                    float v[16];
+                    tmem_ld16(taddr + c, r);
+#pragma unroll
+                    for (int i = 0; i < 16; i++) v[i] = live ? __uint_as_float(r[i]) * 8192.0f : 0.0f;
+                    if (flagged && in) add_flagged(args, bx, by + (float)(h * MY), z0 + c, v);
+                    if (in) {
+#pragma unroll
+                        for (int i = 0; i < 16; i++)
+                            if (c + i < nz) o[(size_t)(c + i) * plane] = v[i] * args.norm;
+                    }
+                }
+            }
+        }
+        tc_fence_before();
+    }
+    __syncthreads();
+    if (s_abort && tid == 0) {
+        atomicExch(args.err, kErrUmmaTimeout);
+        // copies and products in flight end before the CTA's shared memory and accumulators go
+        for (int s = 0; s < SB; s++)
+            for (int k = 0; k < 2; k++) mbar_wait_bounded(&full_b[s], (uint32_t)k, kWaitLimitNs / 8);
+        mbar_wait_bounded(&done, 0, kWaitLimitNs / 8);
+    }
+    __syncthreads();
+    if (warp == kBuildWarps) tmem_dealloc(tmem, args.tmem_cols);
+}
+
+// Map over the slice octets [groups][P][W] of 16-byte cells; box = KW cells x 1 angle x box_groups.
+ufob_status make_octet_map(CUtensorMap *map, const void *base, uint32_t W, uint32_t P, uint32_t groups,
+                           uint32_t pitch, uint64_t group_pitch, uint32_t box_groups)
+{
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+        return fail(UFOB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+    auto fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
+    cuuint64_t dims[3] = {(cuuint64_t)W * 8, P, groups};
+    cuuint64_t strides[2] = {(cuuint64_t)pitch * 16, (cuuint64_t)group_pitch * 16};
+    cuuint32_t box[3] = {KW * 8, 1, box_groups};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void *>(base), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS)
+        return fail(UFOB_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d): cells=%u P=%u groups=%u pitch=%u box=%u",
+                    (int)r, W, P, groups, pitch, box_groups);
+    return UFOB_OK;
+}
+
+template <int KA>
+ufob_status launch(const CUtensorMap &map, UmmaArgs a, cudaStream_t stream)
+{
+    a.tmem_cols = 32;
+    while (a.tmem_cols < MT * a.ns + UmmaShape<KA>::kACols) a.tmem_cols *= 2;
+    static std::atomic<uint64_t> attr_devs{0};
+    UFOB_CUDA_TRY(smem_limit_per_device(k_bp_umma<KA>, (int)UmmaShape<KA>::smem(128), attr_devs));
+    dim3 grid(a.tiles_x * a.tiles_y, (a.nz + a.ns - 1) / a.ns);
+    k_bp_umma<KA><<<grid, kThreads, UmmaShape<KA>::smem(a.ns), stream>>>(map, a);
+    UFOB_CUDA_TRY(cudaGetLastError());
+    note_launch();
+    return UFOB_OK;
+}
+
+}  // namespace
+
+uint32_t bp_umma_slices(uint32_t nz)
+{
+    // Time of one pass over a tile by slices per CTA (ms at 2048^2 x 1500 angles, see above): equal
+    // shares of the stack that take the least in all.
+    static const struct {
+        uint32_t ns;
+        float ms;
+    } kPass[] = {{32, 15.5f}, {64, 16.6f}, {96, 24.2f}, {128, 29.0f}};
+    uint32_t best = 128;
+    float best_t = 1e30f;
+    for (uint32_t chunks = (nz + 127) / 128; chunks <= (nz + 31) / 32; chunks++) {
+        const uint32_t ns = round_up((nz + chunks - 1) / chunks, 16);
+        float ms = kPass[3].ms;
+        for (int i = 3; i >= 0; i--)
+            if (ns <= kPass[i].ns) ms = kPass[i].ms;
+        if (chunks * ms < best_t) {
+            best_t = chunks * ms;
+            best = ns;
+        }
+    }
+    return best;
+}
+
+ufob_status bp_umma_launch(const BPGeometry &g, const void *d_sino, uint32_t pitch, uint64_t group_pitch,
+                           const uint8_t *d_flags, float *d_out, cudaStream_t stream)
+{
+    if (!g.roi_w || !g.roi_h || !g.nz || !g.P) return UFOB_OK;
+    if ((uintptr_t)d_sino & 15) return fail(UFOB_ERR_INVALID, "backproject: slice-octet base must be 16-byte aligned");
+    UmmaArgs a;
+    a.P = g.P;
+    a.nz = g.nz;
+    a.ns = bp_umma_slices(g.nz);
+    a.roi_x = g.roi_x;
+    a.roi_y = g.roi_y;
+    a.roi_w = g.roi_w;
+    a.roi_h = g.roi_h;
+    a.axis = g.axis;
+    a.norm = g.norm;
+    a.sincos = g.d_sincos;
+    a.sino = reinterpret_cast<const uint4 *>(d_sino);
+    a.W = g.W;
+    a.pitch = pitch;
+    a.group_pitch = group_pitch;
+    a.flags = d_flags;
+    a.out = d_out;
+    a.err = device_error_word();
+    a.one = 1;
+    a.tiles_x = (g.roi_w + MX - 1) / MX;
+    a.tiles_y = (g.roi_h + MT * MY - 1) / (MT * MY);
+    CUtensorMap map;
+    UFOB_TRY(make_octet_map(&map, d_sino, g.W, g.P, (g.nz + 7) / 8, pitch, group_pitch, a.ns / 8));
+    // angles per stage by what the accumulators leave of the 512 tensor-memory columns
+    if (a.ns <= 32 || (a.ns > 64 && a.ns <= 96)) return launch<2>(map, a, stream);
+    if (a.ns <= 64) return launch<4>(map, a, stream);
+    return launch<8>(map, a, stream);
+}
+
+}  // namespace ufob

@@ -531,6 +531,18 @@ static ufob_status bp_prepare(ufob_backproject *bp, uint32_t width, uint32_t hei
     return UFOB_OK;
 }
 
+// Whether a stack of FP16 sinograms runs on the tensor cores: the default form of the linear mode
+// (no compensated or half sums, no pinned tile), and enough slices.  A pass takes the same time for
+// any number of slices up to 32 (its weights): 15.5 ms at 2048^2 x 1500, against 7.3 / 10.7 / 15.7 /
+// 30 ms of the slice-quad kernel for up to 4 / 8 / 16 / 32 slices (721 x 1001^2: 2.09 against 1.92 for
+// 16), so it starts where that kernel would take its 32-slice tile.
+static constexpr uint32_t kUmmaMinSlices = 17;
+
+static bool umma_applies(const ufob_bp_props &p, uint32_t nz)
+{
+    return nz >= kUmmaMinSlices && p.mode != UFOB_BP_NEAREST && p.tile < 0 && !p.half_sums && p.compensated <= 0;
+}
+
 // Compensated block sums only on request: with 16-bit sinogram storage the storage rounding
 // (2^-11 relative for FP16) bounds the error, and FP32 sums over 32-angle blocks add orders of
 // magnitude less (2048^2 x 1500 with FP16 cells: the same relative L2 against FP64 to seven
@@ -660,6 +672,7 @@ struct ufob_fbp {
     ufob_backproject *bp = nullptr;
     ufob_dtype storage = UFOB_F32;
     DevBuf work;        // filtered sinograms of one slice group
+    DevBuf flags;       // its angles with a non-finite value (slice octets)
     DevBuf hin[2];      // device staging of host input chunks
     DevBuf hout[2];     // device staging of host output chunks
     cudaStream_t s_copy = nullptr, s_comp = nullptr, s_d2h = nullptr;  // uploads, compute, downloads
@@ -726,7 +739,7 @@ extern "C" ufob_status ufob_fbp_get_requisition(ufob_fbp *x, uint32_t width, uin
 struct ufob_stacked_bp {
     ufob_backproject *bp = nullptr;  // mirrored sine table
     int precision = 2;               // 0 int8, 1 half, 2 single (src/ufo-stacked-backproject-task.c:705-716)
-    DevBuf work, keys;
+    DevBuf work, keys, flags;
 };
 
 extern "C" ufob_status ufob_stacked_bp_create(ufob_stacked_bp **out)
@@ -788,7 +801,16 @@ extern "C" ufob_status ufob_stacked_bp_run(ufob_stacked_bp *sb, const float *d_s
     if (sb->precision == 2)  // single: FP32 rows, linear interpolation
         return ufob_backproject_run(sb->bp, d_sino, UFOB_F32, UFOB_LAYOUT_ROWS, width, height, nslices, 0, 0, d_out,
                                     stream);
-    if (sb->precision == 1) {  // half: FP16 slice-quad cells, FP32 sums
+    if (sb->precision == 1 && umma_applies(sb->bp->props, nslices)) {  // half: FP16 slice octets, FP32 sums
+        BPGeometry g;
+        UFOB_TRY(bp_prepare(sb->bp, width, height, nslices, g, s));
+        UFOB_TRY(sb->work.ensure((size_t)((nslices + 7) / 8) * height * width * 16));
+        UFOB_TRY(sb->flags.ensure(height));
+        UFOB_CUDA_TRY(cudaMemsetAsync(sb->flags.ptr, 0, height, s));
+        UFOB_TRY(pack_octs_launch(d_sino, width, height, nslices, sb->work.ptr, sb->flags.as<uint8_t>(), s));
+        return bp_umma_launch(g, sb->work.ptr, width, (uint64_t)width * height, sb->flags.as<uint8_t>(), d_out, s);
+    }
+    if (sb->precision == 1) {  // few slices: FP16 slice-quad cells, FP32 sums
         const uint32_t cells = width + 1;
         UFOB_TRY(sb->work.ensure((size_t)((nslices + 3) / 4) * height * cells * 16));
         UFOB_TRY(pack_quads_launch(d_sino, width, height, nslices, sb->work.ptr, s));
@@ -817,13 +839,17 @@ static ufob_status fbp_group(ufob_fbp *x, const RowSource &src, uint32_t width, 
     uint32_t nfft, fw;
     UFOB_TRY(filter_sizes(x->f->props, width, &nfft, &fw));
     UFOB_TRY(filter_plan_build(x->f->props, nfft, x->f->plan, s));
-    // F16: slice-quad cells (16 B per detector position and four slices), or pairs for a single
+    // F16: slice octets for the tensor cores (16 B per detector position and eight slices) or, for
+    // few slices, slice-quad cells (16 B per detector position and four slices), or pairs for a single
     // slice (a quad cell would carry three empty slices); BF16: pairs; F32: rows
-    const bool quads = x->storage == UFOB_F16 && nz > 1;
+    const bool umma = x->storage == UFOB_F16 && umma_applies(x->bp->props, nz);
+    const bool quads = x->storage == UFOB_F16 && nz > 1 && !umma;
     const bool pairs = x->storage == UFOB_BF16 || (x->storage == UFOB_F16 && nz == 1);
-    const uint32_t pitch = quads ? fw + 1 : pairs ? round_up(fw + 1, 4) : round_up(fw, 4);
-    const size_t work_bytes = quads ? (size_t)pitch * 16 * height * ((nz + 3) / 4) : (size_t)pitch * 4 * height * nz;
+    const uint32_t pitch = umma ? fw : quads ? fw + 1 : pairs ? round_up(fw + 1, 4) : round_up(fw, 4);
+    const size_t work_bytes = umma    ? (size_t)pitch * 16 * height * ((nz + 7) / 8)
+                              : quads ? (size_t)pitch * 16 * height * ((nz + 3) / 4) : (size_t)pitch * 4 * height * nz;
     UFOB_TRY(x->work.ensure(work_bytes));
+    if (umma) UFOB_TRY(x->flags.ensure(height));
     cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr;
     if (x->timing) {
         e0 = x->next_event();
@@ -833,14 +859,24 @@ static ufob_status fbp_group(ufob_fbp *x, const RowSource &src, uint32_t width, 
         UFOB_CUDA_TRY(cudaEventRecord(e0, s));
     }
     const ufob_layout layout = quads ? UFOB_LAYOUT_QUADS : pairs ? UFOB_LAYOUT_PAIRS : UFOB_LAYOUT_ROWS;
-    if (quads)
+    if (umma) {
+        UFOB_CUDA_TRY(cudaMemsetAsync(x->flags.ptr, 0, height, s));
+        UFOB_TRY(filter_octs_launch_src(x->f->plan, src, width, height, nz, x->work.ptr, x->flags.as<uint8_t>(), fw,
+                                        pitch, s));
+    } else if (quads)
         UFOB_TRY(filter_quads_launch_src(x->f->plan, src, width, height, nz, x->work.ptr, fw, pitch, s));
     else
         UFOB_TRY(filter_rows_launch_src(x->f->plan, src, width, height * nz, x->work.ptr, x->storage, layout, fw,
                                         pitch, s));
     if (x->timing) UFOB_CUDA_TRY(cudaEventRecord(e1, s));
-    UFOB_TRY(ufob_backproject_run(x->bp, x->work.ptr, x->storage, layout, fw, height, nz, pitch,
-                                  (uint64_t)pitch * height, d_out, s));
+    if (umma) {
+        BPGeometry g;
+        UFOB_TRY(bp_prepare(x->bp, fw, height, nz, g, s));
+        UFOB_TRY(bp_umma_launch(g, x->work.ptr, pitch, (uint64_t)pitch * height, x->flags.as<uint8_t>(), d_out, s));
+    } else {
+        UFOB_TRY(ufob_backproject_run(x->bp, x->work.ptr, x->storage, layout, fw, height, nz, pitch,
+                                      (uint64_t)pitch * height, d_out, s));
+    }
     if (x->timing) {
         UFOB_CUDA_TRY(cudaEventRecord(e2, s));
         x->t_filter.emplace_back(e0, e1);
@@ -883,13 +919,18 @@ extern "C" ufob_status ufob_fbp_kernel_times(ufob_fbp *x, double *filter_ms, uin
     return UFOB_OK;
 }
 
-static uint32_t group_slices(uint32_t width, uint32_t height, uint32_t nslices)
+static uint32_t group_slices(const ufob_fbp *x, uint32_t width, uint32_t height, uint32_t nslices)
 {
     // bound the filtered workspace to ~2 GiB, in multiples of 32 slices (whole slice tiles of
     // the backprojectors, which run 4 to 32 slices per CTA) or, for very large slices, of 8
-    const uint64_t per_slice = (uint64_t)(width + 4) * 4 * height;
+    uint64_t per_slice = (uint64_t)(width + 4) * 4 * height;
     uint64_t g = (2ull << 30) / std::max<uint64_t>(per_slice, 1);
     g = g >= 32 ? g / 32 * 32 : std::max<uint64_t>(8, g / 8 * 8);
+    if (x->storage == UFOB_F16 && umma_applies(x->bp->props, nslices)) {
+        // slice octets take 2 bytes a value, and the tensor-core kernel up to 128 slices per CTA
+        const uint64_t g2 = (2ull << 30) / std::max<uint64_t>((uint64_t)(width + 4) * 2 * height, 1);
+        if (g2 >= 128) g = g2 / 128 * 128;
+    }
     return (uint32_t)std::min<uint64_t>(g, nslices);
 }
 
@@ -901,7 +942,7 @@ extern "C" ufob_status ufob_fbp_run(ufob_fbp *x, const float *d_sino, uint32_t w
     uint32_t ow, oh;
     UFOB_TRY(ufob_fbp_get_requisition(x, width, height, &ow, &oh));
     cudaStream_t s = (cudaStream_t)stream;
-    const uint32_t G = group_slices(width, height, nslices);
+    const uint32_t G = group_slices(x, width, height, nslices);
     for (uint32_t z = 0; z < nslices; z += G) {
         const uint32_t nz = std::min(G, nslices - z);
         UFOB_TRY(fbp_group(x, plain_rows(d_sino + (size_t)z * width * height, width), width, height, nz,
@@ -923,7 +964,7 @@ extern "C" ufob_status ufob_fbp_run_projections(ufob_fbp *x, const ufob_preproce
     cudaStream_t s = (cudaStream_t)stream;
     // every slice group reads the same projections: a cone weight restarts at its count each time
     const uint32_t count0 = pre && pre->cone ? ufob_cone_weight_get_count(pre->cone) : 0;
-    const uint32_t G = group_slices(width, n_projections, n_rows);
+    const uint32_t G = group_slices(x, width, n_projections, n_rows);
     for (uint32_t z = 0; z < n_rows; z += G) {
         const uint32_t nz = std::min(G, n_rows - z);
         if (pre && pre->cone) UFOB_TRY(ufob_cone_weight_set_count(pre->cone, count0));

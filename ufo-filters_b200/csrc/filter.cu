@@ -322,7 +322,23 @@ __device__ float2 *fft_smem(float2 *a, float2 *b, const float2 *tw, uint32_t N, 
     return a;
 }
 
-enum OutKind { OUT_F32 = 0, OUT_F16 = 1, OUT_BF16 = 2, OUT_F16_PAIRS = 3, OUT_BF16_PAIRS = 4, OUT_F16_QUADS = 5 };
+enum OutKind {
+    OUT_F32 = 0,
+    OUT_F16 = 1,
+    OUT_BF16 = 2,
+    OUT_F16_PAIRS = 3,
+    OUT_BF16_PAIRS = 4,
+    OUT_F16_QUADS = 5,
+    OUT_F16_OCTS = 6
+};
+
+// Row pairs that share one output cell of a stack layout (two for the slice quads, four for the
+// slice octets), 0 for row-wise layouts.
+template <int OUT>
+__host__ __device__ constexpr uint32_t cell_items()
+{
+    return OUT == OUT_F16_QUADS ? 2u : OUT == OUT_F16_OCTS ? 4u : 0u;
+}
 
 template <int OUT>
 __device__ __forceinline__ void store_value(void *out, size_t idx, float v)
@@ -335,7 +351,7 @@ __device__ __forceinline__ void store_value(void *out, size_t idx, float v)
 template <int OUT>
 __device__ __forceinline__ uint32_t pack_pair(float lo, float hi)
 {
-    if (OUT == OUT_F16_PAIRS || OUT == OUT_F16_QUADS) {
+    if (OUT == OUT_F16_PAIRS || OUT == OUT_F16_QUADS || OUT == OUT_F16_OCTS) {
         __half2 h = __floats2half2_rn(lo, hi);
         return *reinterpret_cast<uint32_t *>(&h);
     } else {
@@ -344,12 +360,16 @@ __device__ __forceinline__ uint32_t pack_pair(float lo, float hi)
     }
 }
 
+// Whether a pair of halves holds an infinity or a NaN (exponent bits all set).
+__device__ __forceinline__ uint32_t half2_nonfinite(uint32_t w) { return ((w & 0x7C007C00u) + 0x04000400u) & 0x80008000u; }
+
 // Rows of one work item (one complex FFT of a + i b): rows 2*pair and
-// 2*pair+1, or for the slice-quad layout (OUT_F16_QUADS, `P` angles per slice)
-// item pair = (group * P + angle) * 2 + half, i.e. slices 4*group + 2*half and
-// 4*group + 2*half + 1 at one angle.
+// 2*pair+1, or for the slice-cell layouts (OUT_F16_QUADS with I = 2 items per
+// cell, OUT_F16_OCTS with I = 4; `P` angles per slice) item pair =
+// (group * P + angle) * I + part, i.e. slices 2*(I*group + part) and the one
+// after it at one angle.
 struct PairMap {
-    uint32_t ra, rb, half;
+    uint32_t ra, rb, part, angle;
     bool hasa, hasb;
     size_t cell0;
 };
@@ -360,14 +380,16 @@ __device__ __forceinline__ PairMap map_pair(uint32_t pair, uint32_t rows, uint32
     PairMap m;
     m.ra = 2 * pair;
     m.rb = 2 * pair + 1;
-    m.half = 0;
+    m.part = m.angle = 0;
     m.cell0 = 0;
     m.hasa = m.ra < rows;
-    if (OUT == OUT_F16_QUADS) {
-        const uint32_t gp = pair >> 1;  // group * P + angle
-        m.half = pair & 1u;
+    if constexpr (cell_items<OUT>() > 0) {
+        constexpr uint32_t I = cell_items<OUT>();
+        const uint32_t gp = pair / I;  // group * P + angle
+        m.part = pair % I;
         const uint32_t grp = gp / P, ang = gp - grp * P;
-        m.ra = (4 * grp + 2 * m.half) * P + ang;
+        m.angle = ang;
+        m.ra = 2 * (I * grp + m.part) * P + ang;
         m.rb = m.ra + P;
         m.hasa = m.ra < rows;
         m.cell0 = (size_t)gp * out_pitch;
@@ -380,19 +402,32 @@ __device__ __forceinline__ PairMap map_pair(uint32_t pair, uint32_t rows, uint32
 // in the output layout; threads t0, t0 + step, ... share the row.
 template <int OUT, typename GET>
 __device__ __forceinline__ void store_pair(const PairMap &m, GET X, void *__restrict__ out, uint32_t out_w,
-                                           uint32_t out_pitch, uint32_t t0, uint32_t step)
+                                           uint32_t out_pitch, uint32_t t0, uint32_t step,
+                                           uint8_t *__restrict__ flags)
 {
     if (OUT == OUT_F16_QUADS) {
-        // words `half` (taps j-1) and 2 + `half` (taps j) of cell j; rows a, b in the low, high halves
+        // words `part` (taps j-1) and 2 + `part` (taps j) of cell j; rows a, b in the low, high halves
         uint32_t *o = reinterpret_cast<uint32_t *>(out) + m.cell0 * 4;
         for (uint32_t j = t0; j < out_pitch; j += step) {
             float2 lo = (j >= 1 && j - 1 < out_w) ? X(j - 1) : make_float2(0.f, 0.f);
             float2 hi = (j < out_w) ? X(j) : make_float2(0.f, 0.f);
             if (!m.hasa) lo.x = hi.x = 0.f;  // slices past the stack: exact zeros, not FFT round-off
             if (!m.hasb) lo.y = hi.y = 0.f;
-            o[(size_t)j * 4 + m.half] = pack_pair<OUT>(lo.x, lo.y);
-            o[(size_t)j * 4 + 2 + m.half] = pack_pair<OUT>(hi.x, hi.y);
+            o[(size_t)j * 4 + m.part] = pack_pair<OUT>(lo.x, lo.y);
+            o[(size_t)j * 4 + 2 + m.part] = pack_pair<OUT>(hi.x, hi.y);
         }
+    } else if (OUT == OUT_F16_OCTS) {
+        uint32_t *o = reinterpret_cast<uint32_t *>(out) + m.cell0 * 4;
+        uint32_t bad = 0;
+        for (uint32_t j = t0; j < out_pitch; j += step) {
+            float2 v = j < out_w ? X(j) : make_float2(0.f, 0.f);
+            if (!m.hasa) v.x = 0.f;  // slices past the stack: exact zeros, not FFT round-off
+            if (!m.hasb) v.y = 0.f;
+            const uint32_t w = pack_pair<OUT>(v.x, v.y);
+            bad |= half2_nonfinite(w);
+            o[(size_t)j * 4 + m.part] = w;
+        }
+        if (bad) flags[m.angle] = 1;
     } else if (OUT == OUT_F16_PAIRS || OUT == OUT_BF16_PAIRS) {
         uint32_t *o = reinterpret_cast<uint32_t *>(out);
         for (uint32_t j = t0; j < out_pitch; j += step) {
@@ -416,7 +451,7 @@ template <int OUT, bool PRE>
 __device__ __forceinline__ void filter_pair(const RowSource &src, uint32_t width, uint32_t rows, uint32_t pair,
                                             float2 *bufA, float2 *bufB, const float2 *tw, const float2 *gains,
                                             uint32_t N, int log2N, void *__restrict__ out, uint32_t out_w,
-                                            uint32_t out_pitch, uint32_t P = 0)
+                                            uint32_t out_pitch, uint32_t P = 0, uint8_t *flags = nullptr)
 {
     const PairMap m = map_pair<OUT>(pair, rows, P, out_pitch);
     uint32_t ya, pa_proj, yb, pb_proj;
@@ -450,7 +485,7 @@ __device__ __forceinline__ void filter_pair(const RowSource &src, uint32_t width
     __syncthreads();
     float2 *other = (Z == bufA) ? bufB : bufA;
     float2 *X = fft_smem<true>(Z, other, tw, N, log2N);
-    store_pair<OUT>(m, [X](uint32_t i) { return X[i]; }, out, out_w, out_pitch, threadIdx.x, blockDim.x);
+    store_pair<OUT>(m, [X](uint32_t i) { return X[i]; }, out, out_w, out_pitch, threadIdx.x, blockDim.x, flags);
 }
 
 template <int OUT, bool PRE>
@@ -458,7 +493,8 @@ __global__ void __launch_bounds__(kFilterThreads) k_filter_rows(const RowSource 
                                                                 const float2 *__restrict__ g_tw,
                                                                 const float2 *__restrict__ g_gains, uint32_t N,
                                                                 int log2N, void *__restrict__ out, uint32_t out_w,
-                                                                uint32_t out_pitch, uint32_t npairs, uint32_t P)
+                                                                uint32_t out_pitch, uint32_t npairs, uint32_t P,
+                                                                uint8_t *__restrict__ flags)
 {
     extern __shared__ float4 smem_f4[];
     float2 *bufA = reinterpret_cast<float2 *>(smem_f4);
@@ -470,7 +506,8 @@ __global__ void __launch_bounds__(kFilterThreads) k_filter_rows(const RowSource 
     for (uint32_t i = threadIdx.x; i <= N / 2; i += blockDim.x) gains[i] = g_gains[i];
 
     for (uint32_t pair = blockIdx.x; pair < npairs; pair += gridDim.x)
-        filter_pair<OUT, PRE>(src, width, rows, pair, bufA, bufB, tw, gains, N, log2N, out, out_w, out_pitch, P);
+        filter_pair<OUT, PRE>(src, width, rows, pair, bufA, bufB, tw, gains, N, log2N, out, out_w, out_pitch, P,
+                              flags);
 }
 
 // ------------------------------------------------------------ register-radix kernel (N = 256 .. 4096)
@@ -707,7 +744,7 @@ __global__ void __launch_bounds__(kFastThreads, 2) k_filter_fast(const RowSource
                                                              const float2 *__restrict__ g_gains,
                                                              void *__restrict__ out, uint32_t out_w,
                                                              uint32_t out_pitch, uint32_t npairs, uint32_t P,
-                                                             int *__restrict__ err)
+                                                             uint8_t *__restrict__ flags, int *__restrict__ err)
 {
     constexpr uint32_t N = 1u << LOGN, T = N / 16, TEAMS = kFastThreads / T;
     constexpr uint32_t R3 = N / 256, LR3 = R3 >= 16 ? 4 : R3 >= 8 ? 3 : R3 >= 4 ? 2 : R3 >= 2 ? 1 : 0;
@@ -744,7 +781,7 @@ __global__ void __launch_bounds__(kFastThreads, 2) k_filter_fast(const RowSource
                       // pairs, where a quad output cell takes both teams' results
     if (STG && t == 0 && iters > 0) issue(0);
     // the cell store of the slice-quad output reads the partner team's result
-    constexpr bool CELLS = OUT == OUT_F16_QUADS && TEAMS % 2 == 0;
+    constexpr bool CELLS = cell_items<OUT>() > 0 && TEAMS % 2 == 0;
     static_assert(2 * T <= 32 || TEAMS + TEAMS / 2 <= 15, "named barrier ids 1 .. 15");
     constexpr uint32_t SG = CELLS ? 2 * T : T;  // threads that share a result buffer
     const uint32_t sid = CELLS ? 1 + TEAMS + (team >> 1) : 1 + team;
@@ -874,7 +911,6 @@ __global__ void __launch_bounds__(kFastThreads, 2) k_filter_fast(const RowSource
                 const size_t xoff = (size_t)(X - bufA);  // this team's result: bufA or bufB
                 const float2 *X0 = gains + (N / 2 + 2) + (size_t)(2 * u) * 2 * N + xoff;
                 const float2 *X1 = X0 + 2 * N;
-                uint4 *o = reinterpret_cast<uint4 *>(out) + m0.cell0;
                 auto taps = [&](const float2 *Xh, const PairMap &mh, uint32_t j, bool prev) {
                     const uint32_t e = prev ? j - 1 : j;
                     float2 v = ((!prev || j >= 1) && e < out_w) ? Xh[e] : make_float2(0.f, 0.f);
@@ -882,12 +918,25 @@ __global__ void __launch_bounds__(kFastThreads, 2) k_filter_fast(const RowSource
                     if (!mh.hasb) v.y = 0.f;
                     return pack_pair<OUT>(v.x, v.y);
                 };
-                for (uint32_t j = i0; j < out_pitch; j += 2 * T)
-                    o[j] = make_uint4(taps(X0, m0, j, true), taps(X1, m1, j, true), taps(X0, m0, j, false),
-                                      taps(X1, m1, j, false));
+                if constexpr (OUT == OUT_F16_QUADS) {
+                    uint4 *o = reinterpret_cast<uint4 *>(out) + m0.cell0;
+                    for (uint32_t j = i0; j < out_pitch; j += 2 * T)
+                        o[j] = make_uint4(taps(X0, m0, j, true), taps(X1, m1, j, true), taps(X0, m0, j, false),
+                                          taps(X1, m1, j, false));
+                } else {
+                    // four of the eight slices: half a cell
+                    uint2 *o = reinterpret_cast<uint2 *>(out) + m0.cell0 * 2 + (m0.part >> 1);
+                    uint32_t bad = 0;
+                    for (uint32_t j = i0; j < out_pitch; j += 2 * T) {
+                        const uint2 w = make_uint2(taps(X0, m0, j, false), taps(X1, m1, j, false));
+                        bad |= half2_nonfinite(w.x) | half2_nonfinite(w.y);
+                        o[(size_t)j * 2] = w;
+                    }
+                    if (bad) flags[m0.angle] = 1;
+                }
             }
         } else {
-            if (live) store_pair<OUT>(m, [X](uint32_t i) { return X[i]; }, out, out_w, out_pitch, t, T);
+            if (live) store_pair<OUT>(m, [X](uint32_t i) { return X[i]; }, out, out_w, out_pitch, t, T, flags);
         }
     }
 }
@@ -925,9 +974,19 @@ __global__ void __launch_bounds__(kFilterThreads) k_filter_batch(const BatchFilt
     }
 }
 
+// Work items of a launch: two rows each, or whole cells of the stack layouts.
+template <int OUT>
+static uint32_t row_pairs(uint32_t rows, uint32_t P)
+{
+    constexpr uint32_t I = cell_items<OUT>();
+    if (I == 0) return (rows + 1) / 2;
+    return (rows / P + 2 * I - 1) / (2 * I) * P * I;
+}
+
 template <int OUT, bool PRE>
 static ufob_status launch_rows_t(const FilterPlan &plan, const RowSource &src, uint32_t width, uint32_t rows,
-                                 void *d_out, uint32_t out_w, uint32_t out_pitch, cudaStream_t s, uint32_t P)
+                                 void *d_out, uint32_t out_w, uint32_t out_pitch, cudaStream_t s, uint32_t P,
+                                 uint8_t *flags)
 {
     const uint32_t N = plan.nfft;
     const size_t smem = sizeof(float2) * (3 * (size_t)N + N / 2 + 1);
@@ -939,13 +998,12 @@ static ufob_status launch_rows_t(const FilterPlan &plan, const RowSource &src, u
     int per_sm = 0;
     UFOB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFilterThreads, smem));
     if (per_sm < 1) return fail(UFOB_ERR_UNSUPPORTED, "filter: FFT width %u does not fit in shared memory", N);
-    // slice-quad layout: two items per (group of four slices, angle)
-    const uint32_t npairs = OUT == OUT_F16_QUADS ? (rows / P + 3) / 4 * P * 2 : (rows + 1) / 2;
+    const uint32_t npairs = row_pairs<OUT>(rows, P);
     uint32_t grid = (uint32_t)num_sms() * (uint32_t)per_sm * 4;
     if (grid > npairs) grid = npairs;
     if (grid == 0) return UFOB_OK;
     kern<<<grid, kFilterThreads, smem, s>>>(src, width, rows, plan.d_twiddle.as<float2>(), plan.d_gains.as<float2>(),
-                                            N, log2N, d_out, out_w, out_pitch, npairs, P);
+                                            N, log2N, d_out, out_w, out_pitch, npairs, P, flags);
     UFOB_CUDA_TRY(cudaGetLastError());
     note_launch();
     return UFOB_OK;
@@ -981,7 +1039,8 @@ static bool rows_stageable(const RowSource &src, uint32_t width, uint32_t N)
 
 template <int OUT, bool PRE, int LOGN>
 static ufob_status launch_fast_t(const FilterPlan &plan, const RowSource &src, uint32_t width, uint32_t rows,
-                                 void *d_out, uint32_t out_w, uint32_t out_pitch, cudaStream_t s, uint32_t P)
+                                 void *d_out, uint32_t out_w, uint32_t out_pitch, cudaStream_t s, uint32_t P,
+                                 uint8_t *flags)
 {
     constexpr uint32_t N = 1u << LOGN, TEAMS = kFastThreads / (N / 16);
     int per_sm = 0, per_sm_stg = 0;
@@ -993,17 +1052,17 @@ static ufob_status launch_fast_t(const FilterPlan &plan, const RowSource &src, u
         UFOB_TRY((fast_occupancy<OUT, false, LOGN, true>(per_sm_stg)));
         stg = per_sm_stg >= per_sm;
     }
-    const uint32_t npairs = OUT == OUT_F16_QUADS ? (rows / P + 3) / 4 * P * 2 : (rows + 1) / 2;
+    const uint32_t npairs = row_pairs<OUT>(rows, P);
     uint32_t grid = (uint32_t)num_sms() * (uint32_t)per_sm;
     grid = std::min(grid, (npairs + TEAMS - 1) / TEAMS);
     if (grid == 0) return UFOB_OK;
     const float2 *tab = plan.d_pass_tw.as<float2>(), *gains = plan.d_gains.as<float2>();
     if (stg)
         k_filter_fast<OUT, false, LOGN, true><<<grid, kFastThreads, fast_smem<LOGN, true>(), s>>>(
-            src, width, rows, tab, gains, d_out, out_w, out_pitch, npairs, P, device_error_word());
+            src, width, rows, tab, gains, d_out, out_w, out_pitch, npairs, P, flags, device_error_word());
     else
         k_filter_fast<OUT, PRE, LOGN, false><<<grid, kFastThreads, fast_smem<LOGN, false>(), s>>>(
-            src, width, rows, tab, gains, d_out, out_w, out_pitch, npairs, P, device_error_word());
+            src, width, rows, tab, gains, d_out, out_w, out_pitch, npairs, P, flags, device_error_word());
     UFOB_CUDA_TRY(cudaGetLastError());
     note_launch();
     return UFOB_OK;
@@ -1011,25 +1070,27 @@ static ufob_status launch_fast_t(const FilterPlan &plan, const RowSource &src, u
 
 template <int OUT, bool PRE>
 static ufob_status launch_rows_p(const FilterPlan &plan, const RowSource &src, uint32_t width, uint32_t rows,
-                                 void *d_out, uint32_t out_w, uint32_t out_pitch, cudaStream_t s, uint32_t P)
+                                 void *d_out, uint32_t out_w, uint32_t out_pitch, cudaStream_t s, uint32_t P,
+                                 uint8_t *flags)
 {
     if (fast_filter_enabled()) switch (plan.nfft) {
-        case 256: return launch_fast_t<OUT, PRE, 8>(plan, src, width, rows, d_out, out_w, out_pitch, s, P);
-        case 512: return launch_fast_t<OUT, PRE, 9>(plan, src, width, rows, d_out, out_w, out_pitch, s, P);
-        case 1024: return launch_fast_t<OUT, PRE, 10>(plan, src, width, rows, d_out, out_w, out_pitch, s, P);
-        case 2048: return launch_fast_t<OUT, PRE, 11>(plan, src, width, rows, d_out, out_w, out_pitch, s, P);
-        case 4096: return launch_fast_t<OUT, PRE, 12>(plan, src, width, rows, d_out, out_w, out_pitch, s, P);
+        case 256: return launch_fast_t<OUT, PRE, 8>(plan, src, width, rows, d_out, out_w, out_pitch, s, P, flags);
+        case 512: return launch_fast_t<OUT, PRE, 9>(plan, src, width, rows, d_out, out_w, out_pitch, s, P, flags);
+        case 1024: return launch_fast_t<OUT, PRE, 10>(plan, src, width, rows, d_out, out_w, out_pitch, s, P, flags);
+        case 2048: return launch_fast_t<OUT, PRE, 11>(plan, src, width, rows, d_out, out_w, out_pitch, s, P, flags);
+        case 4096: return launch_fast_t<OUT, PRE, 12>(plan, src, width, rows, d_out, out_w, out_pitch, s, P, flags);
         default: break;
         }
-    return launch_rows_t<OUT, PRE>(plan, src, width, rows, d_out, out_w, out_pitch, s, P);
+    return launch_rows_t<OUT, PRE>(plan, src, width, rows, d_out, out_w, out_pitch, s, P, flags);
 }
 
 template <int OUT>
 static ufob_status launch_rows(const FilterPlan &plan, const RowSource &src, uint32_t width, uint32_t rows,
-                               void *d_out, uint32_t out_w, uint32_t out_pitch, cudaStream_t s, uint32_t P = 0)
+                               void *d_out, uint32_t out_w, uint32_t out_pitch, cudaStream_t s, uint32_t P = 0,
+                               uint8_t *flags = nullptr)
 {
-    if (src.has_pre()) return launch_rows_p<OUT, true>(plan, src, width, rows, d_out, out_w, out_pitch, s, P);
-    return launch_rows_p<OUT, false>(plan, src, width, rows, d_out, out_w, out_pitch, s, P);
+    if (src.has_pre()) return launch_rows_p<OUT, true>(plan, src, width, rows, d_out, out_w, out_pitch, s, P, flags);
+    return launch_rows_p<OUT, false>(plan, src, width, rows, d_out, out_w, out_pitch, s, P, flags);
 }
 
 ufob_status filter_rows_launch_src(const FilterPlan &plan, const RowSource &src, uint32_t width, uint32_t rows,
@@ -1078,6 +1139,22 @@ ufob_status filter_quads_launch_src(const FilterPlan &plan, const RowSource &src
         return fail(UFOB_ERR_INVALID, "filter: bad slice-quad sizes (width %u, N %u, crop %u, pitch %u)", width, N,
                     out_w, out_pitch);
     return launch_rows<OUT_F16_QUADS>(plan, src, width, P * nz, d_out, out_w, out_pitch, stream, P);
+}
+
+// The same into slice octets: [ceil(nz/8)][P][out_pitch] cells of 16 bytes, cell j of a row
+// holding bin j of eight slices; d_flags[P] (zeroed by the caller) is set to 1 for every angle with
+// a non-finite value (see bp_umma.cu).
+ufob_status filter_octs_launch_src(const FilterPlan &plan, const RowSource &src, uint32_t width, uint32_t P,
+                                   uint32_t nz, void *d_out, uint8_t *d_flags, uint32_t out_w, uint32_t out_pitch,
+                                   cudaStream_t stream)
+{
+    const uint32_t N = plan.nfft;
+    if (N > kMaxFusedFFT || N < 4)
+        return fail(UFOB_ERR_UNSUPPORTED, "filter: FFT width %u outside the supported range [4, %u]", N, kMaxFusedFFT);
+    if (width > N || out_w > N || out_pitch < out_w || !P)
+        return fail(UFOB_ERR_INVALID, "filter: bad slice-octet sizes (width %u, N %u, crop %u, pitch %u)", width, N,
+                    out_w, out_pitch);
+    return launch_rows<OUT_F16_OCTS>(plan, src, width, P * nz, d_out, out_w, out_pitch, stream, P, d_flags);
 }
 
 ufob_status filter_quads_launch(const FilterPlan &plan, const float *d_in, uint32_t width, uint32_t P, uint32_t nz,

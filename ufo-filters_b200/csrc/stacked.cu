@@ -67,6 +67,44 @@ ufob_status pack_quads_launch(const float *d_in, uint32_t W, uint32_t P, uint32_
     return UFOB_OK;
 }
 
+// ------------------------------------------------------------ FP32 stack -> slice octets
+
+// cell (g, p, j): halves of bin j of slices 8g..8g+7; flags[p] = 1 where one is not finite
+__global__ void k_pack_octs(const float *__restrict__ in, uint32_t W, uint32_t P, uint32_t Z, uint4 *__restrict__ out,
+                            uint8_t *__restrict__ flags)
+{
+    const uint32_t g = blockIdx.y;
+    for (uint32_t p = blockIdx.x; p < P; p += gridDim.x) {
+        uint32_t bad = 0;
+        for (uint32_t j = threadIdx.x; j < W; j += blockDim.x) {
+            uint32_t w[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const uint32_t z = 8 * g + 2 * k;
+                const float *row = in + ((uint64_t)z * P + p) * W + j;
+                const float a = z < Z ? __ldg(row) : 0.f, b = z + 1 < Z ? __ldg(row + (uint64_t)P * W) : 0.f;
+                const __half2 h = __floats2half2_rn(a, b);
+                w[k] = *reinterpret_cast<const uint32_t *>(&h);
+                bad |= ((w[k] & 0x7C007C00u) + 0x04000400u) & 0x80008000u;
+            }
+            out[((uint64_t)g * P + p) * W + j] = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        if (bad) flags[p] = 1;
+    }
+}
+
+ufob_status pack_octs_launch(const float *d_in, uint32_t W, uint32_t P, uint32_t Z, void *d_out, uint8_t *d_flags,
+                             cudaStream_t s)
+{
+    const uint32_t groups = (Z + 7) / 8;
+    if (!groups || !P || !W) return UFOB_OK;
+    dim3 grid(std::min<uint32_t>(P, std::max<uint32_t>(1, (uint32_t)num_sms() * 16 / groups)), groups);
+    k_pack_octs<<<grid, 256, 0, s>>>(d_in, W, P, Z, reinterpret_cast<uint4 *>(d_out), d_flags);
+    UFOB_CUDA_TRY(cudaGetLastError());
+    note_launch();
+    return UFOB_OK;
+}
+
 // ------------------------------------------------------------ int8 path
 
 // Order-preserving map of finite floats onto unsigned integers.

@@ -207,6 +207,11 @@ ufob_status filter_rows_launch_src(const FilterPlan &plan, const RowSource &src,
 ufob_status filter_quads_launch_src(const FilterPlan &plan, const RowSource &src, uint32_t width, uint32_t P,
                                     uint32_t nz, void *d_out, uint32_t out_w, uint32_t out_pitch,
                                     cudaStream_t stream);
+// Slice-octet output, as the tensor-core backprojector reads it; d_flags[P], zeroed before,
+// marks the angles that hold a non-finite value.
+ufob_status filter_octs_launch_src(const FilterPlan &plan, const RowSource &src, uint32_t width, uint32_t P,
+                                   uint32_t nz, void *d_out, uint8_t *d_flags, uint32_t out_w, uint32_t out_pitch,
+                                   cudaStream_t stream);
 // RowSource for projections [n][height][pitch]: detector rows first_row ..
 // first_row + n_rows - 1 in projection order (sinograms = false, r = projection
 // * n_rows + row) or as sinograms (true, r = row * n + projection), with the
@@ -215,9 +220,11 @@ ufob_status projection_source(const ufob_preprocess *pre, const float *d_proj, u
                               uint32_t n, uint32_t pitch, bool sinograms, uint32_t first_row, uint32_t n_rows,
                               RowSource &src, cudaStream_t s);
 struct BPGeometry;
-// stacked-backproject helpers: FP32 stack [Z][P][W] -> slice-quad cells
-// [ceil(Z/4)][P][W+1]; the whole int8 path (d_work >= ceil(Z/4)*P*W words,
+// stacked-backproject helpers: FP32 stack [Z][P][W] -> slice-octet cells [ceil(Z/8)][P][W] (flags as
+// the filter's) or slice-quad cells [ceil(Z/4)][P][W+1]; the whole int8 path (d_work >= ceil(Z/4)*P*W words,
 // d_keys = 2 words of device scratch).
+ufob_status pack_octs_launch(const float *d_in, uint32_t W, uint32_t P, uint32_t Z, void *d_out, uint8_t *d_flags,
+                             cudaStream_t s);
 ufob_status pack_quads_launch(const float *d_in, uint32_t W, uint32_t P, uint32_t Z, void *d_out, cudaStream_t s);
 ufob_status stacked_u8_launch(const BPGeometry &g, const float *d_sino, void *d_work, uint32_t *d_keys, float *d_out,
                               cudaStream_t s);
@@ -258,6 +265,10 @@ ufob_status filter_quads_launch(const FilterPlan &plan, const float *d_in, uint3
 ufob_status bp_quads_launch(const BPGeometry &g, const void *d_sino, uint32_t pitch, uint64_t group_pitch,
                             float *d_out, bool kahan, int acc, int tile, cudaStream_t stream);
 int bp_quad_tiles();
+// The same on the tensor cores from slice octets [ceil(nz/8)][P][pitch] (pitch and group_pitch in
+// 16-byte cells).
+ufob_status bp_umma_launch(const BPGeometry &g, const void *d_sino, uint32_t pitch, uint64_t group_pitch,
+                           const uint8_t *d_flags, float *d_out, cudaStream_t stream);
 
 // Kernel arguments of one backprojection (one stack or one batch job).
 struct BPArgs {
