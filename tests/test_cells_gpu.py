@@ -1,0 +1,70 @@
+"""FP32 stacks from slice cells: the same bits as the row kernel (tile 2, 32 x 32 pixels of four
+slices, whose arithmetic and order it keeps) at edges of its 32 x 64 x 8 tiles, odd widths and
+regions, angle counts around its stages and sum blocks, quadrants and exact 0 and 90 degree angles,
+and the FP64 oracle on a few slices."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+import oracle
+import ufob
+
+pytestmark = pytest.mark.gpu
+
+
+def _both(sino, **props):
+    t = torch.from_numpy(sino).cuda()
+    a = ufob.BackprojectTask(**props).process(t)
+    b = ufob.BackprojectTask(tile=2, **props).process(t)
+    torch.cuda.synchronize()
+    ufob.device_status()
+    return a.cpu().numpy(), b.cpu().numpy()
+
+
+# (slices, angles, width, properties); the launches are large enough for the cell kernel (two CTAs
+# per SM: ceil(w / 32) * ceil(h / 64) * ceil(nz / 8) >= 296)
+CASES = [
+    (64, 40, 250, {}),
+    (5, 33, 1100, {}),
+    (37, 1, 353, {}),
+    (37, 7, 353, dict(axis_pos=150.25)),
+    (33, 8, 385, dict(angle_offset=math.pi / 2)),
+    (40, 17, 417, dict(angle_step=math.pi / 2)),  # exact 0, 90, 180, 270 degrees
+    (40, 24, 416, dict(axis_pos=207.5, angle_step=math.pi / 4, angle_offset=5.5)),
+    (70, 31, 256, dict(roi_x=3, roi_y=17, roi_width=243, roi_height=191)),
+    (32, 64, 320, dict(roi_x=250, roi_y=100, roi_width=320, roi_height=500)),  # partly beyond the detector
+]
+
+
+@pytest.mark.parametrize("nz,P,W,props", CASES)
+def test_same_bits_as_rows(cuda, nz, P, W, props):
+    sino = np.random.default_rng(nz * P + W).standard_normal((nz, P, W)).astype(np.float32)
+    got, rows = _both(sino, **props)
+    np.testing.assert_array_equal(got, rows)
+    if not props.get("roi_width"):
+        for z in (0, nz - 1):
+            ref = oracle.backproject(sino[z], **props)
+            assert oracle.rel_l2(got[z], ref) < 2e-5
+
+
+def test_nonfinite_and_groups(cuda):
+    """Two groups of 32 slices; infinities and NaNs reach the same pixels as in the row kernel."""
+    sino = np.random.default_rng(5).standard_normal((41, 30, 300)).astype(np.float32)
+    sino[3, 4, 100], sino[40, 29, 0], sino[35, 7, 299] = math.inf, math.nan, -math.inf
+    got, rows = _both(sino)
+    np.testing.assert_array_equal(got, rows)
+
+
+def test_unaligned_rows(cuda):
+    """A pitch and a base the row kernel has to restage."""
+    nz, P, W = 32, 20, 321
+    buf = torch.randn(nz, P, W + 2, device="cuda")
+    out = [torch.empty(nz, W, W, device="cuda") for _ in range(2)]
+    for o, tile in zip(out, (-1, 2)):
+        bp = ufob.BackprojectTask(tile=tile)
+        ufob.check(ufob.lib().ufob_backproject_run(bp._h, buf.data_ptr() + 4, ufob.F32, ufob.ROWS, W, P, nz, W + 2,
+                                                   (W + 2) * P, o.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    assert torch.equal(out[0], out[1])

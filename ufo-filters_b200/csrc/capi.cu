@@ -374,6 +374,7 @@ struct ufob_backproject {
     ufob_bp_props props;
     DevBuf sincos;
     DevBuf aligned;  // copy of a sinogram whose pitch is not TMA-compatible
+    DevBuf cells;    // slice cells of a group of an FP32 stack
     DevBuf partial;  // per-angle-group images of one small sinogram (split_plan)
     // cache key of the sin/cos table
     uint32_t key_P = 0, key_nproj = 0, key_offset = 0;
@@ -552,6 +553,13 @@ static bool want_kahan(const ufob_bp_props &p, SinoKind, uint32_t)
     return p.compensated > 0;
 }
 
+// Whether an FP32 stack runs from slice cells: the default form (no compensated sums, no pinned tile
+// or angle groups) and enough tiles.
+static bool cells_apply(const ufob_bp_props &p, const BPGeometry &g)
+{
+    return p.mode != UFOB_BP_NEAREST && p.tile < 0 && p.compensated <= 0 && p.angle_groups <= 1 && bp_cells_applies(g);
+}
+
 // A single sinogram is split into 2, 4 or 8 equal angle groups (at least 32 angles each) whose
 // partial images are summed, when that spreads its 32x96 tiles more evenly over the SMs: the
 // busiest SM's share of tiles over the average one drops by more than 5%; 1 = no split.
@@ -635,6 +643,21 @@ extern "C" ufob_status ufob_backproject_run(ufob_backproject *bp, const void *d_
         if (kind != SINO_F32) return fail(UFOB_ERR_INVALID, "backproject: mode=nearest needs an F32 sinogram");
         return bp_nearest_launch(g, (const float *)d_sino, pitch, slice_pitch, d_out, s);
     }
+    const bool kahan = want_kahan(bp->props, kind, height);
+    if (kind == SINO_F32 && cells_apply(bp->props, g)) {
+        // slice cells by groups of 32 slices; without the memory for them the row kernel does it
+        const uint32_t G = std::min(nslices, 32u);
+        if (bp->cells.ensure((size_t)((G + 3) / 4) * 16 * width * height) == UFOB_OK) {
+            for (uint32_t z = 0; z < nslices; z += G) {
+                BPGeometry gz = g;
+                gz.nz = std::min(G, nslices - z);
+                UFOB_TRY(pack_cells_launch((const float *)d_sino + z * slice_pitch, pitch, slice_pitch, width, height,
+                                           gz.nz, bp->cells.ptr, s));
+                UFOB_TRY(bp_cells_launch(gz, bp->cells.ptr, d_out + (size_t)z * g.roi_w * g.roi_h, s));
+            }
+            return UFOB_OK;
+        }
+    }
     const void *src = d_sino;
     if (((uintptr_t)d_sino & 15) || (pitch & 3) || (slice_pitch & 3)) {
         // TMA needs 16-byte aligned rows: restage into an aligned copy
@@ -648,7 +671,6 @@ extern "C" ufob_status ufob_backproject_run(ufob_backproject *bp, const void *d_
         pitch = ap;
         slice_pitch = (uint64_t)ap * height;
     }
-    const bool kahan = want_kahan(bp->props, kind, height);
     const SplitPlan plan = split_plan(g, bp->props.tile, bp->props.angle_groups);
     if (bp->props.angle_groups > 1 && plan.groups != (uint32_t)bp->props.angle_groups)
         return fail(UFOB_ERR_INVALID,

@@ -265,6 +265,15 @@ ufob_status filter_quads_launch(const FilterPlan &plan, const float *d_in, uint3
 ufob_status bp_quads_launch(const BPGeometry &g, const void *d_sino, uint32_t pitch, uint64_t group_pitch,
                             float *d_out, bool kahan, int acc, int tile, cudaStream_t stream);
 int bp_quad_tiles();
+// 4-D map over [groups][P][cells] 16-byte cells.
+ufob_status make_quad_map(CUtensorMap *map, const void *base, uint32_t cells, uint32_t P, uint32_t groups,
+                          uint32_t pitch, uint64_t group_pitch, uint32_t box_cells, uint32_t box_groups);
+// FP32 stacks from slice cells [ceil(nz/4)][P][W] of four floats: the row kernel's image, bit for
+// bit.  pack_cells_launch makes the cells from rows.
+bool bp_cells_applies(const BPGeometry &g);
+ufob_status bp_cells_launch(const BPGeometry &g, const void *d_cells, float *d_out, cudaStream_t stream);
+ufob_status pack_cells_launch(const float *d_in, uint32_t pitch, uint64_t slice_pitch, uint32_t W, uint32_t P,
+                              uint32_t Z, void *d_out, cudaStream_t s);
 // The same on the tensor cores from slice octets [ceil(nz/8)][P][pitch] (pitch and group_pitch in
 // 16-byte cells).
 ufob_status bp_umma_launch(const BPGeometry &g, const void *d_sino, uint32_t pitch, uint64_t group_pitch,
