@@ -69,16 +69,25 @@ __global__ void k_unshuffle_in(const float *__restrict__ fbp, bf16 *__restrict__
     }
 }
 
-// out = fbp + s * depth-to-space(o)   (o FP32 [B][H][W][16])
-__global__ void k_shuffle_out(const float *__restrict__ o, const float *__restrict__ fbp, float *__restrict__ out, int B,
-                              int H, int W, float s)
+// out = fbp + s * depth-to-space(o)   (o FP32 [B][H][W][16]), four output pixels of one o pixel
+// per thread (n4 of them)
+__global__ void k_shuffle_out(const float *__restrict__ o, const float *__restrict__ fbp, float *__restrict__ out,
+                              uint32_t n4, int W, float s)
 {
-    const size_t n = (size_t)B * kS * kS * H * W;
-    GRID_STRIDE(i, n) {
-        const int X = (int)(i % (kS * W)), Y = (int)((i / (kS * W)) % (kS * H));
-        const size_t b = i / ((size_t)kS * kS * H * W);
-        const int c = kS * (Y % kS) + (X % kS);
-        out[i] = fbp[i] + s * o[((b * H + Y / kS) * W + X / kS) * 16 + c];
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += gridDim.x * blockDim.x) {
+        const uint32_t Y = i / W, x = i - Y * W, y = Y / kS;  // rows of all images run on
+        const float4 v = *reinterpret_cast<const float4 *>(o + ((size_t)y * W + x) * 16 + kS * (Y - y * kS));
+        const float4 f = __ldg(reinterpret_cast<const float4 *>(fbp) + i);
+        const float4 r = make_float4(f.x + s * v.x, f.y + s * v.y, f.z + s * v.z, f.w + s * v.w);
+        if (((uintptr_t)out & 15) == 0) {
+            reinterpret_cast<float4 *>(out)[i] = r;
+        } else {
+            float *p = out + (size_t)i * 4;
+            p[0] = r.x;
+            p[1] = r.y;
+            p[2] = r.z;
+            p[3] = r.w;
+        }
     }
 }
 
@@ -104,90 +113,154 @@ __global__ void k_shuffle_out_grad(const float *__restrict__ dout, bf16 *__restr
     }
 }
 
-// 2x2 average pool, NHWC
-__global__ void k_pool(const bf16 *__restrict__ in, bf16 *__restrict__ out, int B, int H, int W, int C)
+// The element-wise kernels below move eight channels (16 bytes of BF16) per thread; element i of
+// `n8` is channel group i % (C / 8) of pixel i / (C / 8), in 32 bits (n8 < 2^32 for any tensor that
+// fits the device).
+struct Vec8 {
+    float v[8];
+};
+
+__device__ __forceinline__ Vec8 load8(const bf16 *p)
 {
-    const int h = H / 2, w = W / 2;
-    const size_t n = (size_t)B * h * w * C;
-    GRID_STRIDE(i, n) {
-        const int c = (int)(i % C);
-        const size_t pix = i / C;
-        const int x = (int)(pix % w), y = (int)((pix / w) % h);
-        const size_t b = pix / ((size_t)w * h);
-        const bf16 *s = in + ((b * H + 2 * y) * W + 2 * x) * C + c;
-        const float v = __bfloat162float(s[0]) + __bfloat162float(s[C]) + __bfloat162float(s[(size_t)W * C]) +
-                        __bfloat162float(s[(size_t)W * C + C]);
-        out[i] = __float2bfloat16(0.25f * v);
+    const uint4 q = __ldg(reinterpret_cast<const uint4 *>(p));
+    const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&q);
+    Vec8 r;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const float2 f = __bfloat1622float2(h[k]);
+        r.v[2 * k] = f.x;
+        r.v[2 * k + 1] = f.y;
+    }
+    return r;
+}
+
+__device__ __forceinline__ Vec8 load8(const float *p)
+{
+    const float4 a = *reinterpret_cast<const float4 *>(p), b = *reinterpret_cast<const float4 *>(p + 4);
+    return Vec8{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}};
+}
+
+__device__ __forceinline__ void store8(bf16 *p, const Vec8 &r)
+{
+    uint4 q;
+    __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&q);
+#pragma unroll
+    for (int k = 0; k < 4; k++) h[k] = __floats2bfloat162_rn(r.v[2 * k], r.v[2 * k + 1]);
+    *reinterpret_cast<uint4 *>(p) = q;
+}
+
+__device__ __forceinline__ void store8(float *p, const Vec8 &r)
+{
+    *reinterpret_cast<float4 *>(p) = make_float4(r.v[0], r.v[1], r.v[2], r.v[3]);
+    *reinterpret_cast<float4 *>(p + 4) = make_float4(r.v[4], r.v[5], r.v[6], r.v[7]);
+}
+
+// Channel offset of element i and its pixel's row base in a w x h image: (image, y, x).
+struct Pix {
+    uint32_t c, x, y, b;
+};
+
+__device__ __forceinline__ Pix split8(uint32_t i, uint32_t groups, uint32_t w, uint32_t h)
+{
+    Pix p;
+    uint32_t pix = i / groups;
+    p.c = (i - pix * groups) * 8;
+    const uint32_t row = pix / w;
+    p.x = pix - row * w;
+    p.b = row / h;
+    p.y = row - p.b * h;
+    return p;
+}
+
+#define GRID_STRIDE32(i, n) \
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += gridDim.x * blockDim.x)
+
+// 2x2 average pool, NHWC
+__global__ void k_pool(uint32_t n8, const bf16 *__restrict__ in, bf16 *__restrict__ out, int H, int W, int C)
+{
+    GRID_STRIDE32(i, n8) {
+        const Pix p = split8(i, C / 8, W / 2, H / 2);
+        const bf16 *s = in + (((size_t)p.b * H + 2 * p.y) * W + 2 * p.x) * C + p.c;
+        const Vec8 a = load8(s), b = load8(s + C), c = load8(s + (size_t)W * C), d = load8(s + (size_t)W * C + C);
+        Vec8 r;
+#pragma unroll
+        for (int k = 0; k < 8; k++) r.v[k] = 0.25f * (a.v[k] + b.v[k] + c.v[k] + d.v[k]);
+        store8(out + (size_t)i * 8, r);
     }
 }
 
-// pool backward: d_in[2y+i][2x+j] (+)= d_out[y][x] / 4 ; accumulate into an FP32 buffer
-__global__ void k_pool_grad(const float *__restrict__ dout, float *__restrict__ din, int B, int H, int W, int C)
+// pool backward: d_in[2y+i][2x+j] += d_out[y][x] / 4 in an FP32 buffer
+__global__ void k_pool_grad(uint32_t n8, const float *__restrict__ dout, float *__restrict__ din, int H, int W, int C)
 {
-    const size_t n = (size_t)B * H * W * C;  // over the full-resolution gradient
-    GRID_STRIDE(i, n) {
-        const int c = (int)(i % C);
-        const size_t pix = i / C;
-        const int x = (int)(pix % W), y = (int)((pix / W) % H);
-        const size_t b = pix / ((size_t)W * H);
-        din[i] += 0.25f * dout[((b * (H / 2) + y / 2) * (W / 2) + x / 2) * C + c];
+    GRID_STRIDE32(i, n8) {  // over the full-resolution gradient
+        const Pix p = split8(i, C / 8, W, H);
+        const Vec8 g = load8(dout + (((size_t)p.b * (H / 2) + p.y / 2) * (W / 2) + p.x / 2) * C + p.c);
+        Vec8 r = load8(din + (size_t)i * 8);
+#pragma unroll
+        for (int k = 0; k < 8; k++) r.v[k] += 0.25f * g.v[k];
+        store8(din + (size_t)i * 8, r);
     }
 }
 
 // out = up2(low) + skip  (nearest), NHWC bf16
-__global__ void k_up_add(const bf16 *__restrict__ low, const bf16 *__restrict__ skip, bf16 *__restrict__ out, int B,
-                         int H, int W, int C)
+__global__ void k_up_add(uint32_t n8, const bf16 *__restrict__ low, const bf16 *__restrict__ skip,
+                         bf16 *__restrict__ out, int H, int W, int C)
 {
-    const size_t n = (size_t)B * H * W * C;
-    GRID_STRIDE(i, n) {
-        const int c = (int)(i % C);
-        const size_t pix = i / C;
-        const int x = (int)(pix % W), y = (int)((pix / W) % H);
-        const size_t b = pix / ((size_t)W * H);
-        out[i] = __float2bfloat16(__bfloat162float(low[((b * (H / 2) + y / 2) * (W / 2) + x / 2) * C + c]) +
-                                  __bfloat162float(skip[i]));
+    GRID_STRIDE32(i, n8) {
+        const Pix p = split8(i, C / 8, W, H);
+        const Vec8 l = load8(low + (((size_t)p.b * (H / 2) + p.y / 2) * (W / 2) + p.x / 2) * C + p.c);
+        Vec8 r = load8(skip + (size_t)i * 8);
+#pragma unroll
+        for (int k = 0; k < 8; k++) r.v[k] += l.v[k];
+        store8(out + (size_t)i * 8, r);
     }
 }
 
 // up backward into the low-resolution FP32 gradient: d_low[y][x] = sum of the 2x2 block
-__global__ void k_up_grad(const float *__restrict__ dout, float *__restrict__ dlow, int B, int H, int W, int C)
+__global__ void k_up_grad(uint32_t n8, const float *__restrict__ dout, float *__restrict__ dlow, int H, int W, int C)
 {
-    const int h = H / 2, w = W / 2;
-    const size_t n = (size_t)B * h * w * C;
-    GRID_STRIDE(i, n) {
-        const int c = (int)(i % C);
-        const size_t pix = i / C;
-        const int x = (int)(pix % w), y = (int)((pix / w) % h);
-        const size_t b = pix / ((size_t)w * h);
-        const float *s = dout + ((b * H + 2 * y) * W + 2 * x) * C + c;
-        dlow[i] = s[0] + s[C] + s[(size_t)W * C] + s[(size_t)W * C + C];
+    GRID_STRIDE32(i, n8) {
+        const Pix p = split8(i, C / 8, W / 2, H / 2);
+        const float *s = dout + (((size_t)p.b * H + 2 * p.y) * W + 2 * p.x) * C + p.c;
+        const Vec8 a = load8(s), b = load8(s + C), c = load8(s + (size_t)W * C), d = load8(s + (size_t)W * C + C);
+        Vec8 r;
+#pragma unroll
+        for (int k = 0; k < 8; k++) r.v[k] = a.v[k] + b.v[k] + c.v[k] + d.v[k];
+        store8(dlow + (size_t)i * 8, r);
     }
 }
 
 // dz = dy * (y > 0) as bf16 (y = the layer's ReLU output), dy FP32
-__global__ void k_relu_grad(const float *__restrict__ dy, const bf16 *__restrict__ y, bf16 *__restrict__ dz, size_t n)
+__global__ void k_relu_grad(uint32_t n8, const float *__restrict__ dy, const bf16 *__restrict__ y, bf16 *__restrict__ dz)
 {
-    GRID_STRIDE(i, n) dz[i] = __float2bfloat16(__bfloat162float(y[i]) > 0.f ? dy[i] : 0.f);
+    GRID_STRIDE32(i, n8) {
+        const Vec8 a = load8(y + (size_t)i * 8);
+        Vec8 r = load8(dy + (size_t)i * 8);
+#pragma unroll
+        for (int k = 0; k < 8; k++) r.v[k] = a.v[k] > 0.f ? r.v[k] : 0.f;
+        store8(dz + (size_t)i * 8, r);
+    }
 }
 
-__global__ void k_bf16_to_f32_add(const bf16 *__restrict__ a, float *__restrict__ out, size_t n)
+// db[c] += sum_p dz[p][c]: eight channels per thread, a block's sums meet in shared memory
+// (256 % (C / 8) == 0)
+__global__ void __launch_bounds__(256) k_bias_grad(const bf16 *__restrict__ dz, float *__restrict__ db, uint32_t npix,
+                                                   int C)
 {
-    GRID_STRIDE(i, n) out[i] += __bfloat162float(a[i]);
-}
-
-__global__ void k_f32_to_bf16(const float *__restrict__ a, bf16 *__restrict__ out, size_t n)
-{
-    GRID_STRIDE(i, n) out[i] = __float2bfloat16(a[i]);
-}
-
-// db[c] += sum_p dz[p][c]
-__global__ void k_bias_grad(const bf16 *__restrict__ dz, float *__restrict__ db, size_t npix, int C)
-{
-    const int c = threadIdx.x % C, lane_group = threadIdx.x / C, groups = blockDim.x / C;
-    float acc = 0.f;
-    for (size_t p = (size_t)blockIdx.x * groups + lane_group; p < npix; p += (size_t)gridDim.x * groups)
-        acc += __bfloat162float(dz[p * C + c]);
-    atomicAdd(db + c, acc);
+    __shared__ float sums[256];
+    const uint32_t groups = C / 8, g = threadIdx.x % groups, first = threadIdx.x / groups, step = 256 / groups;
+    if (threadIdx.x < (uint32_t)C) sums[threadIdx.x] = 0.f;
+    __syncthreads();
+    Vec8 acc = {};
+    for (uint32_t p = blockIdx.x * step + first; p < npix; p += gridDim.x * step) {
+        const Vec8 v = load8(dz + (size_t)p * C + g * 8);
+#pragma unroll
+        for (int k = 0; k < 8; k++) acc.v[k] += v.v[k];
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++) atomicAdd(&sums[g * 8 + k], acc.v[k]);
+    __syncthreads();
+    if (threadIdx.x < (uint32_t)C) atomicAdd(db + threadIdx.x, sums[threadIdx.x]);
 }
 
 // loss = mean (pred - target)^2 ; d_pred = 2 (pred - target) / n
@@ -202,7 +275,13 @@ __global__ void k_mse(const float *__restrict__ pred, const float *__restrict__ 
         acc += (double)d * d;
     }
     for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, acc / (double)n);
+    __shared__ double part[8];  // 256 threads
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {  // one atomic per block: all of them meet in one word
+        for (int k = 1; k < 8; k++) acc += part[k];
+        atomicAdd(loss, acc / (double)n);
+    }
 }
 
 // Adam on FP32 master weights; writes the BF16 forward weights [Cout][9][Cin]
@@ -321,6 +400,15 @@ static ufob_status cnn_workspace(ufob_cnn *c, int B, int H, int W)
         note_launch();                                                     \
     } while (0)
 
+// the same for kernels of eight elements per thread
+#define LAUNCH8(kernel, n, ...)                                                          \
+    do {                                                                                 \
+        const uint32_t n8_ = (uint32_t)((n) / 8);                                        \
+        kernel<<<blocks_for(n8_), 256, 0, s>>>(n8_, __VA_ARGS__);                        \
+        UFOB_CUDA_TRY(cudaGetLastError());                                               \
+        note_launch();                                                                   \
+    } while (0)
+
 static ufob_status cnn_forward(ufob_cnn *c, const float *fbp, float *out, int B, int H2, int W2, cudaStream_t s)
 {
     const int H = H2 / kS, W = W2 / kS;
@@ -331,45 +419,48 @@ static ufob_status cnn_forward(ufob_cnn *c, const float *fbp, float *out, int B,
     LAUNCH(k_unshuffle_in, P0, fbp, bw(c->x0), B, H, W, 1.f / c->scale);
     UFOB_TRY(conv3x3_launch(bw(c->x0), L[0].wf.as<bf16>(), L[0].b.as<float>(), nullptr, bw(c->e1), nullptr, B, H, W, 16,
                             32, 1, s));
-    LAUNCH(k_pool, P0 / 4 * 32, bw(c->e1), bw(c->p1), B, H, W, 32);
+    LAUNCH8(k_pool, P0 / 4 * 32, bw(c->e1), bw(c->p1), H, W, 32);
     UFOB_TRY(conv3x3_launch(bw(c->p1), L[1].wf.as<bf16>(), L[1].b.as<float>(), nullptr, bw(c->e2), nullptr, B, H / 2,
                             W / 2, 32, 64, 1, s));
-    LAUNCH(k_pool, P0 / 16 * 64, bw(c->e2), bw(c->p2), B, H / 2, W / 2, 64);
+    LAUNCH8(k_pool, P0 / 16 * 64, bw(c->e2), bw(c->p2), H / 2, W / 2, 64);
     UFOB_TRY(conv3x3_launch(bw(c->p2), L[2].wf.as<bf16>(), L[2].b.as<float>(), nullptr, bw(c->e3), nullptr, B, H / 4,
                             W / 4, 64, 128, 1, s));
-    LAUNCH(k_pool, P0 / 64 * 128, bw(c->e3), bw(c->p3), B, H / 4, W / 4, 128);
+    LAUNCH8(k_pool, P0 / 64 * 128, bw(c->e3), bw(c->p3), H / 4, W / 4, 128);
     UFOB_TRY(conv3x3_launch(bw(c->p3), L[3].wf.as<bf16>(), L[3].b.as<float>(), nullptr, bw(c->e4), nullptr, B, H / 8,
                             W / 8, 128, 256, 1, s));
     UFOB_TRY(conv3x3_launch(bw(c->e4), L[4].wf.as<bf16>(), L[4].b.as<float>(), nullptr, bw(c->d3), nullptr, B, H / 8,
                             W / 8, 256, 128, 1, s));
-    LAUNCH(k_up_add, P0 / 16 * 128, bw(c->d3), bw(c->e3), bw(c->u3), B, H / 4, W / 4, 128);
+    LAUNCH8(k_up_add, P0 / 16 * 128, bw(c->d3), bw(c->e3), bw(c->u3), H / 4, W / 4, 128);
     UFOB_TRY(conv3x3_launch(bw(c->u3), L[5].wf.as<bf16>(), L[5].b.as<float>(), nullptr, bw(c->d2), nullptr, B, H / 4,
                             W / 4, 128, 64, 1, s));
-    LAUNCH(k_up_add, P0 / 4 * 64, bw(c->d2), bw(c->e2), bw(c->u2), B, H / 2, W / 2, 64);
+    LAUNCH8(k_up_add, P0 / 4 * 64, bw(c->d2), bw(c->e2), bw(c->u2), H / 2, W / 2, 64);
     UFOB_TRY(conv3x3_launch(bw(c->u2), L[6].wf.as<bf16>(), L[6].b.as<float>(), nullptr, bw(c->d1), nullptr, B, H / 2,
                             W / 2, 64, 32, 1, s));
-    LAUNCH(k_up_add, P0 * 32, bw(c->d1), bw(c->e1), bw(c->u1), B, H, W, 32);
+    LAUNCH8(k_up_add, P0 * 32, bw(c->d1), bw(c->e1), bw(c->u1), H, W, 32);
     UFOB_TRY(conv3x3_launch(bw(c->u1), L[7].wf.as<bf16>(), L[7].b.as<float>(), nullptr, nullptr, c->o.as<float>(), B, H,
                             W, 32, 16, 0, s));
-    LAUNCH(k_shuffle_out, P0 * kS * kS, c->o.as<float>(), fbp, out, B, H, W, c->scale);
+    LAUNCH(k_shuffle_out, P0 * kS, c->o.as<float>(), fbp, out, (uint32_t)(P0 * kS), W, c->scale);
     return UFOB_OK;
 }
 
-// Backward of one conv layer: dy (FP32, at the layer output) -> dz (bf16, masked by ReLU),
+// Blocks of the bias gradient: eight per SM, each with a few sweeps of its 256 threads' pixels.
+static unsigned bias_blocks(size_t npix, int C)
+{
+    const size_t sweep = 256 / (C / 8);
+    return (unsigned)std::max<size_t>(1, std::min<size_t>((size_t)num_sms() * 8, npix / (sweep * 4)));
+}
+
+// Backward of one conv layer with a ReLU: dy (FP32, at the layer output) -> dz (bf16, masked by ReLU),
 // weight/bias gradients, and optionally dx (FP32) via the data-gradient convolution.
 static ufob_status conv_backward(ufob_cnn *c, Layer &l, const bf16 *x, const bf16 *y, const float *dy, float *dx,
                                  int B, int H, int W, cudaStream_t s)
 {
     const size_t n = (size_t)B * H * W * l.cout;
     bf16 *dz = c->dz.as<bf16>();
-    if (l.relu) {
-        LAUNCH(k_relu_grad, n, dy, y, dz, n);
-    } else {
-        LAUNCH(k_f32_to_bf16, n, dy, dz, n);
-    }
+    LAUNCH8(k_relu_grad, n, dy, y, dz);
     UFOB_TRY(conv3x3_wgrad_launch(x, dz, l.gw.as<float>(), B, H, W, l.cin, l.cout, s));
-    const int threads = 256 / l.cout * l.cout;
-    k_bias_grad<<<num_sms() * 2, threads, 0, s>>>(dz, l.gb.as<float>(), (size_t)B * H * W, l.cout);
+    k_bias_grad<<<bias_blocks((size_t)B * H * W, l.cout), 256, 0, s>>>(dz, l.gb.as<float>(), (uint32_t)(B * H * W),
+                                                                      l.cout);
     UFOB_CUDA_TRY(cudaGetLastError());
     note_launch();
     if (dx) UFOB_TRY(conv3x3_launch(dz, l.wd.as<bf16>(), nullptr, nullptr, nullptr, dx, B, H, W, l.cout, l.cin, 0, s));
@@ -383,31 +474,30 @@ static ufob_status cnn_backward(ufob_cnn *c, int B, cudaStream_t s)
     auto bw = [&](DevBuf &d) { return d.as<bf16>(); };
     Layer *L = c->L;
     float *ga = c->g_a.as<float>(), *gb = c->g_b.as<float>(), *gc = c->g_c.as<float>();
+    float *g1 = c->g_e1.as<float>(), *g2 = c->g_e2.as<float>(), *g3 = c->g_e3.as<float>();
     bf16 *dzo = c->dz.as<bf16>();
     // out layer: gradient at o from d_pred
     LAUNCH(k_shuffle_out_grad, P0, c->dpred.as<float>(), dzo, B, H, W, c->scale);
     UFOB_TRY(conv3x3_wgrad_launch(bw(c->u1), dzo, L[7].gw.as<float>(), B, H, W, 32, 16, s));
-    k_bias_grad<<<num_sms() * 2, 256, 0, s>>>(dzo, L[7].gb.as<float>(), P0, 16);
+    k_bias_grad<<<bias_blocks(P0, 16), 256, 0, s>>>(dzo, L[7].gb.as<float>(), (uint32_t)P0, 16);
     UFOB_CUDA_TRY(cudaGetLastError());
-    UFOB_TRY(conv3x3_launch(dzo, L[7].wd.as<bf16>(), nullptr, nullptr, nullptr, ga, B, H, W, 16, 32, 0, s));  // d u1
-    // u1 = up(d1) + e1
-    UFOB_CUDA_TRY(cudaMemcpyAsync(c->g_e1.ptr, ga, P0 * 32 * 4, cudaMemcpyDeviceToDevice, s));
-    LAUNCH(k_up_grad, P0 / 4 * 32, ga, gb, B, H, W, 32);  // d d1
-    UFOB_TRY(conv_backward(c, L[6], bw(c->u2), bw(c->d1), gb, ga, B, H / 2, W / 2, s));  // d u2 -> ga
-    UFOB_CUDA_TRY(cudaMemcpyAsync(c->g_e2.ptr, ga, P0 / 4 * 64 * 4, cudaMemcpyDeviceToDevice, s));
-    LAUNCH(k_up_grad, P0 / 16 * 64, ga, gb, B, H / 2, W / 2, 64);  // d d2
-    UFOB_TRY(conv_backward(c, L[5], bw(c->u3), bw(c->d2), gb, ga, B, H / 4, W / 4, s));  // d u3
-    UFOB_CUDA_TRY(cudaMemcpyAsync(c->g_e3.ptr, ga, P0 / 16 * 128 * 4, cudaMemcpyDeviceToDevice, s));
-    LAUNCH(k_up_grad, P0 / 64 * 128, ga, gb, B, H / 4, W / 4, 128);  // d d3
+    note_launch();
+    UFOB_TRY(conv3x3_launch(dzo, L[7].wd.as<bf16>(), nullptr, nullptr, nullptr, g1, B, H, W, 16, 32, 0, s));  // d u1
+    // u1 = up(d1) + e1: d u1 is the skip part of d e1 (likewise u2, u3)
+    LAUNCH8(k_up_grad, P0 / 4 * 32, g1, gb, H, W, 32);  // d d1
+    UFOB_TRY(conv_backward(c, L[6], bw(c->u2), bw(c->d1), gb, g2, B, H / 2, W / 2, s));  // d u2
+    LAUNCH8(k_up_grad, P0 / 16 * 64, g2, gb, H / 2, W / 2, 64);  // d d2
+    UFOB_TRY(conv_backward(c, L[5], bw(c->u3), bw(c->d2), gb, g3, B, H / 4, W / 4, s));  // d u3
+    LAUNCH8(k_up_grad, P0 / 64 * 128, g3, gb, H / 4, W / 4, 128);  // d d3
     UFOB_TRY(conv_backward(c, L[4], bw(c->e4), bw(c->d3), gb, ga, B, H / 8, W / 8, s));  // d e4
     UFOB_TRY(conv_backward(c, L[3], bw(c->p3), bw(c->e4), ga, gb, B, H / 8, W / 8, s));  // d p3
     // e3 gradient = skip part + pool backward of d p3
-    LAUNCH(k_pool_grad, P0 / 16 * 128, gb, c->g_e3.as<float>(), B, H / 4, W / 4, 128);
-    UFOB_TRY(conv_backward(c, L[2], bw(c->p2), bw(c->e3), c->g_e3.as<float>(), gc, B, H / 4, W / 4, s));  // d p2
-    LAUNCH(k_pool_grad, P0 / 4 * 64, gc, c->g_e2.as<float>(), B, H / 2, W / 2, 64);
-    UFOB_TRY(conv_backward(c, L[1], bw(c->p1), bw(c->e2), c->g_e2.as<float>(), gc, B, H / 2, W / 2, s));  // d p1
-    LAUNCH(k_pool_grad, P0 * 32, gc, c->g_e1.as<float>(), B, H, W, 32);
-    UFOB_TRY(conv_backward(c, L[0], bw(c->x0), bw(c->e1), c->g_e1.as<float>(), nullptr, B, H, W, s));
+    LAUNCH8(k_pool_grad, P0 / 16 * 128, gb, g3, H / 4, W / 4, 128);
+    UFOB_TRY(conv_backward(c, L[2], bw(c->p2), bw(c->e3), g3, gc, B, H / 4, W / 4, s));  // d p2
+    LAUNCH8(k_pool_grad, P0 / 4 * 64, gc, g2, H / 2, W / 2, 64);
+    UFOB_TRY(conv_backward(c, L[1], bw(c->p1), bw(c->e2), g2, gc, B, H / 2, W / 2, s));  // d p1
+    LAUNCH8(k_pool_grad, P0 * 32, gc, g1, H, W, 32);
+    UFOB_TRY(conv_backward(c, L[0], bw(c->x0), bw(c->e1), g1, nullptr, B, H, W, s));
     return UFOB_OK;
 }
 
@@ -514,7 +604,10 @@ extern "C" ufob_status ufob_cnn_train_step(ufob_cnn *c, const float *d_fbp, cons
     UFOB_TRY(cnn_forward(c, d_fbp, c->pred.as<float>(), B, H, W, s));
     const size_t n = (size_t)B * H * W;
     UFOB_CUDA_TRY(cudaMemsetAsync(c->loss.ptr, 0, sizeof(double), s));
-    LAUNCH(k_mse, n, c->pred.as<float>(), d_target, c->dpred.as<float>(), c->loss.as<double>(), n);
+    k_mse<<<std::min(blocks_for(n), (unsigned)num_sms() * 8), 256, 0, s>>>(c->pred.as<float>(), d_target,
+                                                                          c->dpred.as<float>(), c->loss.as<double>(), n);
+    UFOB_CUDA_TRY(cudaGetLastError());
+    note_launch();
     for (auto &l : c->L) {
         UFOB_CUDA_TRY(cudaMemsetAsync(l.gw.ptr, 0, l.nw() * 4, s));
         UFOB_CUDA_TRY(cudaMemsetAsync(l.gb.ptr, 0, l.cout * 4, s));
