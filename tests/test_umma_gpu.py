@@ -101,3 +101,17 @@ def test_nonfinite_bins_stay_local(cuda, bad):
     assert np.isfinite(got[~near]).all()
     # the flagged rows are sampled with FP32 weights, the others with 11-bit ones
     assert oracle.rel_l2(got[~near], clean[~near]) < TOL
+
+
+# the host pipeline makes large images in bands of rows: the same bits as one launch, whole chunks
+# and a last chunk of few slices (which the slice-quad kernel takes)
+@pytest.mark.parametrize("nz,chunk", [(20, 32), (70, 32), (64, 64)])
+def test_host_bands(cuda, nz, chunk):
+    P, W = 20, 1030
+    raw = torch.randn(nz, P, W)
+    f = ufob.FBP(filter_props={"size_x": 2048, "crop_width": W}, storage=ufob.F16)
+    got = f.process_host(raw.pin_memory(), out=torch.empty(nz, W, W).pin_memory(), slices_per_chunk=chunk)
+    dev = raw.cuda()
+    parts = [f.process(dev[z:z + chunk].contiguous()).cpu() for z in range(0, nz, chunk)]
+    ufob.device_status()
+    assert torch.equal(got, torch.cat(parts))

@@ -54,6 +54,7 @@ namespace {
 
 constexpr int MX = 11, MY = 10;  // pixels of one accumulator
 constexpr int MT = 2;            // accumulators of a CTA, one above the other
+static_assert(MT * MY == kUmmaTileRows, "tile height");
 constexpr int KT = 16;           // taps of one product
 constexpr int KW = 28;           // staged bins: KT + 10 |sin| + 1, rounded up
 constexpr int SA = 2;            // stages of weights
@@ -156,6 +157,7 @@ struct UmmaArgs {
     uint64_t group_pitch;  // cells per octet
     const uint8_t *flags;  // [P] angles with a non-finite value in some slice
     float *out;
+    uint64_t plane;  // output floats between slices
     int *err;
     uint32_t tiles_x, tiles_y, tmem_cols;
     uint32_t one;  // 1, not known to the compiler: keeps the weights' sums off the busier ALU pipe
@@ -397,7 +399,7 @@ __global__ void __launch_bounds__(kThreads, KA <= 2 ? 4 : 2)
         // results: a pixel of each accumulator per thread, slices along its columns
         tc_fence_after();
         if (__all_sync(0xffffffffu, ok)) {
-            const size_t plane = (size_t)args.roi_w * args.roi_h;
+            const size_t plane = args.plane;
             const bool live = s_live != 0, flagged = s_flagged != 0;
             const uint32_t nz = min(args.ns, args.nz - z0);
             for (int h = 0; h < MT; h++) {
@@ -497,7 +499,7 @@ uint32_t bp_umma_slices(uint32_t nz)
 }
 
 ufob_status bp_umma_launch(const BPGeometry &g, const void *d_sino, uint32_t pitch, uint64_t group_pitch,
-                           const uint8_t *d_flags, float *d_out, cudaStream_t stream)
+                           const uint8_t *d_flags, float *d_out, uint64_t plane, cudaStream_t stream)
 {
     if (!g.roi_w || !g.roi_h || !g.nz || !g.P) return UFOB_OK;
     if ((uintptr_t)d_sino & 15) return fail(UFOB_ERR_INVALID, "backproject: slice-octet base must be 16-byte aligned");
@@ -518,6 +520,7 @@ ufob_status bp_umma_launch(const BPGeometry &g, const void *d_sino, uint32_t pit
     a.group_pitch = group_pitch;
     a.flags = d_flags;
     a.out = d_out;
+    a.plane = plane;
     a.err = device_error_word();
     a.one = 1;
     a.tiles_x = (g.roi_w + MX - 1) / MX;

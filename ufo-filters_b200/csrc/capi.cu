@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <functional>
 #include <string>
 
 #include "ufob_internal.h"
@@ -699,6 +700,7 @@ struct ufob_fbp {
     DevBuf hout[2];     // device staging of host output chunks
     cudaStream_t s_copy = nullptr, s_comp = nullptr, s_d2h = nullptr;  // uploads, compute, downloads
     cudaEvent_t ev_in[2] = {nullptr, nullptr}, ev_done[2] = {nullptr, nullptr}, ev_out[2] = {nullptr, nullptr};
+    cudaEvent_t ev_band = nullptr;
     // optional per-kernel timing: event pairs around every filter / backprojection launch
     bool timing = false;
     std::vector<cudaEvent_t> ev_pool;
@@ -723,6 +725,7 @@ struct ufob_fbp {
             if (ev_done[i]) cudaEventDestroy(ev_done[i]);
             if (ev_out[i]) cudaEventDestroy(ev_out[i]);
         }
+        if (ev_band) cudaEventDestroy(ev_band);
         if (s_copy) cudaStreamDestroy(s_copy);
         if (s_d2h) cudaStreamDestroy(s_d2h);
         if (s_comp) cudaStreamDestroy(s_comp);
@@ -830,7 +833,7 @@ extern "C" ufob_status ufob_stacked_bp_run(ufob_stacked_bp *sb, const float *d_s
         UFOB_TRY(sb->flags.ensure(height));
         UFOB_CUDA_TRY(cudaMemsetAsync(sb->flags.ptr, 0, height, s));
         UFOB_TRY(pack_octs_launch(d_sino, width, height, nslices, sb->work.ptr, sb->flags.as<uint8_t>(), s));
-        return bp_umma_launch(g, sb->work.ptr, width, (uint64_t)width * height, sb->flags.as<uint8_t>(), d_out, s);
+        return bp_umma_launch(g, sb->work.ptr, width, (uint64_t)width * height, sb->flags.as<uint8_t>(), d_out, (uint64_t)g.roi_w * g.roi_h, s);
     }
     if (sb->precision == 1) {  // few slices: FP16 slice-quad cells, FP32 sums
         const uint32_t cells = width + 1;
@@ -855,8 +858,11 @@ extern "C" void ufob_stacked_bp_destroy(ufob_stacked_bp *sb)
 
 // Filter + backproject `nz` slices already on the device; logical row
 // slice * height + angle of `src` is sinogram row `angle` of slice `slice`.
+// With `bands`, the image is made in up to `bands` bands of rows (where the backprojector can write
+// them in place) and done(first row, rows) is called after each band's work is on the stream.
 static ufob_status fbp_group(ufob_fbp *x, const RowSource &src, uint32_t width, uint32_t height, uint32_t nz,
-                             float *d_out, cudaStream_t s)
+                             float *d_out, cudaStream_t s, uint32_t bands = 1,
+                             const std::function<ufob_status(uint32_t, uint32_t)> &done = nullptr)
 {
     uint32_t nfft, fw;
     UFOB_TRY(filter_sizes(x->f->props, width, &nfft, &fw));
@@ -894,10 +900,21 @@ static ufob_status fbp_group(ufob_fbp *x, const RowSource &src, uint32_t width, 
     if (umma) {
         BPGeometry g;
         UFOB_TRY(bp_prepare(x->bp, fw, height, nz, g, s));
-        UFOB_TRY(bp_umma_launch(g, x->work.ptr, pitch, (uint64_t)pitch * height, x->flags.as<uint8_t>(), d_out, s));
+        // whole tile rows per band: the same tiles, and the same results, as in one launch
+        const uint32_t oh = g.roi_h, y0 = g.roi_y, rows = round_up((oh + bands - 1) / bands, kUmmaTileRows);
+        for (uint32_t y = 0; y < oh; y += rows) {
+            g.roi_y = y0 + y;
+            g.roi_h = std::min(rows, oh - y);
+            UFOB_TRY(bp_umma_launch(g, x->work.ptr, pitch, (uint64_t)pitch * height, x->flags.as<uint8_t>(),
+                                    d_out + (size_t)y * g.roi_w, (uint64_t)g.roi_w * oh, s));
+            if (done) UFOB_TRY(done(y, g.roi_h));
+        }
     } else {
+        uint32_t ow, oh;
         UFOB_TRY(ufob_backproject_run(x->bp, x->work.ptr, x->storage, layout, fw, height, nz, pitch,
                                       (uint64_t)pitch * height, d_out, s));
+        UFOB_TRY(ufob_backproject_get_requisition(x->bp, fw, height, &ow, &oh));
+        if (done) UFOB_TRY(done(0, oh));
     }
     if (x->timing) {
         UFOB_CUDA_TRY(cudaEventRecord(e2, s));
@@ -1011,6 +1028,7 @@ extern "C" ufob_status ufob_fbp_run_host(ufob_fbp *x, const float *h_sino, uint3
         UFOB_CUDA_TRY(cudaStreamCreateWithFlags(&x->s_copy, cudaStreamNonBlocking));
         UFOB_CUDA_TRY(cudaStreamCreateWithFlags(&x->s_d2h, cudaStreamNonBlocking));
         UFOB_CUDA_TRY(cudaStreamCreateWithFlags(&x->s_comp, cudaStreamNonBlocking));
+        UFOB_CUDA_TRY(cudaEventCreateWithFlags(&x->ev_band, cudaEventDisableTiming));
         for (int i = 0; i < 2; i++) {
             UFOB_CUDA_TRY(cudaEventCreateWithFlags(&x->ev_in[i], cudaEventDisableTiming));
             UFOB_CUDA_TRY(cudaEventCreateWithFlags(&x->ev_done[i], cudaEventDisableTiming));
@@ -1025,8 +1043,14 @@ extern "C" ufob_status ufob_fbp_run_host(ufob_fbp *x, const float *h_sino, uint3
     // Pipeline: H2D(c) on the upload stream -> filter+BP(c) on the compute stream -> D2H(c) on the download
     // stream, double-buffered so chunk c+1's upload and chunk c-1's download overlap chunk c's compute.
     // Chunk sizes: a short first chunk (compute starts after a small upload) and a short last one
-    // (little download left after the last compute), `chunk` slices in between.
-    const uint32_t edge = chunk >= 32 ? 16 : 0;
+    // (little download left after the last compute), `chunk` slices in between.  On the tensor cores
+    // 16 slices take as long as 32 (and 64 hardly longer), so there all chunks are whole, and a chunk's
+    // image is downloaded in four bands of rows while the next band is computed: 32 slices of
+    // 2048^2 x 1500 angles 40.0 -> 25.6 ms.
+    const bool umma = x->storage == UFOB_F16 && umma_applies(x->bp->props, chunk);
+    const uint32_t edge = chunk >= 32 && !umma ? 16 : 0;
+    // at least two waves of CTAs (four per SM) in every band
+    const uint32_t bands = std::max(1u, std::min(4u, (ow / 11) * (oh / kUmmaTileRows) / (8 * (uint32_t)num_sms())));
     auto chunk_at = [&](uint32_t z) -> uint32_t {
         const uint32_t rest = nslices - z;
         if (edge && z == 0 && nslices >= chunk + 2 * edge) return edge;
@@ -1044,12 +1068,28 @@ extern "C" ufob_status ufob_fbp_run_host(ufob_fbp *x, const float *h_sino, uint3
         UFOB_CUDA_TRY(cudaEventRecord(x->ev_in[b], x->s_copy));
         UFOB_CUDA_TRY(cudaStreamWaitEvent(x->s_comp, x->ev_in[b], 0));
         if (c >= 2) UFOB_CUDA_TRY(cudaStreamWaitEvent(x->s_comp, x->ev_out[b], 0));  // hout[b] downloaded
+        const size_t plane = (size_t)ow * oh * 4;
         UFOB_TRY(fbp_group(x, plain_rows(x->hin[b].as<float>(), width), width, height, nz, x->hout[b].as<float>(),
-                           x->s_comp));
+                           x->s_comp, bands, [&](uint32_t y, uint32_t rows) -> ufob_status {
+                               // a wait takes the event as recorded last, so one event serves all bands
+                               UFOB_CUDA_TRY(cudaEventRecord(x->ev_band, x->s_comp));
+                               UFOB_CUDA_TRY(cudaStreamWaitEvent(x->s_d2h, x->ev_band, 0));
+                               const size_t off = (size_t)y * ow * 4, bytes = (size_t)rows * ow * 4;
+                               char *dst = (char *)(h_out + (size_t)z * ow * oh) + off;
+                               if (rows == oh)
+                                   UFOB_CUDA_TRY(cudaMemcpyAsync(dst, x->hout[b].ptr, nz * plane,
+                                                                 cudaMemcpyDeviceToHost, x->s_d2h));
+                               else if (plane >> 31)  // past the largest pitch
+                                   for (uint32_t i = 0; i < nz; i++)
+                                       UFOB_CUDA_TRY(cudaMemcpyAsync(dst + i * plane,
+                                                                     x->hout[b].as<char>() + off + i * plane, bytes,
+                                                                     cudaMemcpyDeviceToHost, x->s_d2h));
+                               else
+                                   UFOB_CUDA_TRY(cudaMemcpy2DAsync(dst, plane, x->hout[b].as<char>() + off, plane,
+                                                                   bytes, nz, cudaMemcpyDeviceToHost, x->s_d2h));
+                               return UFOB_OK;
+                           }));
         UFOB_CUDA_TRY(cudaEventRecord(x->ev_done[b], x->s_comp));
-        UFOB_CUDA_TRY(cudaStreamWaitEvent(x->s_d2h, x->ev_done[b], 0));
-        UFOB_CUDA_TRY(cudaMemcpyAsync(h_out + (size_t)z * ow * oh, x->hout[b].ptr, (size_t)nz * ow * oh * 4,
-                                      cudaMemcpyDeviceToHost, x->s_d2h));
         UFOB_CUDA_TRY(cudaEventRecord(x->ev_out[b], x->s_d2h));
     }
     UFOB_CUDA_TRY(cudaStreamSynchronize(x->s_copy));

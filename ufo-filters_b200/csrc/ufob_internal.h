@@ -275,9 +275,10 @@ ufob_status bp_cells_launch(const BPGeometry &g, const void *d_cells, float *d_o
 ufob_status pack_cells_launch(const float *d_in, uint32_t pitch, uint64_t slice_pitch, uint32_t W, uint32_t P,
                               uint32_t Z, void *d_out, cudaStream_t s);
 // The same on the tensor cores from slice octets [ceil(nz/8)][P][pitch] (pitch and group_pitch in
-// 16-byte cells).
+// 16-byte cells), slices `plane` floats apart in the output.  Its tiles are kUmmaTileRows rows high.
+constexpr uint32_t kUmmaTileRows = 20;
 ufob_status bp_umma_launch(const BPGeometry &g, const void *d_sino, uint32_t pitch, uint64_t group_pitch,
-                           const uint8_t *d_flags, float *d_out, cudaStream_t stream);
+                           const uint8_t *d_flags, float *d_out, uint64_t plane, cudaStream_t stream);
 
 // Kernel arguments of one backprojection (one stack or one batch job).
 struct BPArgs {
