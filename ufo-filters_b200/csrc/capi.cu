@@ -56,6 +56,7 @@ ufob_status DevBuf::ensure(size_t n)
     cudaError_t e = cudaMalloc(&ptr, n);
     if (e != cudaSuccess) {
         ptr = nullptr;
+        cudaGetLastError();  // callers that can do without go on to launch
         return cuda_fail(e, "cudaMalloc");
     }
     g_device_allocs.fetch_add(1, std::memory_order_relaxed);

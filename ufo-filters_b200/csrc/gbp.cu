@@ -34,6 +34,7 @@
 #include <climits>
 #include <cmath>
 #include <string>
+#include <type_traits>
 
 #include "f32x2.cuh"
 #include "tma.cuh"
@@ -206,11 +207,32 @@ __host__ __device__ inline void gbp_table_entry(const double *g, int flags, doub
     for (int i = 0; i < kTab; i++) vals[i] = v[i];
 }
 
+// Sweep of a parallel-beam centre position as a column along z: u (or v) is affine in the centre with
+// factor 1, so the slices' centres, relative to the one in the table, take the place of z and the
+// slices' common z goes into the constants.  For the horizontal centre u and v also change places
+// (over transposed projections), because the column kernel's z moves v.
+enum { SWEEP_NONE = 0, SWEEP_CENTER_X = 1, SWEEP_CENTER_Z = 2 };
+
+__host__ __device__ inline void gbp_sweep_entry(double t[kTab], int sweep, double z)
+{
+    if (sweep == SWEEP_NONE) return;
+    t[3] += t[2] * z;
+    t[7] += t[6] * z;
+    t[2] = sweep == SWEEP_CENTER_X ? 1.0 : 0.0;
+    t[6] = sweep == SWEEP_CENTER_Z ? 1.0 : 0.0;
+    if (sweep == SWEEP_CENTER_X)
+        for (int i = 0; i < 4; i++) {
+            const double u = t[i];
+            t[i] = t[4 + i];
+            t[4 + i] = u;
+        }
+}
+
 // One table entry per (slice-or-0, projection).  geom: [n_proj][GC_NCOLS]
 // FP64; when param_col >= 0 the column is replaced by slice_values[slice].
 __global__ void k_gbp_tables(const double *__restrict__ geom, uint32_t n_proj, uint32_t n_tab_slices, int param_col,
                              const double *__restrict__ slice_values, int flags, double x0, double dxs, double y0,
-                             double dys, float *__restrict__ tf, double *__restrict__ td)
+                             double dys, int sweep, double sweep_z, float *__restrict__ tf, double *__restrict__ td)
 {
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t sl = blockIdx.y;
@@ -220,6 +242,7 @@ __global__ void k_gbp_tables(const double *__restrict__ geom, uint32_t n_proj, u
     if (param_col >= 0) g[param_col] = slice_values[sl];
     double vals[kTab];
     gbp_table_entry(g, flags, x0, dxs, y0, dys, vals);
+    gbp_sweep_entry(vals, sweep, sweep_z);
     const size_t o = ((size_t)sl * n_proj + p) * kTab;
     for (int i = 0; i < kTab; i++) {
         td[o + i] = vals[i];
@@ -499,9 +522,13 @@ __global__ void __launch_bounds__(256) k_gbp(const GBPArgs a)
 // column).  TMA's zero fill outside the detector is the reference's CLAMP
 // addressing.  A projection whose window for the tile exceeds the staged box
 // (where the plan underestimated it) is sampled from global memory instead.
+//
+// Bound by issue (22.9 instructions per update when both rows of every sample were read).  In the
+// affine geometries a voxel's upper row is a row of the voxel before, already interpolated along u:
+// one new row per voxel.  1024 projections of 1024^2 -> 512^2 x 96, tilted by 30 degrees: 24.7 -> 21.1 ms.
 
 struct GBPColArgs {
-    const float *proj;    // [n][H][W]
+    const float *proj;    // [n][H][pitch]
     const float *tab;     // [n][kTab] FP32 tables
     const double *zvals;  // z value of each slice
     uint32_t W, H, n_proj, nx, ny, nz, burst;
@@ -509,6 +536,7 @@ struct GBPColArgs {
     float norm;
     float *vol;
     int *err;
+    uint32_t pitch;  // floats between detector rows (last: among the sizes above, the cone kernel ran 1.4% slower)
 };
 
 template <int PB, int S>
@@ -548,14 +576,27 @@ __global__ void __launch_bounds__(256, 2) k_gbp_col(const __grid_constant__ CUte
     // a warp covers 16 x 2 columns: its samples of one row then span fewer than 32 banks
     const int ix = x0 + (warp & 1) * 16 + (lane & 15), iy = y0 + (warp >> 1) * 2 + (lane >> 4);
     const float fx = (float)ix, fy = (float)iy;
-    // z of the column's voxels as packed pairs (2j, 2j + 1)
-    uint64_t zz[ZT / 2];
+    // the column's voxels as packed pairs: neighbours for the cone, else (j, j + ZT / 2), so that each
+    // lane walks half of the column
+    constexpr int ZP = ZT / 2, Z0 = CONE ? 2 : 1, Z1 = CONE ? 1 : ZP;  // pair j: voxels Z0 j, Z0 j + Z1
+    uint64_t zz[ZP];
 #pragma unroll
-    for (int j = 0; j < ZT / 2; j++)
-        zz[j] = f2pack((float)c.zvals[min(z0 + 2 * j, (int)c.nz - 1)], (float)c.zvals[min(z0 + 2 * j + 1, (int)c.nz - 1)]);
+    for (int j = 0; j < ZP; j++)
+        zz[j] = f2pack((float)c.zvals[min(z0 + Z0 * j, (int)c.nz - 1)],
+                       (float)c.zvals[min(z0 + Z0 * j + Z1, (int)c.nz - 1)]);
+    float zstep = 0.f;  // largest step of a walk, with the sign of all of them (z values are equally spaced)
+    if constexpr (!CONE) {
+        float last = (float)c.zvals[min(z0, (int)c.nz - 1)];
+#pragma unroll
+        for (int k = 1; k < ZT; k++) {
+            const float z = (float)c.zvals[min(z0 + k, (int)c.nz - 1)];
+            if (fabsf(z - last) > fabsf(zstep)) zstep = z - last;
+            last = z;
+        }
+    }
     float zlo, zhi, zdummy;
     f2unpack(zz[0], zlo, zdummy);
-    f2unpack(zz[ZT / 2 - 1], zdummy, zhi);
+    f2unpack(zz[ZP - 1], zdummy, zhi);
     if (tid == 0) {
         for (int q = 0; q < S; q++) {
             mbar_init(&sm.full[q], 1);
@@ -645,7 +686,7 @@ __global__ void __launch_bounds__(256, 2) k_gbp_col(const __grid_constant__ CUte
     const float Wf = (float)c.W + 2.0f, Hf = (float)c.H + 2.0f;
     const int bw = (int)c.bw;
     float acc[ZT];
-    uint64_t bsum[ZT / 2];  // burst sums of voxels (2j, 2j + 1)
+    uint64_t bsum[ZT / 2];  // burst sums of the pairs
 #pragma unroll
     for (int k = 0; k < ZT; k++) acc[k] = 0.f;
 #pragma unroll
@@ -695,33 +736,102 @@ __global__ void __launch_bounds__(256, 2) k_gbp_col(const __grid_constant__ CUte
                     const float *col = win + iu;
                     const uint64_t AA = f2pack(a, a), AV = f2pack(Av, Av), BV = f2pack(Bv, Bv);
                     const uint64_t MM = f2pack(M, M), WG = f2pack(wgt, wgt);
+                    if constexpr (CONE) {
+                        // Cone beams magnify about half of a volume to more than a row per voxel, and
+                        // their warps mix both, so both rows of every voxel are read (walking where
+                        // possible was 1% slower).
 #pragma unroll
-                    for (int j = 0; j < ZT / 2; j++) {
+                        for (int j = 0; j < ZP; j++) {
+                            const uint64_t vp = f2fma(AV, zz[j], BV);
+                            const uint64_t rv = f2add_rd(vp, MM);
+                            const uint64_t bb = f2sub(vp, f2sub(rv, MM));
+                            float r0, r1;
+                            f2unpack(rv, r0, r1);
+                            // one unsigned clamp keeps every read inside the window (the plan's guard
+                            // texels already do for every in-range footprint)
+                            const uint32_t i0 = min((uint32_t)(__float_as_int(r0) - vbase), c.bh - 2u);
+                            const uint32_t i1 = min((uint32_t)(__float_as_int(r1) - vbase), c.bh - 2u);
+                            const float *p0 = col + i0 * (uint32_t)bw, *p1 = col + i1 * (uint32_t)bw;
+                            const uint64_t t00 = f2pack(p0[0], p1[0]), t10 = f2pack(p0[1], p1[1]);
+                            const uint64_t t01 = f2pack(p0[bw], p1[bw]), t11 = f2pack(p0[bw + 1], p1[bw + 1]);
+                            const uint64_t top = f2fma(AA, f2sub(t10, t00), t00), bot = f2fma(AA, f2sub(t11, t01), t01);
+                            const uint64_t val = f2fma(bb, f2sub(bot, top), top);
+                            bsum[j] = f2fma(val, WG, bsum[j]);
+                        }
+                    } else {
+                    // row i's two texels of one lane's voxel, interpolated along u
+                    auto rows = [&](const float *base, uint32_t i0, uint32_t i1) {
+                        const float *p0 = base + i0 * (uint32_t)bw, *p1 = base + i1 * (uint32_t)bw;
+                        const uint64_t t0 = f2pack(p0[0], p1[0]), t1 = f2pack(p0[1], p1[1]);
+                        return f2fma(AA, f2sub(t1, t0), t0);
+                    };
+                    // fraction along v of pair j, and its rows; one unsigned clamp keeps every read
+                    // inside the window (the plan's guard texels already do for every in-range footprint)
+                    auto locate = [&](int j, uint32_t &i0, uint32_t &i1) {
                         const uint64_t vp = f2fma(AV, zz[j], BV);
                         const uint64_t rv = f2add_rd(vp, MM);
-                        const uint64_t bb = f2sub(vp, f2sub(rv, MM));
                         float r0, r1;
                         f2unpack(rv, r0, r1);
-                        // one unsigned clamp keeps every read inside the window (the plan's guard
-                        // texels already do for every in-range footprint)
-                        const uint32_t i0 = min((uint32_t)(__float_as_int(r0) - vbase), c.bh - 2u);
-                        const uint32_t i1 = min((uint32_t)(__float_as_int(r1) - vbase), c.bh - 2u);
-                        const float *p0 = col + i0 * (uint32_t)bw, *p1 = col + i1 * (uint32_t)bw;
-                        const uint64_t t00 = f2pack(p0[0], p1[0]), t10 = f2pack(p0[1], p1[1]);
-                        const uint64_t t01 = f2pack(p0[bw], p1[bw]), t11 = f2pack(p0[bw + 1], p1[bw + 1]);
-                        const uint64_t top = f2fma(AA, f2sub(t10, t00), t00), bot = f2fma(AA, f2sub(t11, t01), t01);
+                        i0 = min((uint32_t)(__float_as_int(r0) - vbase), c.bh - 2u);
+                        i1 = min((uint32_t)(__float_as_int(r1) - vbase), c.bh - 2u);
+                        return f2sub(vp, f2sub(rv, MM));
+                    };
+                    auto add = [&](int j, uint64_t bb, uint64_t top, uint64_t bot) {
                         const uint64_t val = f2fma(bb, f2sub(bot, top), top);
-                        bsum[j] = CONE ? f2fma(val, WG, bsum[j]) : f2add(bsum[j], val);
+                        bsum[j] = f2add(bsum[j], val);
+                    };
+                    // Where v moves by less than a row from voxel to voxel (0.99: rounding), a walk in
+                    // the direction of growing v reads one new row per voxel: its upper row is the
+                    // upper or the lower one of the voxel before.
+                    auto walk = [&](auto down) {
+                        uint64_t top = 0, bot = 0;
+                        uint32_t l0 = 0, l1 = 0;
+#pragma unroll
+                        for (int i = 0; i < ZP; i++) {
+                            const int j = decltype(down)::value ? ZP - 1 - i : i;
+                            uint32_t i0, i1;
+                            const uint64_t bb = locate(j, i0, i1);
+                            if (i == 0) {
+                                top = rows(col, i0, i1);
+                            } else {
+                                float t0, t1, b0, b1;
+                                f2unpack(top, t0, t1);
+                                f2unpack(bot, b0, b1);
+                                top = f2pack(i0 != l0 ? b0 : t0, i1 != l1 ? b1 : t1);
+                            }
+                            bot = rows(col + bw, i0, i1);
+                            l0 = i0;
+                            l1 = i1;
+                            add(j, bb, top, bot);
+                        }
+                    };
+                    const float vstep = Av * zstep;
+                    if (__all_sync(__activemask(), vstep >= 0.f && vstep < 0.99f)) {
+                        walk(std::false_type());
+                    } else if (__all_sync(__activemask(), vstep <= 0.f && vstep > -0.99f)) {
+                        walk(std::true_type());
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < ZP; j++) {
+                            uint32_t i0, i1;
+                            const uint64_t bb = locate(j, i0, i1);
+                            const float *p0 = col + i0 * (uint32_t)bw, *p1 = col + i1 * (uint32_t)bw;
+                            const uint64_t t00 = f2pack(p0[0], p1[0]), t10 = f2pack(p0[1], p1[1]);
+                            const uint64_t t01 = f2pack(p0[bw], p1[bw]), t11 = f2pack(p0[bw + 1], p1[bw + 1]);
+                            add(j, bb, f2fma(AA, f2sub(t10, t00), t00), f2fma(AA, f2sub(t11, t01), t01));
+                        }
+                    }
                     }
                 } else {
                     // window not staged: the same footprints and weights from global memory
-                    const float *img = c.proj + (size_t)p * c.W * c.H;
+                    const uint32_t pitch = CONE ? c.W : c.pitch;  // only sweeps are padded
+                    const float *img = c.proj + (size_t)p * pitch * c.H;
                     const float u = fminf(fmaxf(uxy * inv, -2.0f), Wf);
                     const float ru = u + M1;
                     const float a = (u + 0.5f) - (ru - M1);
                     const int i0 = __float_as_int(ru) - M1b - 1;
                     auto texel0 = [&](int i, int j) {
-                        return ((unsigned)i < c.W && (unsigned)j < c.H) ? __ldg(img + (size_t)j * c.W + i) : 0.f;
+                        return ((unsigned)i < c.W && (unsigned)j < c.H) ? __ldg(img + (size_t)j * pitch + i) : 0.f;
                     };
                     for (int j = 0; j < ZT / 2; j++) {
                         float zp[2], bs[2];
@@ -746,8 +856,8 @@ __global__ void __launch_bounds__(256, 2) k_gbp_col(const __grid_constant__ CUte
                     for (int j = 0; j < ZT / 2; j++) {
                         float b0, b1;
                         f2unpack(bsum[j], b0, b1);
-                        acc[2 * j] = acc[2 * j] + __fmul_rn(c.norm, b0);
-                        acc[2 * j + 1] = acc[2 * j + 1] + __fmul_rn(c.norm, b1);
+                        acc[Z0 * j] = acc[Z0 * j] + __fmul_rn(c.norm, b0);
+                        acc[Z0 * j + Z1] = acc[Z0 * j + Z1] + __fmul_rn(c.norm, b1);
                         bsum[j] = 0;
                     }
                     in_burst = 0;
@@ -856,7 +966,7 @@ static ufob_status launch_gbp_col_t(const GBPColArgs &c, cudaStream_t s)
     const size_t smem = Sm::bytes(c.slot_floats);
     UFOB_CUDA_TRY(smem_limit_per_device(kern, 227 * 1024, attr_devs));
     CUtensorMap map;
-    UFOB_TRY(make_image_map(&map, c.proj, c.W, c.H, c.n_proj, c.W, (uint64_t)c.W * c.H, c.bw, c.bh));
+    UFOB_TRY(make_image_map(&map, c.proj, c.W, c.H, c.n_proj, c.pitch, (uint64_t)c.pitch * c.H, c.bw, c.bh));
     dim3 grid((c.nx + 31) / 32, (c.ny + 7) / 8, (c.nz + kColZT - 1) / kColZT);
     kern<<<grid, 256, smem, s>>>(map, c);
     UFOB_CUDA_TRY(cudaGetLastError());
@@ -864,13 +974,20 @@ static ufob_status launch_gbp_col_t(const GBPColArgs &c, cudaStream_t s)
     return UFOB_OK;
 }
 
+static constexpr size_t kColBudget = 110 * 1024;  // shared memory of two CTAs per SM
+
+static uint32_t col_slot_floats(const GBPColArgs &c) { return (c.bw * c.bh + 31) / 32 * 32; }  // 128-byte aligned
+
+// Whether the smallest ring of launch_gbp_col holds the window.
+static bool gbp_col_fits(const GBPColArgs &c) { return GBPColSmem<4, 2>::bytes(col_slot_floats(c)) <= kColBudget; }
+
 // Launches the column kernel with a ring that keeps two CTAs per SM; false when the window is too
 // large for that.
 static ufob_status launch_gbp_col(GBPColArgs c, bool cone, bool *launched, cudaStream_t s)
 {
     *launched = false;
-    c.slot_floats = (c.bw * c.bh + 31) / 32 * 32;  // 128-byte aligned TMA destinations
-    constexpr size_t kBudget = 110 * 1024;           // two CTAs per SM
+    c.slot_floats = col_slot_floats(c);
+    constexpr size_t kBudget = kColBudget;
     if (GBPColSmem<8, 3>::bytes(c.slot_floats) <= kBudget) {
         *launched = true;
         return cone ? launch_gbp_col_t<true, 8, 3>(c, s) : launch_gbp_col_t<false, 8, 3>(c, s);
@@ -1049,6 +1166,25 @@ __global__ void k_proj_round_half(const float4 *__restrict__ in, uint64_t n4, fl
         v.w = __half2float(__float2half_rn(v.w));
         out[i] = v;
     }
+}
+
+// [n][H][W] -> [n][W][pitch] (pitch >= H), optionally rounded to FP16 on the way; 32 x 32 tiles
+// through shared memory, both sides in 128-byte rows.
+__global__ void k_proj_transpose(const float *__restrict__ in, uint32_t W, uint32_t H, uint32_t pitch, int half,
+                                 float *__restrict__ out)
+{
+    __shared__ float tile[32][33];
+    const uint32_t x0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
+    const float *src = in + (size_t)blockIdx.z * W * H;
+    float *dst = out + (size_t)blockIdx.z * W * pitch;
+    for (uint32_t r = threadIdx.y; r < 32; r += 8)
+        if (x0 + threadIdx.x < W && y0 + r < H) {
+            const float v = __ldg(src + (size_t)(y0 + r) * W + x0 + threadIdx.x);
+            tile[r][threadIdx.x] = half ? __half2float(__float2half_rn(v)) : v;
+        }
+    __syncthreads();
+    for (uint32_t r = threadIdx.y; r < 32; r += 8)
+        if (y0 + threadIdx.x < H && x0 + r < W) dst[(size_t)(x0 + r) * pitch + y0 + threadIdx.x] = tile[threadIdx.x][r];
 }
 
 // One 2-D texture object per projection of a [n][H][W] stack: FP32 with row
@@ -1271,6 +1407,85 @@ static ufob_status half_projections(ufob_gbp *g, const float *d_proj, uint32_t W
     return UFOB_OK;
 }
 
+// Runs one geometry on the staged column kernel, where its tables and windows allow (*launched).
+// table: [n][GC_NCOLS]; zvals: z of each slice, or the swept centres relative to the table's.
+static ufob_status gbp_staged(ufob_gbp *g, const float *d_proj, uint32_t W, uint32_t H,
+                              const std::vector<double> &table, int flags, double x0, double dxs, double y0, double dys,
+                              uint32_t nx, uint32_t ny, const std::vector<double> &zvals, int sweep, void *d_vol,
+                              bool *launched, cudaStream_t s)
+{
+    const uint32_t n = g->num_projections, nz = (uint32_t)zvals.size();
+    const bool cone = !(flags & GF_PARALLEL), turned = sweep == SWEEP_CENTER_X;
+    const uint32_t dw = turned ? H : W, dh = turned ? W : H, pitch = turned ? round_up(H, 4) : W;
+    // the plan (host FP64 tables, window size) is kept while the geometry stays the same
+    std::vector<double> key(table);
+    key.insert(key.end(), {(double)flags, x0, dxs, y0, dys, (double)nx, (double)ny, (double)W, (double)H, (double)sweep,
+                           g->z});
+    key.insert(key.end(), zvals.begin(), zvals.end());
+    if (key != g->col_key) {
+        std::vector<double> tabs((size_t)n * kTab);
+        for (uint32_t p = 0; p < n; p++) {
+            gbp_table_entry(&table[(size_t)p * GC_NCOLS], flags, x0, dxs, y0, dys, &tabs[(size_t)p * kTab]);
+            gbp_sweep_entry(&tabs[(size_t)p * kTab], sweep, g->z);
+        }
+        g->col_plan = gbp_col_plan(tabs, n, cone, nx, ny, zvals, dw, dh);
+        g->col_key.swap(key);
+    }
+    if (!g->col_plan.ok) return UFOB_OK;
+    GBPColArgs c;
+    c.bw = g->col_plan.bw;
+    c.bh = g->col_plan.bh;
+    if (!gbp_col_fits(c)) return UFOB_OK;
+    UFOB_TRY(g->d_geom.ensure(table.size() * sizeof(double) + nz * sizeof(double)));
+    UFOB_TRY(g->d_zvals.ensure(nz * sizeof(double) * 2));
+    UFOB_TRY(g->d_tab_f.ensure((size_t)n * kTab * sizeof(float)));
+    UFOB_TRY(g->d_tab_d.ensure((size_t)n * kTab * sizeof(double)));
+    UFOB_CUDA_TRY(cudaMemcpyAsync(g->d_geom.ptr, table.data(), table.size() * sizeof(double), cudaMemcpyHostToDevice, s));
+    UFOB_CUDA_TRY(cudaMemcpyAsync(g->d_zvals.ptr, zvals.data(), nz * sizeof(double), cudaMemcpyHostToDevice, s));
+    k_gbp_tables<<<dim3((n + 127) / 128, 1), 128, 0, s>>>(g->d_geom.as<double>(), n, 1, -1, nullptr, flags, x0, dxs, y0,
+                                                          dys, sweep, g->z, g->d_tab_f.as<float>(),
+                                                          g->d_tab_d.as<double>());
+    UFOB_CUDA_TRY(cudaGetLastError());
+    note_launch();
+    const float *src = d_proj;
+    // compute-type half: FP16 samples with FP32 coordinates, weights and sums, the arithmetic of the
+    // FP16 gathers, staged from a rounded FP32 copy
+    const int half = g->compute_type == 2;
+    if (turned) {
+        k_proj_transpose<<<dim3((W + 31) / 32, (H + 31) / 32, n), dim3(32, 8), 0, s>>>(d_proj, W, H, pitch, half,
+                                                                                     g->d_proj_h.as<float>());
+        UFOB_CUDA_TRY(cudaGetLastError());
+        note_launch();
+        src = g->d_proj_h.as<float>();
+    } else if (half) {
+        const uint64_t n4 = (uint64_t)n * H * W / 4;
+        UFOB_TRY(g->d_proj_h.ensure(n4 * 16));
+        if (n4) {
+            const uint32_t grid = (uint32_t)std::min<uint64_t>((n4 + 255) / 256, (uint64_t)num_sms() * 16);
+            k_proj_round_half<<<grid, 256, 0, s>>>(reinterpret_cast<const float4 *>(d_proj), n4,
+                                                   g->d_proj_h.as<float4>());
+            UFOB_CUDA_TRY(cudaGetLastError());
+            note_launch();
+        }
+        src = g->d_proj_h.as<float>();
+    }
+    c.proj = src;
+    c.tab = g->d_tab_f.as<float>();
+    c.zvals = g->d_zvals.as<double>();
+    c.W = dw;
+    c.H = dh;
+    c.pitch = pitch;
+    c.n_proj = n;
+    c.nx = nx;
+    c.ny = ny;
+    c.nz = nz;
+    c.burst = g->burst ? g->burst : 8;  // "GENERIC" entry of the node table (ufo-conebeam.c:21-26)
+    c.norm = (float)(fabs(g->overall_angle) / n);  // :292
+    c.vol = static_cast<float *>(d_vol);
+    c.err = device_error_word();
+    return launch_gbp_col(c, cone, launched, s);
+}
+
 static ufob_status gbp_compute(ufob_gbp *g, const float *d_proj, uint32_t W, uint32_t H, void *d_vol, cudaStream_t s)
 {
     UFOB_TRY(ufob_gbp_setup(g));
@@ -1327,8 +1542,35 @@ static ufob_status gbp_compute(ufob_gbp *g, const float *d_proj, uint32_t W, uin
     std::vector<double> slice_values(nz);
     for (uint32_t k = 0; k < nz; k++) slice_values[k] = rs + k * rstep;
     const bool paramz = pcol == -1;
+    // sweeps of a parallel-beam centre run as columns of the staged kernel (which they share with
+    // parameter z), from 9 slices: a column has 16, and half-empty ones still match the gathers
+    // (360 x 512^2 -> 40 x 512^2: 6.74 -> 4.46 ms); the transposed projections of the horizontal one need their memory
+    const bool stageable = (g->compute_type == 0 || g->compute_type == 2) && !g->interpolation && g->staging &&
+                           g->result_type == RT_FLOAT && g->store_type == ST_FLOAT && g->addressing_mode == AD_CLAMP;
+    const uint32_t tpitch = round_up(H, 4);
+    int sweep = SWEEP_NONE;
+    if (stageable && parallel && nz > 8 && n <= 65535 && pcol == GC_CENTER_X &&
+        g->d_proj_h.ensure((size_t)n * W * tpitch * sizeof(float)) == UFOB_OK)
+        sweep = SWEEP_CENTER_X;
+    if (stageable && parallel && nz > 8 && pcol == GC_CENTER_Z && W % 4 == 0 && !((uintptr_t)d_proj & 15))
+        sweep = SWEEP_CENTER_Z;
+    if (sweep) {
+        std::vector<double> swept(table), rel(slice_values);
+        const double mid = slice_values[nz / 2];
+        for (uint32_t p = 0; p < n; p++) swept[(size_t)p * GC_NCOLS + pcol] = mid;
+        for (double &v : rel) v -= mid;
+        bool launched = false;
+        UFOB_TRY(gbp_staged(g, d_proj, W, H, swept, flags, x0, dxs, y0, dys, nx, ny, rel, sweep, d_vol, &launched, s));
+        if (launched) return UFOB_OK;
+    }
     std::vector<double> zvals(nz, g->z);
     if (paramz) zvals = slice_values;
+    if (stageable && paramz && W % 4 == 0 && !((uintptr_t)d_proj & 15)) {
+        bool launched = false;
+        UFOB_TRY(gbp_staged(g, d_proj, W, H, table, flags, x0, dxs, y0, dys, nx, ny, zvals, SWEEP_NONE, d_vol,
+                            &launched, s));
+        if (launched) return UFOB_OK;
+    }
     const uint32_t tab_slices = paramz ? 1 : nz;
     UFOB_TRY(g->d_geom.ensure(table.size() * sizeof(double) + nz * sizeof(double)));
     UFOB_TRY(g->d_zvals.ensure(nz * sizeof(double) * 2));
@@ -1339,8 +1581,8 @@ static ufob_status gbp_compute(ufob_gbp *g, const float *d_proj, uint32_t W, uin
     UFOB_CUDA_TRY(cudaMemcpyAsync(d_slicev, slice_values.data(), nz * sizeof(double), cudaMemcpyHostToDevice, s));
     UFOB_CUDA_TRY(cudaMemcpyAsync(g->d_zvals.ptr, zvals.data(), nz * sizeof(double), cudaMemcpyHostToDevice, s));
     k_gbp_tables<<<dim3((n + 127) / 128, tab_slices), 128, 0, s>>>(d_table, n, tab_slices, paramz ? -1 : pcol, d_slicev,
-                                                                  flags, x0, dxs, y0, dys, g->d_tab_f.as<float>(),
-                                                                  g->d_tab_d.as<double>());
+                                                                  flags, x0, dxs, y0, dys, SWEEP_NONE, 0.0,
+                                                                  g->d_tab_f.as<float>(), g->d_tab_d.as<double>());
     UFOB_CUDA_TRY(cudaGetLastError());
     note_launch();
 
@@ -1371,58 +1613,6 @@ static ufob_status gbp_compute(ufob_gbp *g, const float *d_proj, uint32_t W, uin
                     : launch_gbp_rt<false, double>(a, g->result_type, paramz, s);
     }
     a.tab = g->d_tab_f.ptr;
-    if ((g->compute_type == 0 || g->compute_type == 2) && !g->interpolation && g->staging &&
-        g->result_type == RT_FLOAT && g->store_type == ST_FLOAT && paramz && a.addr == AD_CLAMP && W % 4 == 0 &&
-        !((uintptr_t)d_proj & 15)) {
-        // TMA-staged detector windows for geometries whose u does not depend on z; the plan (host
-        // FP64 tables, window size) is kept while the geometry stays the same
-        std::vector<double> key(table);
-        key.insert(key.end(), {(double)flags, x0, dxs, y0, dys, (double)nx, (double)ny, (double)W, (double)H});
-        key.insert(key.end(), zvals.begin(), zvals.end());
-        if (key != g->col_key) {
-            std::vector<double> tabs((size_t)n * kTab);
-            for (uint32_t p = 0; p < n; p++)
-                gbp_table_entry(&table[(size_t)p * GC_NCOLS], flags, x0, dxs, y0, dys, &tabs[(size_t)p * kTab]);
-            g->col_plan = gbp_col_plan(tabs, n, cone, nx, ny, zvals, W, H);
-            g->col_key.swap(key);
-        }
-        if (g->col_plan.ok) {
-            const float *src = d_proj;
-            if (g->compute_type == 2) {
-                // compute-type half: FP16 samples with FP32 coordinates, weights and sums, the
-                // arithmetic of the FP16 gathers, staged from a rounded FP32 copy
-                const uint64_t n4 = (uint64_t)n * H * W / 4;
-                UFOB_TRY(g->d_proj_h.ensure(n4 * 16));
-                if (n4) {
-                    const uint32_t grid = (uint32_t)std::min<uint64_t>((n4 + 255) / 256, (uint64_t)num_sms() * 16);
-                    k_proj_round_half<<<grid, 256, 0, s>>>(reinterpret_cast<const float4 *>(d_proj), n4,
-                                                           g->d_proj_h.as<float4>());
-                    UFOB_CUDA_TRY(cudaGetLastError());
-                    note_launch();
-                }
-                src = g->d_proj_h.as<float>();
-            }
-            GBPColArgs c;
-            c.proj = src;
-            c.tab = g->d_tab_f.as<float>();
-            c.zvals = a.zvals;
-            c.W = W;
-            c.H = H;
-            c.n_proj = n;
-            c.nx = nx;
-            c.ny = ny;
-            c.nz = nz;
-            c.burst = a.burst;
-            c.bw = g->col_plan.bw;
-            c.bh = g->col_plan.bh;
-            c.norm = (float)a.norm;
-            c.vol = static_cast<float *>(d_vol);
-            c.err = device_error_word();
-            bool launched = false;
-            UFOB_TRY(launch_gbp_col(c, cone, &launched, s));
-            if (launched) return UFOB_OK;
-        }
-    }
     if (g->compute_type == 2) {
         // FP16 samples: the gather unit returns 16-bit texels at twice the FP32 rate;
         // coordinates, weights and sums stay FP32
@@ -1741,7 +1931,7 @@ static ufob_status lamino_compute(ufob_lamino *l, const float *d_proj, uint32_t 
             c.proj = d_proj;
             c.tab = g.d_tab_f.as<float>();
             c.zvals = a.zvals;
-            c.W = W;
+            c.W = c.pitch = W;
             c.H = H;
             c.n_proj = n;
             c.nx = nx;
