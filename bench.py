@@ -30,6 +30,7 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, os.path.join(ROOT, "ufo-filters_b200"))
 
 METRIC = "FBP GUPS (voxel·angle updates/s), 2048²×1500, 1 B200; chosen vs plain at error"
+TENSOR_FALLBACK_TFLOPS = 1590.0
 HBM_FALLBACK_GBS = 6650.0  # copy bandwidth measured earlier on this pool's B200s, used without MEASURED_PEAKS.json
 WORKLOAD = "batched parallel-beam FBP: 2048 slices x 2048 px x 1500 angles on [0, pi), float32"
 I0 = 1.0e4  # photons per ray (Beer-Lambert + Poisson noise)
@@ -557,7 +558,7 @@ def main():
         e2e = {"value": nz_e2e * float(W) * W * P * world / dt / 1e9, "unit": "GUPS",
                "h2d_bytes_per_step": nz_e2e * P * W * 4, "d2h_bytes_per_step": nz_e2e * W * W * 4,
                "slices": nz_e2e, "s_per_step": dt,
-               "api": "ufob_fbp_run_host (C ABI), pinned host buffers, 64-slice chunks (16-slice first and last) on two streams"}
+               "api": "ufob_fbp_run_host (C ABI), pinned host buffers, 64-slice chunks, images downloaded in bands of rows"}
         del fbp, h_in, h_out
 
     # the other four workloads (one-GPU configurations), timed on this GPU after the main arm, with
@@ -578,38 +579,48 @@ def main():
 
     # roofline of the dominant kernel (backprojection)
     bp_ms, bp_n = chosen["kernel_ms_per_step"]["backproject"], chosen["kernel_launches_per_step"]["backproject"]
-    # on-chip bytes per update: 2 FP32 taps / one FP16 tap pair (a 16-byte cell serves 4 slices)
-    gather_bytes = 8.0 if storage == ufob.F32 else 4.0
     upd_per_launch = updates_per_step / bp_n
     avg_launch_s = bp_ms / bp_n * 1e-3
-    achieved = upd_per_launch * gather_bytes / avg_launch_s / 1e9
-    bp_kernel = "k_bp_linear" if storage == ufob.F32 else "k_bp_quads"
-    traffic_per_upd = read_profile_traffic("bp_linear_c1.md" if storage == ufob.F32 else "bp_quads_c1.md")
-    roofline = {"bound": "smem", "kernel": bp_kernel, "achieved": achieved, "peak": smem_gbs, "unit": "GB/s",
-                "frac": achieved / smem_gbs,
-                "traffic": traffic_per_upd * upd_per_launch if traffic_per_upd is not None else None,
-                "algorithmic_bytes_per_update": gather_bytes,
-                "peak_source": "measured on this GPU by ufob_measure_peaks (32-bit shared loads); MEASURED_PEAKS.json "
-                               "has no shared-memory figure",
-                "gups_achieved_kernel": upd_per_launch / avg_launch_s / 1e9,
-                "gups_roofline": smem_gbs / gather_bytes,
-                "fp32_tflops_measured": fp32_tflops}
+    gups_kernel = upd_per_launch / avg_launch_s / 1e9
+    peaks = {}
+    try:
+        peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
+    except (OSError, ValueError):
+        pass
+    if storage == ufob.F32:
+        # slice cells: nine 4-byte taps from shared memory per eight updates
+        per_update = 4.5
+        achieved, peak, unit = gups_kernel * per_update, smem_gbs, "GB/s"
+        roofline = {"bound": "smem", "kernel": "k_bp_cells", "algorithmic_bytes_per_update": per_update,
+                    "peak_source": "measured on this GPU by ufob_measure_peaks (32-bit shared loads); "
+                                   "MEASURED_PEAKS.json has no shared-memory figure"}
+    else:
+        # one product of 128 rows (110 pixels) x 16 taps per angle and slice: dense operations, most of
+        # them with zero weights
+        per_update = 2.0 * 16 * 128 / 110
+        peak = float(peaks.get("bf16_tflops") or TENSOR_FALLBACK_TFLOPS)
+        achieved, unit = gups_kernel * per_update / 1e3, "TFLOP/s"
+        roofline = {"bound": "tensor", "kernel": "k_bp_umma", "dense_flop_per_update": per_update,
+                    "peak_source": "MEASURED_PEAKS.json bf16_tflops" if peaks.get("bf16_tflops") else
+                    "fallback: 1590 TFLOP/s measured earlier on this pool (MEASURED_PEAKS.json absent)"}
+    traffic_per_upd = read_profile_traffic("bp_cells_c1.md" if storage == ufob.F32 else "bp_umma_c1.md")
+    roofline.update({"achieved": achieved, "peak": peak, "unit": unit, "frac": achieved / peak,
+                     "traffic": traffic_per_upd * upd_per_launch if traffic_per_upd is not None else None,
+                     "gups_achieved_kernel": gups_kernel, "gups_roofline": gups_kernel * peak / achieved,
+                     "fp32_tflops_measured": fp32_tflops})
     # independent cross-check of the measured peak: 128 bytes per SM per clock (one shared-memory
     # wavefront) at the median SM clock sampled during the timed region
     sm_mhz = chosen["clocks"].get("sm_mhz")
-    if sm_mhz:
+    if sm_mhz and storage == ufob.F32:
         nominal = torch.cuda.get_device_properties(dev).multi_processor_count * 128.0 * sm_mhz * 1e6 / 1e9
         roofline["peak_nominal_gbs"] = nominal
         roofline["frac_of_nominal"] = achieved / nominal
     # the pool's measured copy bandwidth when the file is there, else the earlier pool measurement
     hbm_peak, hbm_source = HBM_FALLBACK_GBS, "fallback: 6.65 TB/s measured earlier on this pool (MEASURED_PEAKS.json absent)"
-    try:
-        hbm_peak = float(json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))["hbm_gbs"])
-        hbm_source = "MEASURED_PEAKS.json hbm_gbs"
-    except (OSError, KeyError, ValueError, TypeError):
-        pass
+    if peaks.get("hbm_gbs"):
+        hbm_peak, hbm_source = float(peaks["hbm_gbs"]), "MEASURED_PEAKS.json hbm_gbs"
     f_ms, f_n = chosen["kernel_ms_per_step"]["filter"], chosen["kernel_launches_per_step"]["filter"]
-    f_bytes = Z * P * W * 4.0 + Z * P * (W if storage == ufob.F32 else (W + 1)) * 4.0
+    f_bytes = Z * P * W * (8.0 if storage == ufob.F32 else 6.0)
     f_kernel = "k_filter_fast" if 256 <= W <= 4096 and os.environ.get("UFOB_FILTER_RADIX4") != "1" else "k_filter_rows"
     roofline_filter = {"bound": "hbm", "kernel": f_kernel, "achieved": f_bytes / (f_ms * 1e-3) / 1e9,
                        "peak": hbm_peak, "unit": "GB/s",
