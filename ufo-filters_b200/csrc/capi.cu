@@ -648,8 +648,11 @@ extern "C" ufob_status ufob_backproject_run(ufob_backproject *bp, const void *d_
     const bool kahan = want_kahan(bp->props, kind, height);
     if (kind == SINO_F32 && cells_apply(bp->props, g)) {
         // slice cells by groups of 32 slices; without the memory for them the row kernel does it
+        // (nor do captured graphs use them, which would keep the address of a buffer that may grow)
         const uint32_t G = std::min(nslices, 32u);
-        if (bp->cells.ensure((size_t)((G + 3) / 4) * 16 * width * height) == UFOB_OK) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
+        if (cap == cudaStreamCaptureStatusNone && bp->cells.ensure((size_t)((G + 3) / 4) * 16 * width * height) == UFOB_OK) {
             for (uint32_t z = 0; z < nslices; z += G) {
                 BPGeometry gz = g;
                 gz.nz = std::min(G, nslices - z);
