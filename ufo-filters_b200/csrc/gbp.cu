@@ -537,6 +537,7 @@ struct GBPColArgs {
     float *vol;
     int *err;
     uint32_t pitch;  // floats between detector rows (last: among the sizes above, the cone kernel ran 1.4% slower)
+    int walk;        // every projection moves v by less than 0.99 rows per voxel
 };
 
 template <int PB, int S>
@@ -564,7 +565,8 @@ struct GBPColSmem {
     }
 };
 
-template <bool CONE, int ZT, int PB, int S>
+// WALK: affine geometries whose v moves by less than a row per voxel (the others read both rows).
+template <bool CONE, bool WALK, int ZT, int PB, int S>
 __global__ void __launch_bounds__(256, 2) k_gbp_col(const __grid_constant__ CUtensorMap map, const GBPColArgs c)
 {
     static_assert(PB <= 32 && kTab % 4 == 0, "one producer lane per projection of a stage");
@@ -576,16 +578,16 @@ __global__ void __launch_bounds__(256, 2) k_gbp_col(const __grid_constant__ CUte
     // a warp covers 16 x 2 columns: its samples of one row then span fewer than 32 banks
     const int ix = x0 + (warp & 1) * 16 + (lane & 15), iy = y0 + (warp >> 1) * 2 + (lane >> 4);
     const float fx = (float)ix, fy = (float)iy;
-    // the column's voxels as packed pairs: neighbours for the cone, else (j, j + ZT / 2), so that each
-    // lane walks half of the column
-    constexpr int ZP = ZT / 2, Z0 = CONE ? 2 : 1, Z1 = CONE ? 1 : ZP;  // pair j: voxels Z0 j, Z0 j + Z1
+    // the column's voxels as packed pairs: neighbours, or (j, j + ZT / 2) where each lane walks half of
+    // the column
+    constexpr int ZP = ZT / 2, Z0 = WALK ? 1 : 2, Z1 = WALK ? ZP : 1;  // pair j: voxels Z0 j, Z0 j + Z1
     uint64_t zz[ZP];
 #pragma unroll
     for (int j = 0; j < ZP; j++)
         zz[j] = f2pack((float)c.zvals[min(z0 + Z0 * j, (int)c.nz - 1)],
                        (float)c.zvals[min(z0 + Z0 * j + Z1, (int)c.nz - 1)]);
     float zstep = 0.f;  // largest step of a walk, with the sign of all of them (z values are equally spaced)
-    if constexpr (!CONE) {
+    if constexpr (WALK) {
         float last = (float)c.zvals[min(z0, (int)c.nz - 1)];
 #pragma unroll
         for (int k = 1; k < ZT; k++) {
@@ -736,10 +738,8 @@ __global__ void __launch_bounds__(256, 2) k_gbp_col(const __grid_constant__ CUte
                     const float *col = win + iu;
                     const uint64_t AA = f2pack(a, a), AV = f2pack(Av, Av), BV = f2pack(Bv, Bv);
                     const uint64_t MM = f2pack(M, M), WG = f2pack(wgt, wgt);
-                    if constexpr (CONE) {
-                        // Cone beams magnify about half of a volume to more than a row per voxel, and
-                        // their warps mix both, so both rows of every voxel are read (walking where
-                        // possible was 1% slower).
+                    if constexpr (!WALK) {
+                        // both rows of every voxel
 #pragma unroll
                         for (int j = 0; j < ZP; j++) {
                             const uint64_t vp = f2fma(AV, zz[j], BV);
@@ -756,7 +756,7 @@ __global__ void __launch_bounds__(256, 2) k_gbp_col(const __grid_constant__ CUte
                             const uint64_t t01 = f2pack(p0[bw], p1[bw]), t11 = f2pack(p0[bw + 1], p1[bw + 1]);
                             const uint64_t top = f2fma(AA, f2sub(t10, t00), t00), bot = f2fma(AA, f2sub(t11, t01), t01);
                             const uint64_t val = f2fma(bb, f2sub(bot, top), top);
-                            bsum[j] = f2fma(val, WG, bsum[j]);
+                            bsum[j] = CONE ? f2fma(val, WG, bsum[j]) : f2add(bsum[j], val);
                         }
                     } else {
                     // row i's two texels of one lane's voxel, interpolated along u
@@ -811,8 +811,7 @@ __global__ void __launch_bounds__(256, 2) k_gbp_col(const __grid_constant__ CUte
                     } else if (__all_sync(__activemask(), vstep <= 0.f && vstep > -0.99f)) {
                         walk(std::true_type());
                     } else {
-                        // both rows of every voxel (one row per voxel and more, as in parallel beam:
-                        // 1103 -> 1019 GUPS with pairs half a column apart in place of neighbours)
+                        // a projection past the plan's rows per voxel
 #pragma unroll
                         for (int j = 0; j < ZP; j++) {
                             const uint64_t vp = f2fma(AV, zz[j], BV);
@@ -906,6 +905,7 @@ __global__ void __launch_bounds__(256, 2) k_gbp_col(const __grid_constant__ CUte
 // (all projections), plus two texels of margin each way.
 struct GBPColPlan {
     bool ok = false;
+    bool walk = false;  // affine, and v moves by less than 0.99 rows per voxel in every projection
     uint32_t bw = 0, bh = 0;
 };
 
@@ -961,16 +961,21 @@ static GBPColPlan gbp_col_plan(const std::vector<double> &tabs, uint32_t n, bool
     const double bw = std::ceil((wmax + 2.0) / 4.0) * 4.0, bh = hmax + 2.0;
     if (!(bw >= 4 && bw <= 256 && bh >= 2 && bh <= 256)) return plan;
     plan.ok = true;
+    double step = 0.0;
+    for (uint32_t k = 1; k < nz; k++) step = std::max(step, std::fabs(zvals[k] - zvals[k - 1]));
+    plan.walk = !cone;
+    for (uint32_t p = 0; p < n; p++)
+        plan.walk = plan.walk && std::fabs(tabs[(size_t)p * kTab + 6]) * step < 0.99;
     plan.bw = (uint32_t)bw;
     plan.bh = (uint32_t)bh;
     return plan;
 }
 
-template <bool CONE, int PB, int S>
-static ufob_status launch_gbp_col_t(const GBPColArgs &c, cudaStream_t s)
+template <bool CONE, bool WALK, int PB, int S>
+static ufob_status launch_gbp_col_m(const GBPColArgs &c, cudaStream_t s)
 {
     using Sm = GBPColSmem<PB, S>;
-    auto kern = k_gbp_col<CONE, kColZT, PB, S>;
+    auto kern = k_gbp_col<CONE, WALK, kColZT, PB, S>;
     static std::atomic<uint64_t> attr_devs{0};
     const size_t smem = Sm::bytes(c.slot_floats);
     UFOB_CUDA_TRY(smem_limit_per_device(kern, 227 * 1024, attr_devs));
@@ -981,6 +986,17 @@ static ufob_status launch_gbp_col_t(const GBPColArgs &c, cudaStream_t s)
     UFOB_CUDA_TRY(cudaGetLastError());
     note_launch();
     return UFOB_OK;
+}
+
+// The instance for the geometry.  Cone beams magnify about half of a volume to more than a row per
+// voxel, and their warps mix both, so they read both rows (walking where possible was 1% slower); so
+// does parallel beam with one row per voxel (1103 GUPS, 1019 with the walk's pairing of voxels).
+template <bool CONE, int PB, int S>
+static ufob_status launch_gbp_col_t(const GBPColArgs &c, cudaStream_t s)
+{
+    if constexpr (!CONE)
+        if (c.walk) return launch_gbp_col_m<false, true, PB, S>(c, s);
+    return launch_gbp_col_m<CONE, false, PB, S>(c, s);
 }
 
 static constexpr size_t kColBudget = 110 * 1024;  // shared memory of two CTAs per SM
@@ -1444,6 +1460,7 @@ static ufob_status gbp_staged(ufob_gbp *g, const float *d_proj, uint32_t W, uint
     GBPColArgs c;
     c.bw = g->col_plan.bw;
     c.bh = g->col_plan.bh;
+    c.walk = g->col_plan.walk;
     if (!gbp_col_fits(c)) return UFOB_OK;
     UFOB_TRY(g->d_geom.ensure(table.size() * sizeof(double) + nz * sizeof(double)));
     UFOB_TRY(g->d_zvals.ensure(nz * sizeof(double) * 2));
@@ -1948,6 +1965,7 @@ static ufob_status lamino_compute(ufob_lamino *l, const float *d_proj, uint32_t 
             c.nz = nz;
             c.burst = a.burst;
             c.bw = g.col_plan.bw;
+            c.walk = g.col_plan.walk;
             c.bh = g.col_plan.bh;
             c.norm = norm;
             c.vol = d_vol;
