@@ -59,6 +59,20 @@ def test_angle_counts(cuda, nz, P):
     assert oracle.rel_l2(_fbp(raw, 64), _ref(raw, 64)) < TOL
 
 
+# the issuing lanes read window starts that the other lanes of their warps write, anew for every 32
+# angles: passes over seven such groups agree to the bit, for each stage length
+@pytest.mark.parametrize("nz", [20, 50, 120])
+def test_passes_repeat(cuda, nz):
+    raw = _raw(nz, 200, 150, nz)
+    f = ufob.FBP(filter_props={"size_x": 256, "crop_width": 150}, storage=ufob.F16)
+    dev = torch.from_numpy(raw).cuda()
+    first = f.process(dev).clone()
+    for _ in range(4):
+        assert torch.equal(f.process(dev), first)
+    ufob.device_status()
+    assert oracle.rel_l2(first[nz - 1:].cpu().numpy(), _ref(raw[nz - 1:], 256)) < TOL
+
+
 def test_roi_axis_offset(cuda):
     raw = _raw(18, 60, 100, 4)
     bp = dict(axis_pos=43.3, angle_step=math.pi / 50, angle_offset=0.7, roi_x=70, roi_y=5, roi_width=61,

@@ -339,6 +339,7 @@ __global__ void __launch_bounds__(kThreads, KA <= 2 ? 4 : 2)
                     if (skip) s_flagged = 1;
                 }
                 skips = __any_sync(0xffffffffu, skip);
+                __syncwarp();  // the issuing lane reads the other lanes' entries
             }
             const uint32_t n = min(32u, P - p0);
             if (lane == 0) {
