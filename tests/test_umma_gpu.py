@@ -113,8 +113,61 @@ def test_nonfinite_bins_stay_local(cuda, bad):
         near[z] |= np.abs(h - j) < 1.001
     assert not np.isfinite(got[touched]).any()
     assert np.isfinite(got[~near]).all()
-    # the flagged rows are sampled with FP32 weights, the others with 11-bit ones
     assert oracle.rel_l2(got[~near], clean[~near]) < TOL
+
+
+# bad bins in several octets, stages and windows, for each stage length: every finite pixel has the bits
+# of the same stack with zeros in their place, and the other slices those of the clean stack
+@pytest.mark.parametrize("nz", [20, 50, 90, 120, 250])
+def test_nonfinite_bins_leave_the_rest(cuda, nz):
+    P, W = 70, 120
+    raw = _raw(nz, P, W, nz)
+    rng = np.random.default_rng(nz)
+    zeroed, dirty = raw.copy(), raw.copy()
+    bad_slices = sorted({0, 7, 9, nz // 2, nz - 1})
+    for z in bad_slices:
+        for _ in range(12):
+            p, j = rng.integers(P), rng.integers(W)
+            dirty[z, p, j] = rng.choice([math.nan, math.inf, -math.inf, 1.0e6, -1.0e6])
+            zeroed[z, p, j] = 0.0
+    dirty[9, :, 31], zeroed[9, :, 31] = math.nan, 0.0  # a dead detector pixel
+    t = ufob.StackedBackprojectTask(precision_mode="half", axis_pos=57.3)
+    clean, want, got = (t.process(torch.from_numpy(x).cuda()).cpu().numpy() for x in (raw, zeroed, dirty))
+    ufob.device_status()
+    finite = np.isfinite(got)
+    assert not finite.all() and finite.any()
+    np.testing.assert_array_equal(got[finite], want[finite])
+    good = [z for z in range(nz) if z not in bad_slices]
+    np.testing.assert_array_equal(got[good], clean[good])
+
+
+# a dead slice (the FFT fills its rows with NaN, and those of the slice it is transformed with) costs its
+# octet one look-up per pixel: the pass stays near the clean one (sampling all slices at the angles
+# concerned took 40 times as long)
+def test_dead_slice_is_cheap(cuda):
+    nz, P, W = 64, 600, 512
+    f = ufob.FBP(storage=ufob.F16)
+    clean = torch.randn(nz, P, W, device="cuda")
+    dead = clean.clone()
+    dead[17, :, 200] = math.nan
+
+    def ms(x, out):
+        f.process(x, out=out)
+        a, b = torch.cuda.Event(True), torch.cuda.Event(True)
+        a.record()
+        for _ in range(5):
+            f.process(x, out=out)
+        b.record()
+        torch.cuda.synchronize()
+        return a.elapsed_time(b)
+
+    outs = [torch.empty(nz, W, W, device="cuda") for _ in range(2)]
+    t_clean, t_dead = ms(clean, outs[0]), ms(dead, outs[1])
+    ufob.device_status()
+    assert t_dead < 5 * t_clean, (t_dead, t_clean)
+    good = [z for z in range(nz) if z not in (16, 17)]
+    assert torch.equal(outs[0][good], outs[1][good])
+    assert torch.isnan(outs[1][17, W // 4:3 * W // 4, W // 4:3 * W // 4]).all()
 
 
 # the host pipeline makes large images in bands of rows: the same bits as one launch, whole chunks

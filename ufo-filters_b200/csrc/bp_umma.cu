@@ -36,14 +36,18 @@
 // and larger stages (KA = 4, 8) the cases that leave room for fewer CTAs.  2048^2 x 1500 angles, ms per
 // pass: ns <= 32 15.5, 64 16.6, 96 24.2, 128 29.0 (13.0, 24.3, 25.0, 27.8 TGUPS; slice quads 6.6).
 //
-// A non-finite value of a window would reach every pixel of its tile (0 * inf), so the filter
-// flags the angles that hold one; their products are skipped and the epilogue adds them by direct
-// sampling, which touches the pixels whose taps they are.
+// A non-finite value of a window would reach every pixel of its tile (0 * inf).  The filter flags
+// the slices and angles that have one; k_octs_finite puts -0 in the place of such values in these rows
+// (and +0 for any -0), notes which class they were and their range, and the epilogue looks up which pixels
+// interpolate them: a pixel with a non-finite sample is infinite or NaN whatever its other samples are.
+// (Zeroing them in the staged windows cost clean stacks 2 to 9%; leaving the flagged angles out of the
+// products and sampling them in the epilogue took 724 ms for 64 x 1500 x 2048 with one dead slice.)
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <climits>
 
 #include "tma.cuh"
 #include "ufob_internal.h"
@@ -60,7 +64,7 @@ constexpr int KW = 28;           // staged bins: KT + 10 |sin| + 1, rounded up
 constexpr int SA = 2;            // stages of weights
 constexpr int kBuildWarps = 4;
 constexpr int kThreads = 32 * (kBuildWarps + 1 + MT);
-constexpr uint32_t kSkip = 0xffffffffu;
+enum { CLASS_NAN = 1, CLASS_POS = 2, CLASS_NEG = 4 };  // flag bytes: what the -0 of a row stand for
 constexpr int kErrUmmaTimeout = 0x1003;
 
 // KA angles per stage.
@@ -152,16 +156,36 @@ struct UmmaArgs {
     uint32_t roi_x, roi_y, roi_w, roi_h;
     float axis, norm;
     const float2 *sincos;
-    const uint4 *sino;     // slice octets, for the flagged angles
+    const uint4 *sino;     // slice octets, for the flagged ones
     uint32_t W, pitch;     // bins, cells per row
     uint64_t group_pitch;  // cells per octet
-    const uint8_t *flags;  // [P] angles with a non-finite value in some slice
+    const uint2 *flags;    // [octets][P] classes of the octet's slices
+    const int2 *ranges;    // [octets][P] first and last bin with a non-finite value (none: INT_MAX, -1)
+    const uint32_t *any;   // [octets] slices with one at some angle
     float *out;
     uint64_t plane;  // output floats between slices
     int *err;
     uint32_t tiles_x, tiles_y, tmem_cols;
     uint32_t one;  // 1, not known to the compiler: keeps the weights' sums off the busier ALU pipe
 };
+
+// Tile of a CTA.  Tiles go in bands about 200 pixels wide, walked top to bottom: the CTAs resident at
+// one time cover a compact region, whose windows the L2 serves to all of them.
+__device__ __forceinline__ void tile_origin(const UmmaArgs &args, int &x0, int &y0)
+{
+    constexpr uint32_t GW = 18;
+    const uint32_t id = blockIdx.x, band_tiles = GW * args.tiles_y;
+    const uint32_t band = id / band_tiles, rr = id - band * band_tiles;
+    const uint32_t bw = min(GW, args.tiles_x - band * GW);
+    x0 = (int)(band * GW + rr % bw) * MX;
+    y0 = (int)(rr / bw) * (MT * MY);
+}
+
+// Centre of the tile's upper accumulator along one axis
+__device__ __forceinline__ float tile_centre(uint32_t roi0, int first, int pixels, float axis)
+{
+    return (float)(roi0 + first) - axis + 0.5f + 0.5f * (pixels - 1);
+}
 
 // First detector bin reached by the accumulator centred at (cx, cy).  Every role computes it with
 // the same operations, so they agree to the bit.
@@ -174,32 +198,156 @@ __device__ __forceinline__ int window_start(float cx, float cy, float2 sc, float
     return (int)e;
 }
 
-// v[0..15] += samples of the flagged angles at one pixel, slices z .. z + 15 (not weighted by norm)
-__device__ __noinline__ void add_flagged(const UmmaArgs &a, float bx, float by, uint32_t z, float (&v)[16])
+// Value that bin `h` (16 bits) of a row of class `cls` stands for.
+__device__ __forceinline__ float octet_value(uint32_t h, uint32_t cls)
 {
-    for (uint32_t p = 0; p < a.P; p++) {
-        if (!__ldg(a.flags + p)) continue;
-        const float2 sc = __ldg(&a.sincos[p]);
-        const float h = fmaf(by, sc.x, fmaf(bx, sc.y, a.axis)) - 0.5f;
-        const float e = floorf(h), f = h - e;
-        if (!(e >= -1.0f && e < (float)a.W)) continue;
-        const int j = (int)e;
-        for (uint32_t q = 0; q < 2; q++) {
-            const uint32_t g = z / 8 + q;
-            if (g * 8 >= a.nz) break;
+    if (h == 0x8000u && cls) return cls == CLASS_NAN ? NAN : cls == CLASS_POS ? INFINITY : -INFINITY;
+    return __half2float(__ushort_as_half((unsigned short)h));
+}
+
+// Slices of octet g (of those in `bad`) whose samples at this lane's pixel sum to NaN (bits 0..7), to
+// +infinity (8..15) or to -infinity (16..23), by a whole warp: a lane per angle finds those whose
+// window at the tile centred at (cx, cy) has a non-finite value, and all lanes sample these.  Done once
+// all of `bad` are NaN at every pixel, as after the first angles of slices whose rows the filter's FFT has
+// filled with NaN.
+__device__ __forceinline__ uint32_t nonfinite_slices(const UmmaArgs &a, float cx, float cy, float bx, float by, bool in,
+                                                     uint32_t g, uint32_t bad)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    const size_t row0 = (size_t)g * a.P;
+    uint32_t nan = 0, pos = 0, neg = 0;
+    for (uint32_t p0 = 0; p0 < a.P; p0 += 32) {
+        const uint32_t pl = min(p0 + lane, a.P - 1);
+        const int2 r = __ldg(a.ranges + row0 + pl);
+        const float2 sl = __ldg(&a.sincos[pl]);
+        const int w0 = min(window_start(cx, cy, sl, a.axis), window_start(cx, cy + MY, sl, a.axis));
+        uint32_t hits = __ballot_sync(0xffffffffu, p0 + lane < a.P && r.x <= w0 + KW && r.y >= w0 - 1);
+        for (; hits && __any_sync(0xffffffffu, in && (bad & ~nan)); hits &= hits - 1) {
+            const uint32_t q = __ffs(hits) - 1, p = p0 + q;
+            const float s = __shfl_sync(0xffffffffu, sl.x, q), c = __shfl_sync(0xffffffffu, sl.y, q);
+            const int first = __shfl_sync(0xffffffffu, r.x, q), last = __shfl_sync(0xffffffffu, r.y, q);
+            const float h = fmaf(by, s, fmaf(bx, c, a.axis)) - 0.5f;
+            const float e = floorf(h), f = h - e;
+            if (!in || !(e >= -1.0f && e < (float)a.W)) continue;
+            const int j = (int)e;
+            if (j + 1 < first || j > last) continue;
+            const uint2 cls = __ldg(a.flags + row0 + p);
             const uint4 *row = a.sino + (size_t)g * a.group_pitch + (size_t)p * a.pitch;
             const uint4 zero = make_uint4(0, 0, 0, 0);
             const uint4 lo = j >= 0 ? __ldg(row + j) : zero, hi = j + 1 < (int)a.W ? __ldg(row + j + 1) : zero;
             const uint32_t l[4] = {lo.x, lo.y, lo.z, lo.w}, u[4] = {hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const float2 s0 = __half22float2(*reinterpret_cast<const __half2 *>(&l[i]));
-                const float2 s1 = __half22float2(*reinterpret_cast<const __half2 *>(&u[i]));
-                v[8 * q + 2 * i] += (1.0f - f) * s0.x + f * s1.x;
-                v[8 * q + 2 * i + 1] += (1.0f - f) * s0.y + f * s1.y;
+            for (int k = 0; k < 8; k++) {
+                const uint32_t b = ((k < 4 ? cls.x : cls.y) >> (8 * (k & 3))) & 0xffu;
+                const float s0 = octet_value((l[k / 2] >> (16 * (k & 1))) & 0xffffu, b);
+                const float s1 = octet_value((u[k / 2] >> (16 * (k & 1))) & 0xffffu, b);
+                const float v = (1.0f - f) * s0 + f * s1;
+                if (v != v) nan |= 1u << k;
+                if (v == INFINITY) pos |= 1u << k;
+                if (v == -INFINITY) neg |= 1u << k;
+            }
+            nan |= pos & neg;
+        }
+        if (hits) break;
+    }
+    return nan | (pos & ~nan) << 8 | (neg & ~nan) << 16;
+}
+
+// Writes the infinities and NaNs of a CTA's tile over its stored results.  Everything is found anew from
+// the block's and thread's indices, so that it keeps no register of the kernel's loops; and it is inlined:
+// a call anywhere in the kernel made clean stacks 3 to 8% slower.
+__device__ __forceinline__ void store_nonfinite(const UmmaArgs &args)
+{
+    int x0, y0;
+    tile_origin(args, x0, y0);
+    const uint32_t lane = threadIdx.x & 31, z0 = blockIdx.y * args.ns, nz = min(args.ns, args.nz - z0);
+    const float cx = tile_centre(args.roi_x, x0, MX, args.axis), cy = tile_centre(args.roi_y, y0, MY, args.axis);
+    constexpr uint32_t R = (MX * MT * MY + 31) / 32;  // warps' shares of the tile's pixels
+    for (uint32_t item = threadIdx.x >> 5; item < R * ((nz + 7) / 8); item += kThreads / 32) {
+        const uint32_t q = item / R, pix = (item - q * R) * 32 + lane, bad = __ldg(args.any + z0 / 8 + q);
+        if (!bad) continue;
+        const int px = x0 + (int)(pix % MX), py = y0 + (int)(pix / MX);
+        const bool in = pix < MX * MT * MY && px < (int)args.roi_w && py < (int)args.roi_h;
+        const float bx = (float)(args.roi_x + px) - args.axis + 0.5f, by = (float)(args.roi_y + py) - args.axis + 0.5f;
+        const uint32_t k = nonfinite_slices(args, cx, cy, bx, by, in, z0 / 8 + q, bad);
+        float *o = args.out + (size_t)(z0 + 8 * q) * args.plane + (size_t)py * args.roi_w + px;
+        for (uint32_t bits = in ? (k | k >> 8 | k >> 16) & 0xffu : 0; bits; bits &= bits - 1) {
+            const uint32_t i = __ffs(bits) - 1;
+            o[(size_t)i * args.plane] = (k >> i) & 1u ? NAN : (k >> (8 + i)) & 1u ? INFINITY : -INFINITY;
+        }
+    }
+}
+
+// Flagged rows of a slice octet (blockIdx.x): -0 for the non-finite values of the flagged slices, whose
+// bytes then hold the class (a row with several classes counts as NaN), and +0 for any -0 they had.
+// Without flags, one read of their words (2 us in all).
+__global__ void __launch_bounds__(1024) k_octs_finite(uint4 *__restrict__ cells, uint32_t W, uint32_t pitch,
+                                                      uint64_t group_pitch, uint32_t P, uint2 *__restrict__ flags,
+                                                      int2 *__restrict__ ranges, uint32_t *__restrict__ any)
+{
+    __shared__ uint32_t s_any;
+    const uint32_t g = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    flags += (size_t)g * P;
+    ranges += (size_t)g * P;
+    uint32_t some = 0;
+    for (uint32_t p = threadIdx.x; p < P; p += 1024) some |= flags[p].x | flags[p].y;
+    if (threadIdx.x == 0) any[g] = s_any = 0;
+    if (!__syncthreads_or((int)some)) return;
+    for (uint32_t base = 0; base < P; base += 1024) {
+        const uint32_t p = base + lane * 32 + warp;  // neighbouring angles go to different warps
+        const uint2 mine = p < P ? flags[p] : make_uint2(0, 0);
+        const bool found = (mine.x | mine.y) != 0;
+        if (p < P && !found) ranges[p] = make_int2(INT_MAX, -1);
+        for (uint32_t rows = __ballot_sync(0xffffffffu, found); rows; rows &= rows - 1) {
+            const int from = __ffs(rows) - 1;
+            const uint32_t r = base + from * 32 + warp;
+            const uint32_t fx = __shfl_sync(0xffffffffu, mine.x, from), fy = __shfl_sync(0xffffffffu, mine.y, from);
+            uint4 *row = cells + (size_t)g * group_pitch + (size_t)r * pitch;
+            uint32_t nan = 0, pos = 0, neg = 0;
+            int lo = INT_MAX, hi = -1;
+#pragma unroll 4
+            for (uint32_t j = lane; j < W; j += 32) {
+                const uint4 v = row[j];
+                uint32_t w[4] = {v.x, v.y, v.z, v.w};
+                uint32_t bad = 0;
+#pragma unroll
+                for (int k = 0; k < 8; k++) {
+                    const uint32_t sh = 16 * (k & 1), h = (w[k / 2] >> sh) & 0xffffu;
+                    if (!((k < 4 ? fx : fy) >> (8 * (k & 3)) & 1u)) continue;
+                    if ((h & 0x7C00u) == 0x7C00u) {
+                        ((h & 0x3ffu) ? nan : h >> 15 ? neg : pos) |= 1u << k;
+                        w[k / 2] = (w[k / 2] & ~(0xffffu << sh)) | 0x8000u << sh;
+                        bad = 1;
+                    } else if (h == 0x8000u) {
+                        w[k / 2] &= ~(0xffffu << sh);
+                    }
+                }
+                if (bad) {
+                    lo = min(lo, (int)j);
+                    hi = (int)j;
+                }
+                if (w[0] != v.x || w[1] != v.y || w[2] != v.z || w[3] != v.w)
+                    row[j] = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+            nan = __reduce_or_sync(0xffffffffu, nan);
+            pos = __reduce_or_sync(0xffffffffu, pos);
+            neg = __reduce_or_sync(0xffffffffu, neg);
+            lo = __reduce_min_sync(0xffffffffu, lo);
+            hi = __reduce_max_sync(0xffffffffu, hi);
+            if (lane == 0) {
+                uint2 f = make_uint2(0, 0);
+                for (int k = 0; k < 8; k++) {
+                    const uint32_t n = (nan >> k) & 1u, a = (pos >> k) & 1u, b = (neg >> k) & 1u;
+                    (k < 4 ? f.x : f.y) |= (n || (a && b) ? CLASS_NAN : a ? CLASS_POS : b ? CLASS_NEG : 0) << (8 * (k & 3));
+                }
+                flags[r] = f;
+                ranges[r] = make_int2(lo, hi);
+                atomicOr(&s_any, nan | pos | neg);
             }
         }
     }
+    __syncthreads();
+    if (threadIdx.x == 0) any[g] = s_any;
 }
 
 template <int KA>
@@ -215,22 +363,25 @@ __global__ void __launch_bounds__(kThreads, KA <= 2 ? 4 : 2)
     __shared__ int s_win[32];
     __shared__ uint32_t s_off[MT][32];
     __shared__ uint32_t tslot;
-    __shared__ int s_abort, s_flagged, s_live;
+    __shared__ uint32_t s_any;  // an octet has a non-finite value
+    __shared__ int s_abort;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t bbytes = Sh::window_bytes(args.ns);
     const uint32_t base = (smem_u32(smem_dyn) + 127u) & ~127u;
     unsigned char *gbase = smem_dyn + (base - smem_u32(smem_dyn));
 
-    // tiles in bands about 200 pixels wide, walked top to bottom: the CTAs resident at one time
-    // cover a compact region, whose windows the L2 serves to all of them
-    constexpr uint32_t GW = 18;
-    const uint32_t id = blockIdx.x, band_tiles = GW * args.tiles_y;
-    const uint32_t band = id / band_tiles, rr = id - band * band_tiles;
-    const uint32_t bw = min(GW, args.tiles_x - band * GW);
-    const int x0 = (int)(band * GW + rr % bw) * MX, y0 = (int)(rr / bw) * (MT * MY);
+    int x0, y0;
+    tile_origin(args, x0, y0);
     const uint32_t z0 = blockIdx.y * args.ns;
 
     if (warp == kBuildWarps) tmem_alloc(&tslot, args.tmem_cols);
+    if (warp == 0) {
+        const uint32_t o = z0 / 8 + lane;
+        const bool any = 8u * lane < args.ns && o < (args.nz + 7) / 8 && __ldg(args.any + o) != 0;
+        if (lane == 0) s_any = 0;
+        __syncwarp();
+        if (any) s_any = 1;
+    }
     if (tid == 0) {
         for (int s = 0; s < SA; s++) mbar_init(&full_a[s], kBuildWarps);
         for (int s = 0; s < SB; s++) {
@@ -238,7 +389,7 @@ __global__ void __launch_bounds__(kThreads, KA <= 2 ? 4 : 2)
             mbar_init(&empty[s], MT);
         }
         mbar_init(&done, MT);
-        s_abort = s_flagged = s_live = 0;
+        s_abort = 0;
         fence_barrier_init();
     }
     tc_fence_before();
@@ -249,9 +400,7 @@ __global__ void __launch_bounds__(kThreads, KA <= 2 ? 4 : 2)
 
     const uint32_t P = args.P;
     const float axis = args.axis;
-    // centre of the upper accumulator
-    const float cx = (float)(args.roi_x + x0) - axis + 0.5f + 0.5f * (MX - 1);
-    const float cy = (float)(args.roi_y + y0) - axis + 0.5f + 0.5f * (MY - 1);
+    const float cx = tile_centre(args.roi_x, x0, MX, axis), cy = tile_centre(args.roi_y, y0, MY, axis);
     // row of both accumulators of a builder thread and its pixel in the upper one (rows past
     // MX * MY repeat pixel 0 and are not stored)
     const int row = (warp & 3) * 32 + lane;
@@ -322,7 +471,7 @@ __global__ void __launch_bounds__(kThreads, KA <= 2 ? 4 : 2)
         const uint32_t dcol = tmem + (uint32_t)m * args.ns;
         const uint32_t acol = tmem + MT * args.ns + (uint32_t)m * (KT / 2);
         uint32_t acc = 0;
-        bool ok = true, skips = false;
+        bool ok = true;
         for (uint32_t p0 = 0; p0 < P; p0 += 32) {
             {
                 // windows of the next 32 angles, and where in them the accumulators' taps start
@@ -330,15 +479,11 @@ __global__ void __launch_bounds__(kThreads, KA <= 2 ? 4 : 2)
                 const float2 sc = __ldg(&args.sincos[p]);
                 const int w0 = window_start(cx, cy, sc, axis), w1 = window_start(cx, cy + MY, sc, axis);
                 const int wm = min(w0, w1);
-                const bool skip = !produce && __ldg(args.flags + p) != 0;
                 __syncwarp();
-                if (produce) {
+                if (produce)
                     s_win[lane] = wm;
-                } else {
-                    s_off[m][lane] = skip ? kSkip : (uint32_t)min((m ? w1 : w0) - wm, KW - KT);
-                    if (skip) s_flagged = 1;
-                }
-                skips = __any_sync(0xffffffffu, skip);
+                else
+                    s_off[m][lane] = (uint32_t)min((m ? w1 : w0) - wm, KW - KT);
                 __syncwarp();  // the issuing lane reads the other lanes' entries
             }
             const uint32_t n = min(32u, P - p0);
@@ -363,23 +508,20 @@ __global__ void __launch_bounds__(kThreads, KA <= 2 ? 4 : 2)
                              wait_or_abort(&full_a[sa], (it / SA) & 1u, abort_flag);
                         if (!ok) break;
                         tc_fence_after();
-                        if (!skips && nval == KA) {
+                        if (nval == KA) {
 #pragma unroll
                             for (int a = 0; a < KA; a++)
                                 mma_f16(dcol, acol + (sa * KA + a) * (MT * (KT / 2)),
                                         desc0 + (uint64_t)((sb * KA + a) * (bbytes >> 4) + off[a]), idesc,
                                         a > 0 ? 1u : acc);
-                            acc = 1;
                         } else {
 #pragma unroll 1
-                            for (uint32_t a = 0; a < nval; a++) {
-                                const uint32_t o = s_off[m][j + a];
-                                if (o == kSkip) continue;
+                            for (uint32_t a = 0; a < nval; a++)
                                 mma_f16(dcol, acol + (sa * KA + a) * (MT * (KT / 2)),
-                                        desc0 + (uint64_t)((sb * KA + a) * (bbytes >> 4) + o), idesc, acc);
-                                acc = 1;
-                            }
+                                        desc0 + (uint64_t)((sb * KA + a) * (bbytes >> 4) + s_off[m][j + a]), idesc,
+                                        a > 0 ? 1u : acc);
                         }
+                        acc = 1;
                         mma_commit(&empty[sb]);
                     }
                 }
@@ -387,10 +529,7 @@ __global__ void __launch_bounds__(kThreads, KA <= 2 ? 4 : 2)
             ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
             if (!ok) break;
         }
-        if (!produce && lane == 0) {
-            if (m == 0) s_live = (int)acc;  // read after the CTA barrier below
-            mma_commit(&done);
-        }
+        if (!produce && lane == 0) mma_commit(&done);
     }
     __syncwarp();
     bool ok = true;
@@ -401,7 +540,6 @@ __global__ void __launch_bounds__(kThreads, KA <= 2 ? 4 : 2)
         tc_fence_after();
         if (__all_sync(0xffffffffu, ok)) {
             const size_t plane = args.plane;
-            const bool live = s_live != 0, flagged = s_flagged != 0;
             const uint32_t nz = min(args.ns, args.nz - z0);
             for (int h = 0; h < MT; h++) {
                 const int y = py + h * MY;
@@ -413,8 +551,7 @@ __global__ void __launch_bounds__(kThreads, KA <= 2 ? 4 : 2)
                     float v[16];
                     tmem_ld16(taddr + c, r);
 #pragma unroll
-                    for (int i = 0; i < 16; i++) v[i] = live ? __uint_as_float(r[i]) * 8192.0f : 0.0f;
-                    if (flagged && in) add_flagged(args, bx, by + (float)(h * MY), z0 + c, v);
+                    for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]) * 8192.0f;
                     if (in) {
 #pragma unroll
                         for (int i = 0; i < 16; i++)
@@ -435,6 +572,7 @@ __global__ void __launch_bounds__(kThreads, KA <= 2 ? 4 : 2)
     }
     __syncthreads();
     if (warp == kBuildWarps) tmem_dealloc(tmem, args.tmem_cols);
+    if (s_any && !s_abort) store_nonfinite(args);
 }
 
 // Map over the slice octets [groups][P][W] of 16-byte cells; box = KW cells x 1 angle x box_groups.
@@ -499,6 +637,27 @@ uint32_t bp_umma_slices(uint32_t nz)
     return best;
 }
 
+size_t umma_flag_bytes(uint32_t P, uint32_t nz)
+{
+    const size_t octs = (nz + 7) / 8;
+    return octs * P * (sizeof(uint2) + sizeof(int2)) + octs * 4;
+}
+
+ufob_status umma_finite_launch(const BPGeometry &g, void *d_sino, uint32_t pitch, uint64_t group_pitch,
+                               uint8_t *d_flags, cudaStream_t stream)
+{
+    const uint32_t octs = (g.nz + 7) / 8;
+    if (!octs || !g.P) return UFOB_OK;
+    const size_t words = (size_t)octs * g.P;
+    uint2 *flags = reinterpret_cast<uint2 *>(d_flags);
+    int2 *ranges = reinterpret_cast<int2 *>(flags + words);
+    k_octs_finite<<<octs, 1024, 0, stream>>>(reinterpret_cast<uint4 *>(d_sino), g.W, pitch, group_pitch, g.P, flags,
+                                             ranges, reinterpret_cast<uint32_t *>(ranges + words));
+    UFOB_CUDA_TRY(cudaGetLastError());
+    note_launch();
+    return UFOB_OK;
+}
+
 ufob_status bp_umma_launch(const BPGeometry &g, const void *d_sino, uint32_t pitch, uint64_t group_pitch,
                            const uint8_t *d_flags, float *d_out, uint64_t plane, cudaStream_t stream)
 {
@@ -519,7 +678,10 @@ ufob_status bp_umma_launch(const BPGeometry &g, const void *d_sino, uint32_t pit
     a.W = g.W;
     a.pitch = pitch;
     a.group_pitch = group_pitch;
-    a.flags = d_flags;
+    const size_t words = (size_t)((g.nz + 7) / 8) * g.P;
+    a.flags = reinterpret_cast<const uint2 *>(d_flags);
+    a.ranges = reinterpret_cast<const int2 *>(a.flags + words);
+    a.any = reinterpret_cast<const uint32_t *>(a.ranges + words);
     a.out = d_out;
     a.plane = plane;
     a.err = device_error_word();

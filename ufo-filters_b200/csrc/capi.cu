@@ -699,7 +699,7 @@ struct ufob_fbp {
     ufob_backproject *bp = nullptr;
     ufob_dtype storage = UFOB_F32;
     DevBuf work;        // filtered sinograms of one slice group
-    DevBuf flags;       // its angles with a non-finite value (slice octets)
+    DevBuf flags;       // where it is not finite (slice octets)
     DevBuf hin[2];      // device staging of host input chunks
     DevBuf hout[2];     // device staging of host output chunks
     cudaStream_t s_copy = nullptr, s_comp = nullptr, s_d2h = nullptr;  // uploads, compute, downloads
@@ -834,10 +834,12 @@ extern "C" ufob_status ufob_stacked_bp_run(ufob_stacked_bp *sb, const float *d_s
         BPGeometry g;
         UFOB_TRY(bp_prepare(sb->bp, width, height, nslices, g, s));
         UFOB_TRY(sb->work.ensure((size_t)((nslices + 7) / 8) * height * width * 16));
-        UFOB_TRY(sb->flags.ensure(height));
-        UFOB_CUDA_TRY(cudaMemsetAsync(sb->flags.ptr, 0, height, s));
-        UFOB_TRY(pack_octs_launch(d_sino, width, height, nslices, sb->work.ptr, sb->flags.as<uint8_t>(), s));
-        return bp_umma_launch(g, sb->work.ptr, width, (uint64_t)width * height, sb->flags.as<uint8_t>(), d_out, (uint64_t)g.roi_w * g.roi_h, s);
+        UFOB_TRY(sb->flags.ensure(umma_flag_bytes(height, nslices)));
+        uint8_t *flags = sb->flags.as<uint8_t>();
+        const uint64_t group_pitch = (uint64_t)width * height, plane = (uint64_t)g.roi_w * g.roi_h;
+        UFOB_TRY(pack_octs_launch(d_sino, width, height, nslices, sb->work.ptr, flags, s));
+        UFOB_TRY(umma_finite_launch(g, sb->work.ptr, width, group_pitch, flags, s));
+        return bp_umma_launch(g, sb->work.ptr, width, group_pitch, flags, d_out, plane, s);
     }
     if (sb->precision == 1) {  // few slices: FP16 slice-quad cells, FP32 sums
         const uint32_t cells = width + 1;
@@ -881,7 +883,7 @@ static ufob_status fbp_group(ufob_fbp *x, const RowSource &src, uint32_t width, 
     const size_t work_bytes = umma    ? (size_t)pitch * 16 * height * ((nz + 7) / 8)
                               : quads ? (size_t)pitch * 16 * height * ((nz + 3) / 4) : (size_t)pitch * 4 * height * nz;
     UFOB_TRY(x->work.ensure(work_bytes));
-    if (umma) UFOB_TRY(x->flags.ensure(height));
+    if (umma) UFOB_TRY(x->flags.ensure(umma_flag_bytes(height, nz)));
     cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr;
     if (x->timing) {
         e0 = x->next_event();
@@ -892,7 +894,6 @@ static ufob_status fbp_group(ufob_fbp *x, const RowSource &src, uint32_t width, 
     }
     const ufob_layout layout = quads ? UFOB_LAYOUT_QUADS : pairs ? UFOB_LAYOUT_PAIRS : UFOB_LAYOUT_ROWS;
     if (umma) {
-        UFOB_CUDA_TRY(cudaMemsetAsync(x->flags.ptr, 0, height, s));
         UFOB_TRY(filter_octs_launch_src(x->f->plan, src, width, height, nz, x->work.ptr, x->flags.as<uint8_t>(), fw,
                                         pitch, s));
     } else if (quads)
@@ -904,6 +905,7 @@ static ufob_status fbp_group(ufob_fbp *x, const RowSource &src, uint32_t width, 
     if (umma) {
         BPGeometry g;
         UFOB_TRY(bp_prepare(x->bp, fw, height, nz, g, s));
+        UFOB_TRY(umma_finite_launch(g, x->work.ptr, pitch, (uint64_t)pitch * height, x->flags.as<uint8_t>(), s));
         // whole tile rows per band: the same tiles, and the same results, as in one launch
         const uint32_t oh = g.roi_h, y0 = g.roi_y, rows = round_up((oh + bands - 1) / bands, kUmmaTileRows);
         for (uint32_t y = 0; y < oh; y += rows) {

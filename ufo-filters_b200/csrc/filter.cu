@@ -360,8 +360,22 @@ __device__ __forceinline__ uint32_t pack_pair(float lo, float hi)
     }
 }
 
-// Whether a pair of halves holds an infinity or a NaN (exponent bits all set).
+// Bits 15 and 31: the lower and the upper of a pair of halves is an infinity or a NaN (exponent bits all set).
 __device__ __forceinline__ uint32_t half2_nonfinite(uint32_t w) { return ((w & 0x7C007C00u) + 0x04000400u) & 0x80008000u; }
+
+// Flag bytes of an item's two slices: cleared by one thread before the transforms (whose barriers order
+// it before the stores), set by those that store a non-finite value.
+template <int OUT>
+__device__ __forceinline__ void clear_flags(uint8_t *flags, uint32_t cell, uint32_t part)
+{
+    if (OUT == OUT_F16_OCTS) *reinterpret_cast<uint16_t *>(flags + (size_t)cell * 8 + 2 * part) = 0;
+}
+
+__device__ __forceinline__ void set_flags(uint8_t *flags, uint32_t cell, uint32_t part, uint32_t bad)
+{
+    if (bad & 0x8000u) flags[(size_t)cell * 8 + 2 * part] = 1;
+    if (bad >> 31) flags[(size_t)cell * 8 + 2 * part + 1] = 1;
+}
 
 // Rows of one work item (one complex FFT of a + i b): rows 2*pair and
 // 2*pair+1, or for the slice-cell layouts (OUT_F16_QUADS with I = 2 items per
@@ -369,7 +383,7 @@ __device__ __forceinline__ uint32_t half2_nonfinite(uint32_t w) { return ((w & 0
 // (group * P + angle) * I + part, i.e. slices 2*(I*group + part) and the one
 // after it at one angle.
 struct PairMap {
-    uint32_t ra, rb, part, angle;
+    uint32_t ra, rb, part, cell;  // cell: (group, angle), as the rows of cells lie
     bool hasa, hasb;
     size_t cell0;
 };
@@ -380,7 +394,7 @@ __device__ __forceinline__ PairMap map_pair(uint32_t pair, uint32_t rows, uint32
     PairMap m;
     m.ra = 2 * pair;
     m.rb = 2 * pair + 1;
-    m.part = m.angle = 0;
+    m.part = m.cell = 0;
     m.cell0 = 0;
     m.hasa = m.ra < rows;
     if constexpr (cell_items<OUT>() > 0) {
@@ -388,7 +402,7 @@ __device__ __forceinline__ PairMap map_pair(uint32_t pair, uint32_t rows, uint32
         const uint32_t gp = pair / I;  // group * P + angle
         m.part = pair % I;
         const uint32_t grp = gp / P, ang = gp - grp * P;
-        m.angle = ang;
+        m.cell = gp;
         m.ra = 2 * (I * grp + m.part) * P + ang;
         m.rb = m.ra + P;
         m.hasa = m.ra < rows;
@@ -427,7 +441,7 @@ __device__ __forceinline__ void store_pair(const PairMap &m, GET X, void *__rest
             bad |= half2_nonfinite(w);
             o[(size_t)j * 4 + m.part] = w;
         }
-        if (bad) flags[m.angle] = 1;
+        if (bad) set_flags(flags, m.cell, m.part, bad);
     } else if (OUT == OUT_F16_PAIRS || OUT == OUT_BF16_PAIRS) {
         uint32_t *o = reinterpret_cast<uint32_t *>(out);
         for (uint32_t j = t0; j < out_pitch; j += step) {
@@ -454,6 +468,7 @@ __device__ __forceinline__ void filter_pair(const RowSource &src, uint32_t width
                                             uint32_t out_pitch, uint32_t P = 0, uint8_t *flags = nullptr)
 {
     const PairMap m = map_pair<OUT>(pair, rows, P, out_pitch);
+    if (threadIdx.x == 0) clear_flags<OUT>(flags, m.cell, m.part);
     uint32_t ya, pa_proj, yb, pb_proj;
     const float *pa = row_start(src, m.hasa ? m.ra : 0, ya, pa_proj);
     const float *pb = row_start(src, m.hasb ? m.rb : 0, yb, pb_proj);
@@ -789,6 +804,7 @@ __global__ void __launch_bounds__(kFastThreads, 2) k_filter_fast(const RowSource
         const uint32_t pair = (it * gridDim.x + blockIdx.x) * TEAMS + team;
         const bool live = pair < npairs;
         const PairMap m = map_pair<OUT>(live ? pair : 0, live ? rows : 0, P, out_pitch);
+        if (live && t == 0) clear_flags<OUT>(flags, m.cell, m.part);
         // pass 1 loads elements t + m N/16 of rows a, b (staged, or straight from global memory)
         float2 v[16];
         bool failed = false;
@@ -926,13 +942,15 @@ __global__ void __launch_bounds__(kFastThreads, 2) k_filter_fast(const RowSource
                 } else {
                     // four of the eight slices: half a cell
                     uint2 *o = reinterpret_cast<uint2 *>(out) + m0.cell0 * 2 + (m0.part >> 1);
-                    uint32_t bad = 0;
+                    uint32_t bad0 = 0, bad1 = 0;
                     for (uint32_t j = i0; j < out_pitch; j += 2 * T) {
                         const uint2 w = make_uint2(taps(X0, m0, j, false), taps(X1, m1, j, false));
-                        bad |= half2_nonfinite(w.x) | half2_nonfinite(w.y);
+                        bad0 |= half2_nonfinite(w.x);
+                        bad1 |= half2_nonfinite(w.y);
                         o[(size_t)j * 2] = w;
                     }
-                    if (bad) flags[m0.angle] = 1;
+                    if (bad0) set_flags(flags, m0.cell, m0.part, bad0);
+                    if (bad1) set_flags(flags, m1.cell, m1.part, bad1);
                 }
             }
         } else {
@@ -1142,8 +1160,8 @@ ufob_status filter_quads_launch_src(const FilterPlan &plan, const RowSource &src
 }
 
 // The same into slice octets: [ceil(nz/8)][P][out_pitch] cells of 16 bytes, cell j of a row
-// holding bin j of eight slices; d_flags[P] (zeroed by the caller) is set to 1 for every angle with
-// a non-finite value (see bp_umma.cu).
+// holding bin j of eight slices; d_flags[octets][P][8] tells which slices have a non-finite value at
+// which angles (see bp_umma.cu).
 ufob_status filter_octs_launch_src(const FilterPlan &plan, const RowSource &src, uint32_t width, uint32_t P,
                                    uint32_t nz, void *d_out, uint8_t *d_flags, uint32_t out_w, uint32_t out_pitch,
                                    cudaStream_t stream)

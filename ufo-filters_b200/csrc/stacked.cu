@@ -69,13 +69,14 @@ ufob_status pack_quads_launch(const float *d_in, uint32_t W, uint32_t P, uint32_
 
 // ------------------------------------------------------------ FP32 stack -> slice octets
 
-// cell (g, p, j): halves of bin j of slices 8g..8g+7; flags[p] = 1 where one is not finite
+// cell (g, p, j): halves of bin j of slices 8g..8g+7; byte k of flags[g * P + p] = 1 where slice 8g + k is
+// not finite
 __global__ void k_pack_octs(const float *__restrict__ in, uint32_t W, uint32_t P, uint32_t Z, uint4 *__restrict__ out,
-                            uint8_t *__restrict__ flags)
+                            uint2 *__restrict__ flags)
 {
     const uint32_t g = blockIdx.y;
     for (uint32_t p = blockIdx.x; p < P; p += gridDim.x) {
-        uint32_t bad = 0;
+        uint32_t bad[4] = {};
         for (uint32_t j = threadIdx.x; j < W; j += blockDim.x) {
             uint32_t w[4];
 #pragma unroll
@@ -85,11 +86,18 @@ __global__ void k_pack_octs(const float *__restrict__ in, uint32_t W, uint32_t P
                 const float a = z < Z ? __ldg(row) : 0.f, b = z + 1 < Z ? __ldg(row + (uint64_t)P * W) : 0.f;
                 const __half2 h = __floats2half2_rn(a, b);
                 w[k] = *reinterpret_cast<const uint32_t *>(&h);
-                bad |= ((w[k] & 0x7C007C00u) + 0x04000400u) & 0x80008000u;
+                bad[k] |= ((w[k] & 0x7C007C00u) + 0x04000400u) & 0x80008000u;
             }
             out[((uint64_t)g * P + p) * W + j] = make_uint4(w[0], w[1], w[2], w[3]);
         }
-        if (bad) flags[p] = 1;
+        uint2 f = make_uint2(0, 0);
+        if (__syncthreads_or((int)(bad[0] | bad[1] | bad[2] | bad[3]))) {
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+                if (__syncthreads_or((int)(bad[k / 2] & (k & 1 ? 0x80000000u : 0x8000u))))
+                    (k < 4 ? f.x : f.y) |= 1u << (8 * (k & 3));
+        }
+        if (threadIdx.x == 0) flags[(uint64_t)g * P + p] = f;
     }
 }
 
@@ -99,7 +107,8 @@ ufob_status pack_octs_launch(const float *d_in, uint32_t W, uint32_t P, uint32_t
     const uint32_t groups = (Z + 7) / 8;
     if (!groups || !P || !W) return UFOB_OK;
     dim3 grid(std::min<uint32_t>(P, std::max<uint32_t>(1, (uint32_t)num_sms() * 16 / groups)), groups);
-    k_pack_octs<<<grid, 256, 0, s>>>(d_in, W, P, Z, reinterpret_cast<uint4 *>(d_out), d_flags);
+    k_pack_octs<<<grid, 256, 0, s>>>(d_in, W, P, Z, reinterpret_cast<uint4 *>(d_out),
+                                 reinterpret_cast<uint2 *>(d_flags));
     UFOB_CUDA_TRY(cudaGetLastError());
     note_launch();
     return UFOB_OK;

@@ -207,8 +207,8 @@ ufob_status filter_rows_launch_src(const FilterPlan &plan, const RowSource &src,
 ufob_status filter_quads_launch_src(const FilterPlan &plan, const RowSource &src, uint32_t width, uint32_t P,
                                     uint32_t nz, void *d_out, uint32_t out_w, uint32_t out_pitch,
                                     cudaStream_t stream);
-// Slice-octet output, as the tensor-core backprojector reads it; d_flags[P], zeroed before,
-// marks the angles that hold a non-finite value.
+// Slice-octet output for the tensor-core backprojector; byte k of d_flags[octets][P][8] is set to 1 where
+// slice k of the octet has a non-finite value at the angle, and to 0 elsewhere.
 ufob_status filter_octs_launch_src(const FilterPlan &plan, const RowSource &src, uint32_t width, uint32_t P,
                                    uint32_t nz, void *d_out, uint8_t *d_flags, uint32_t out_w, uint32_t out_pitch,
                                    cudaStream_t stream);
@@ -276,7 +276,11 @@ ufob_status pack_cells_launch(const float *d_in, uint32_t pitch, uint64_t slice_
                               uint32_t Z, void *d_out, cudaStream_t s);
 // The same on the tensor cores from slice octets [ceil(nz/8)][P][pitch] (pitch and group_pitch in
 // 16-byte cells), slices `plane` floats apart in the output.  Its tiles are kUmmaTileRows rows high.
+// Octets and flags, umma_flag_bytes() of them, pass through umma_finite_launch() before.
 constexpr uint32_t kUmmaTileRows = 20;
+size_t umma_flag_bytes(uint32_t P, uint32_t nz);
+ufob_status umma_finite_launch(const BPGeometry &g, void *d_sino, uint32_t pitch, uint64_t group_pitch,
+                               uint8_t *d_flags, cudaStream_t stream);
 ufob_status bp_umma_launch(const BPGeometry &g, const void *d_sino, uint32_t pitch, uint64_t group_pitch,
                            const uint8_t *d_flags, float *d_out, uint64_t plane, cudaStream_t stream);
 
