@@ -59,6 +59,34 @@ def test_angle_counts(cuda, nz, P):
     assert oracle.rel_l2(_fbp(raw, 64), _ref(raw, 64)) < TOL
 
 
+# blocks of 64 angles whose sums are added to the totals: block ends, for either split of the totals
+# between registers and shared memory (up to 32, 64, 96 and 128 slices)
+@pytest.mark.parametrize("nz", [17, 33, 65, 128])
+@pytest.mark.parametrize("P", [63, 64, 65, 127, 128, 129, 200])
+def test_angle_blocks(cuda, nz, P):
+    raw = _raw(nz, P, 40, P)
+    got, ref = _fbp(raw, 64), _ref(raw, 64)
+    for z in range(nz):
+        assert oracle.rel_l2(got[z], ref[z]) < TOL, z
+
+
+# Large sums of one sign, as of rows that were not filtered: the tensor cores cut each addition off at the
+# accumulator's last bit, on average half of 2^-23 of the sum so far.  In a block of 64 angles that is at
+# most 64 / 4 * 2^-23 = 1.9e-6 of its sum; the weights' rounding (2^-12 at most, 2^-12 / sqrt(3) in the mean)
+# of neighbouring bins 0.4 apart adds 0.4 * 1.4e-4 / sqrt(1500) = 1.5e-6 and FP32 totals less.  (One sum over
+# all 1500 angles: 3.8e-5.)  The reference takes the rows as stored, rounded to 16 bits.
+@pytest.mark.parametrize("nz", [20, 50, 120])
+def test_sums_of_one_sign(cuda, nz):
+    P, W = 1500, 96
+    raw = np.random.default_rng(nz).uniform(1.0, 2.0, (nz, P, W)).astype(np.float16).astype(np.float32)
+    t = ufob.StackedBackprojectTask(precision_mode="half", axis_pos=W / 2)
+    got = t.process(torch.from_numpy(raw).cuda()).cpu().numpy()
+    ufob.device_status()
+    for z in (0, nz - 1):
+        ref = oracle.stacked_backproject(raw[z:z + 1], "single", axis_pos=W / 2)[0]
+        assert oracle.rel_l2(got[z], ref) < 5e-6, z
+
+
 # the issuing lanes read window starts that the other lanes of their warps write, anew for every 32
 # angles: passes over seven such groups agree to the bit, for each stage length
 @pytest.mark.parametrize("nz", [20, 50, 120])

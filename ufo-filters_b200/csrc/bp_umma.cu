@@ -26,15 +26,22 @@
 //     0..2048 read as FP16 are n * 2^-24 exactly (subnormals and the first normals), so the
 //     accumulators count in 2^-13 of the sum.  Errors of the weights are at most 2^-12 (the
 //     slice-quad kernel: 10 fractional bits).
-//   Accumulators: FP32 in tensor memory over all angles, MT * ns columns.
+//   Accumulators: FP32 in tensor memory, MT * ns columns, over blocks of 64 angles whose sums the
+//     builders add to totals in registers and shared memory.  The tensor cores cut an addition off at the
+//     accumulator's last bit: one sum over 1500 angles of rows in [1, 2) is 3.9e-5 too small, 6000 angles
+//     1.6e-4, with blocks 1.1e-6 for any number (the slice-quad kernel's error, rounding of the rows
+//     included, 4.6e-6 and 2.3e-6; this one's 4.3e-6 and 2.4e-6).  Costs 1.1 of 15.1 ms for 32 slices, 0.9 of
+//     16.8 for 64; blocks of 32 angles 0.5 to 1 ms more, of 128 a bias of 2.2e-6.
 //
 // Roles of a CTA: four builder warps, a producer warp (one TMA per angle), an MMA warp per
 // accumulator (the issuing lane's instructions, not the tensor pipe, limit one warp for both: 29
 // against 24 ms).  Stages of KA angles; SA stages of weights, SB of windows; a stage's products
 // arrive on one barrier that frees its weights and its windows.  What bounds it is the fixed cost
-// of a stage (barriers, issue latencies), so small CTAs (KA = 2, four per SM) run up to 32 slices
-// and larger stages (KA = 4, 8) the cases that leave room for fewer CTAs.  2048^2 x 1500 angles, ms per
-// pass: ns <= 32 15.5, 64 16.6, 96 24.2, 128 29.0 (13.0, 24.3, 25.0, 27.8 TGUPS; slice quads 6.6).
+// of a stage (barriers, issue latencies), so up to 64 slices two CTAs share an SM (KA = 4); above,
+// tensor memory holds one CTA, whose stages are longer (KA = 8) and whose totals are mostly registers.
+// 2048^2 x 1500 angles, ms per pass: ns <= 32 16.2, 64 17.6, 96 23.6, 128 28.9 (12.4, 22.9, 25.6,
+// 27.9 TGUPS; slice quads 6.6).  Four CTAs per SM with KA = 2 up to 32 slices: 16.2 (2% faster without the
+// totals, which then are all in shared memory); two with KA = 2 for 96: 26.4.
 //
 // A non-finite value of a window would reach every pixel of its tile (0 * inf).  The filter flags
 // the slices and angles that have one; k_octs_finite puts -0 in the place of such values in these rows
@@ -62,18 +69,24 @@ static_assert(MT * MY == kUmmaTileRows, "tile height");
 constexpr int KT = 16;           // taps of one product
 constexpr int KW = 28;           // staged bins: KT + 10 |sin| + 1, rounded up
 constexpr int SA = 2;            // stages of weights
+constexpr int kBlock = 64;       // angles per sum in tensor memory
 constexpr int kBuildWarps = 4;
 constexpr int kThreads = 32 * (kBuildWarps + 1 + MT);
 enum { CLASS_NAN = 1, CLASS_POS = 2, CLASS_NEG = 4 };  // flag bytes: what the -0 of a row stand for
 constexpr int kErrUmmaTimeout = 0x1003;
 
-// KA angles per stage.
-template <int KA>
+// KA angles per stage, SB stages of windows, CTAs per SM, and how many 16-column chunks of a builder
+// thread's totals are in registers (the others in shared memory).
+template <int KA_, int SB_, int CTAS_, int RC_>
 struct UmmaShape {
-    static constexpr int SB = 16 / KA;  // stages of windows
+    static constexpr int KA = KA_, SB = SB_, CTAS = CTAS_, RC = RC_;
     static constexpr uint32_t kACols = SA * KA * MT * (KT / 2);  // tensor-memory columns of the weights
     static constexpr uint32_t window_bytes(uint32_t ns) { return ns * KW * 2; }  // one angle, all slices
-    static constexpr uint32_t smem(uint32_t ns) { return SB * KA * window_bytes(ns) + 128; }
+    static constexpr uint32_t totals_bytes(uint32_t ns)
+    {
+        return MT * ns > 16u * RC ? (MT * ns - 16 * RC) * MX * MY * 4 : 0;
+    }
+    static constexpr uint32_t smem(uint32_t ns) { return SB * KA * window_bytes(ns) + totals_bytes(ns) + 128; }
 };
 
 __device__ __forceinline__ void tmem_alloc(uint32_t *slot, uint32_t ncols)
@@ -111,6 +124,7 @@ __device__ __forceinline__ void mma_commit(uint64_t *bar)
                  : "memory");
 }
 
+// Sixteen columns of a warp's lanes; the registers hold them after tmem_wait16.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16])
 {
     asm volatile(
@@ -119,7 +133,15 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16])
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
           "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void tmem_wait16(uint32_t (&r)[16])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+                 :
+                 : "memory");
 }
 
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
@@ -350,15 +372,15 @@ __global__ void __launch_bounds__(1024) k_octs_finite(uint4 *__restrict__ cells,
     if (threadIdx.x == 0) any[g] = s_any;
 }
 
-template <int KA>
-__global__ void __launch_bounds__(kThreads, KA <= 2 ? 4 : 2)
+template <typename Sh>
+__global__ void __launch_bounds__(kThreads, Sh::CTAS)
     k_bp_umma(const __grid_constant__ CUtensorMap map, const __grid_constant__ UmmaArgs args)
 {
-    using Sh = UmmaShape<KA>;
-    constexpr int SB = Sh::SB;
-    static_assert(32 % KA == 0 && SB >= SA, "whole stages per 32 angles; one barrier ring serves both slots");
+    constexpr int KA = Sh::KA, SB = Sh::SB, RC = Sh::RC;
+    static_assert(32 % KA == 0 && kBlock % 32 == 0 && SB >= SA,
+                  "whole stages per 32 angles; one barrier ring serves both slots");
     extern __shared__ unsigned char smem_dyn[];
-    __shared__ uint64_t full_a[SA], full_b[SB], empty[SB], done;
+    __shared__ uint64_t full_a[SA], full_b[SB], empty[SB], added, done;
     __shared__ float4 s_tab[kBuildWarps][32];
     __shared__ int s_win[32];
     __shared__ uint32_t s_off[MT][32];
@@ -388,6 +410,7 @@ __global__ void __launch_bounds__(kThreads, KA <= 2 ? 4 : 2)
             mbar_init(&full_b[s], 1);
             mbar_init(&empty[s], MT);
         }
+        mbar_init(&added, kBuildWarps);
         mbar_init(&done, MT);
         s_abort = 0;
         fence_barrier_init();
@@ -409,6 +432,44 @@ __global__ void __launch_bounds__(kThreads, KA <= 2 ? 4 : 2)
     const float bx = (float)(args.roi_x + px) - axis + 0.5f;
     const float by = (float)(args.roi_y + py) - axis + 0.5f;
 
+    // Totals of a builder thread's pixels over the blocks added so far, as 16-column chunks of the
+    // accumulators' columns: registers, then shared memory.
+    const uint32_t chunks = MT * args.ns / 16;
+    float4 *totals = reinterpret_cast<float4 *>(gbase + SB * KA * bbytes) + row;
+    float tot[RC > 0 ? 16 * RC : 1];
+    const uint32_t tlane = tmem + ((uint32_t)(warp & 3) << 21);
+    // adds the accumulators' sums, whose products are done, and lets the next block's begin
+    auto add_block = [&](bool first) {
+        tc_fence_after();
+        uint32_t r[16];
+#pragma unroll
+        for (int q = 0; q < RC; q++) {
+            tmem_ld16(tlane + 16 * q, r);
+            tmem_wait16(r);
+#pragma unroll
+            for (int i = 0; i < 16; i++) tot[16 * q + i] = __uint_as_float(r[i]) + (first ? 0.0f : tot[16 * q + i]);
+        }
+#pragma unroll 1
+        for (uint32_t q = RC; q < chunks; q++) {
+            float4 *t = totals + (q - RC) * 4 * (MX * MY), v[4];
+            tmem_ld16(tlane + 16 * q, r);
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                v[i] = first || row >= MX * MY ? make_float4(0.f, 0.f, 0.f, 0.f) : t[i * (MX * MY)];
+            tmem_wait16(r);
+            if (row < MX * MY)
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    t[i * (MX * MY)] = make_float4(v[i].x + __uint_as_float(r[4 * i]), v[i].y + __uint_as_float(r[4 * i + 1]),
+                                                   v[i].z + __uint_as_float(r[4 * i + 2]),
+                                                   v[i].w + __uint_as_float(r[4 * i + 3]));
+            __syncwarp();
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&added);
+    };
+
     if (warp < kBuildWarps) {
         const float kFix = 6144.0f;  // 1.5 * 2^12: 11 fractional bits left in the mantissa
         const uint32_t ta = tmem + MT * args.ns + ((uint32_t)warp << 21);
@@ -416,6 +477,14 @@ __global__ void __launch_bounds__(kThreads, KA <= 2 ? 4 : 2)
         float4 *tab = s_tab[warp];
         bool ok = true;
         for (uint32_t p0 = 0; p0 < P && ok; p0 += 32) {
+            if (p0 && p0 % kBlock == 0) {
+                // the sums of the block that ended with the group before, once its products are done
+                const uint32_t prev = p0 / KA - 1;
+                ok = wait_or_abort(&empty[prev % SB], (prev / SB) & 1u, abort_flag);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                add_block(p0 == kBlock);
+            }
             {
                 const float2 sc = __ldg(&args.sincos[min(p0 + lane, P - 1)]);
                 __syncwarp();
@@ -487,7 +556,12 @@ __global__ void __launch_bounds__(kThreads, KA <= 2 ? 4 : 2)
                 __syncwarp();  // the issuing lane reads the other lanes' entries
             }
             const uint32_t n = min(32u, P - p0);
-            if (lane == 0) {
+            if (!produce && p0 % kBlock == 0) {
+                // a block's first products overwrite the sums of the one before, once these are added
+                acc = 0;
+                if (p0 && lane == 0) ok = wait_or_abort(&added, (p0 / kBlock - 1) & 1u, abort_flag);
+            }
+            if (lane == 0 && ok) {
                 for (uint32_t j = 0; j < n; j += KA) {
                     const uint32_t it = (p0 + j) / KA, sb = it % SB, sa = it % SA;
                     const uint32_t nval = min((uint32_t)KA, n - j);
@@ -541,23 +615,41 @@ __global__ void __launch_bounds__(kThreads, KA <= 2 ? 4 : 2)
         if (__all_sync(0xffffffffu, ok)) {
             const size_t plane = args.plane;
             const uint32_t nz = min(args.ns, args.nz - z0);
-            for (int h = 0; h < MT; h++) {
-                const int y = py + h * MY;
-                const bool in = row < MX * MY && px < (int)args.roi_w && y < (int)args.roi_h;
-                const uint32_t taddr = tmem + (uint32_t)h * args.ns + ((uint32_t)warp << 21);
-                float *o = args.out + (size_t)z0 * plane + (size_t)y * args.roi_w + px;
-                for (uint32_t c = 0; c < nz; c += 16) {
-                    uint32_t r[16];
-                    float v[16];
-                    tmem_ld16(taddr + c, r);
+            const bool added_some = P > kBlock;
+            // chunk q, with the totals so far in v
+            auto store = [&](uint32_t q, float (&v)[16]) {
+                const uint32_t h = 16 * q >= args.ns, c = 16 * q - h * args.ns;
+                const int y = py + (int)h * MY;
+                if (c >= nz) return;
+                uint32_t r[16];
+                tmem_ld16(tlane + 16 * q, r);
+                tmem_wait16(r);
+                if (row < MX * MY && px < (int)args.roi_w && y < (int)args.roi_h) {
+                    float *o = args.out + (size_t)(z0 + c) * plane + (size_t)y * args.roi_w + px;
 #pragma unroll
-                    for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]) * 8192.0f;
-                    if (in) {
-#pragma unroll
-                        for (int i = 0; i < 16; i++)
-                            if (c + i < nz) o[(size_t)(c + i) * plane] = v[i] * args.norm;
+                    for (int i = 0; i < 16; i++) {
+                        const float sum = (__uint_as_float(r[i]) + (added_some ? v[i] : 0.0f)) * 8192.0f;
+                        if (c + i < nz) o[(size_t)i * plane] = sum * args.norm;
                     }
                 }
+                __syncwarp();
+            };
+#pragma unroll
+            for (int q = 0; q < RC; q++) {
+                float v[16];
+#pragma unroll
+                for (int i = 0; i < 16; i++) v[i] = tot[16 * q + i];
+                if (q < (int)chunks) store(q, v);
+            }
+#pragma unroll 1
+            for (uint32_t q = RC; q < chunks; q++) {
+                float v[16] = {};
+                if (added_some && row < MX * MY) {
+                    const float4 *t = totals + (q - RC) * 4 * (MX * MY);
+#pragma unroll
+                    for (int i = 0; i < 4; i++) *reinterpret_cast<float4 *>(v + 4 * i) = t[i * (MX * MY)];
+                }
+                store(q, v);
             }
         }
         tc_fence_before();
@@ -598,15 +690,15 @@ ufob_status make_octet_map(CUtensorMap *map, const void *base, uint32_t W, uint3
     return UFOB_OK;
 }
 
-template <int KA>
-ufob_status launch(const CUtensorMap &map, UmmaArgs a, cudaStream_t stream)
+template <typename Sh>
+ufob_status launch(const CUtensorMap &map, UmmaArgs a, uint32_t most_slices, cudaStream_t stream)
 {
     a.tmem_cols = 32;
-    while (a.tmem_cols < MT * a.ns + UmmaShape<KA>::kACols) a.tmem_cols *= 2;
+    while (a.tmem_cols < MT * a.ns + Sh::kACols) a.tmem_cols *= 2;
     static std::atomic<uint64_t> attr_devs{0};
-    UFOB_CUDA_TRY(smem_limit_per_device(k_bp_umma<KA>, (int)UmmaShape<KA>::smem(128), attr_devs));
+    UFOB_CUDA_TRY(smem_limit_per_device(k_bp_umma<Sh>, (int)Sh::smem(most_slices), attr_devs));
     dim3 grid(a.tiles_x * a.tiles_y, (a.nz + a.ns - 1) / a.ns);
-    k_bp_umma<KA><<<grid, kThreads, UmmaShape<KA>::smem(a.ns), stream>>>(map, a);
+    k_bp_umma<Sh><<<grid, kThreads, Sh::smem(a.ns), stream>>>(map, a);
     UFOB_CUDA_TRY(cudaGetLastError());
     note_launch();
     return UFOB_OK;
@@ -616,12 +708,12 @@ ufob_status launch(const CUtensorMap &map, UmmaArgs a, cudaStream_t stream)
 
 uint32_t bp_umma_slices(uint32_t nz)
 {
-    // Time of one pass over a tile by slices per CTA (ms at 2048^2 x 1500 angles, see above): equal
+    // Time of one pass over a tile by slices per CTA (ms at 2048^2 x 1500 angles, as above): equal
     // shares of the stack that take the least in all.
     static const struct {
         uint32_t ns;
         float ms;
-    } kPass[] = {{32, 15.5f}, {64, 16.6f}, {96, 24.2f}, {128, 29.0f}};
+    } kPass[] = {{32, 16.2f}, {64, 17.6f}, {96, 23.6f}, {128, 28.9f}};
     uint32_t best = 128;
     float best_t = 1e30f;
     for (uint32_t chunks = (nz + 127) / 128; chunks <= (nz + 31) / 32; chunks++) {
@@ -690,10 +782,9 @@ ufob_status bp_umma_launch(const BPGeometry &g, const void *d_sino, uint32_t pit
     a.tiles_y = (g.roi_h + MT * MY - 1) / (MT * MY);
     CUtensorMap map;
     UFOB_TRY(make_octet_map(&map, d_sino, g.W, g.P, (g.nz + 7) / 8, pitch, group_pitch, a.ns / 8));
-    // angles per stage by what the accumulators leave of the 512 tensor-memory columns
-    if (a.ns <= 32 || (a.ns > 64 && a.ns <= 96)) return launch<2>(map, a, stream);
-    if (a.ns <= 64) return launch<4>(map, a, stream);
-    return launch<8>(map, a, stream);
+    // two CTAs per SM while the accumulators and four angles' weights of both fit in tensor memory
+    if (a.ns <= 64) return launch<UmmaShape<4, 4, 2, 4>>(map, a, 64, stream);
+    return launch<UmmaShape<8, 3, 1, 12>>(map, a, 128, stream);
 }
 
 }  // namespace ufob
