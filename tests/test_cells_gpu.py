@@ -68,3 +68,27 @@ def test_unaligned_rows(cuda):
                                                    (W + 2) * P, o.data_ptr(), torch.cuda.current_stream().cuda_stream))
     torch.cuda.synchronize()
     assert torch.equal(out[0], out[1])
+
+
+# One handle driven on several streams by one thread: the cells of a call must not be packed while another
+# call's kernel still reads the buffer (the table is built, and the buffer grown, by the first call).
+@pytest.mark.parametrize("make", [lambda: ufob.BackprojectTask(axis_pos=190.0),
+                                  lambda: ufob.StackedBackprojectTask(precision_mode="single", axis_pos=190.0)])
+def test_two_streams(cuda, make):
+    nz, P, W = 70, 120, 384
+    task = make()
+    stacks = [torch.randn(nz, P, W, device="cuda") for _ in range(2)]
+    want = [task.process(x).clone() for x in stacks]
+    outs = [torch.empty_like(w) for w in want]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    for _ in range(5):
+        for o in outs:
+            o.zero_()
+        torch.cuda.synchronize()
+        for x, o, st in zip(stacks, outs, streams):
+            task.process(x, out=o, stream=st)
+        torch.cuda.synchronize()
+        for o, w in zip(outs, want):
+            assert torch.equal(o, w)
+    ufob.device_status()

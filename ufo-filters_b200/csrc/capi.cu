@@ -376,12 +376,17 @@ struct ufob_backproject {
     ufob_bp_props props;
     DevBuf sincos;
     DevBuf aligned;  // copy of a sinogram whose pitch is not TMA-compatible
-    DevBuf cells;    // slice cells of a group of an FP32 stack
+    DevBuf cells;    // slice cells of a group of an FP32 stack, which one call at a time may use:
+    cudaEvent_t cells_free = nullptr;  // after the last one's kernels, for calls on other streams
     DevBuf partial;  // per-angle-group images of one small sinogram (split_plan)
     // cache key of the sin/cos table
     uint32_t key_P = 0, key_nproj = 0, key_offset = 0;
     double key_step = 0, key_aoff = 0;
     bool mirror = false;  // stacked-backproject orientation (-sin table)
+    ~ufob_backproject()
+    {
+        if (cells_free) cudaEventDestroy(cells_free);
+    }
 };
 
 extern "C" {
@@ -649,10 +654,14 @@ extern "C" ufob_status ufob_backproject_run(ufob_backproject *bp, const void *d_
     if (kind == SINO_F32 && cells_apply(bp->props, g)) {
         // slice cells by groups of 32 slices; without the memory for them the row kernel does it
         // (nor do captured graphs use them, which would keep the address of a buffer that may grow)
-        const uint32_t G = std::min(nslices, 32u);
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
+        const uint32_t G = std::min(nslices, 32u);
         if (cap == cudaStreamCaptureStatusNone && bp->cells.ensure((size_t)((G + 3) / 4) * 16 * width * height) == UFOB_OK) {
+            if (bp->cells_free)
+                UFOB_CUDA_TRY(cudaStreamWaitEvent(s, bp->cells_free, 0));
+            else
+                UFOB_CUDA_TRY(cudaEventCreateWithFlags(&bp->cells_free, cudaEventDisableTiming));
             for (uint32_t z = 0; z < nslices; z += G) {
                 BPGeometry gz = g;
                 gz.nz = std::min(G, nslices - z);
@@ -660,6 +669,7 @@ extern "C" ufob_status ufob_backproject_run(ufob_backproject *bp, const void *d_
                                            gz.nz, bp->cells.ptr, s));
                 UFOB_TRY(bp_cells_launch(gz, bp->cells.ptr, d_out + (size_t)z * g.roi_w * g.roi_h, s));
             }
+            UFOB_CUDA_TRY(cudaEventRecord(bp->cells_free, s));
             return UFOB_OK;
         }
     }
