@@ -92,3 +92,20 @@ def test_two_streams(cuda, make):
         for o, w in zip(outs, want):
             assert torch.equal(o, w)
     ufob.device_status()
+
+
+# The buffer stays within 2 GiB: eight slices of 8192 x 9000 are 2.36 GB as cells, so they run from rows.
+def test_large_sinograms_take_no_cells(cuda):
+    nz, P, W = 5, 9000, 8192
+    sino = torch.zeros(nz, P, W, device="cuda")
+    sino[:, :, ::7] = torch.rand(nz, P, (W + 6) // 7, device="cuda")
+    roi = dict(roi_x=3500, roi_y=3600, roi_width=1024, roi_height=1024)  # 512 tiles of 32 x 64
+    task = ufob.BackprojectTask(**roi)
+    out = torch.empty(nz, 1024, 1024, device="cuda")
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    task.process(sino, out=out)
+    torch.cuda.synchronize()
+    assert before - torch.cuda.mem_get_info()[0] < 64 << 20
+    want = ufob.BackprojectTask(tile=2, **roi).process(sino)
+    assert torch.equal(out, want)

@@ -56,12 +56,26 @@ ufob_status DevBuf::ensure(size_t n)
     cudaError_t e = cudaMalloc(&ptr, n);
     if (e != cudaSuccess) {
         ptr = nullptr;
-        cudaGetLastError();  // callers that can do without go on to launch
         return cuda_fail(e, "cudaMalloc");
     }
     g_device_allocs.fetch_add(1, std::memory_order_relaxed);
     bytes = n;
     return UFOB_OK;
+}
+
+bool DevBuf::grow(size_t n)
+{
+    if (n <= bytes && ptr) return true;
+    void *more = nullptr;
+    if (cudaMalloc(&more, n) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    g_device_allocs.fetch_add(1, std::memory_order_relaxed);
+    release();
+    ptr = more;
+    bytes = n;
+    return true;
 }
 
 static int g_num_sms = 0;
@@ -567,6 +581,17 @@ static bool cells_apply(const ufob_bp_props &p, const BPGeometry &g)
     return p.mode != UFOB_BP_NEAREST && p.tile < 0 && p.compensated <= 0 && p.angle_groups <= 1 && bp_cells_applies(g);
 }
 
+// Slices whose cells fit the handle's buffer: groups of 32, within 2 GiB and the memory there is, whole
+// 8-slice tiles; 0 = too few (sinograms of more than 64 M samples, or no memory), the row kernel does it.
+static uint32_t cells_group(ufob_backproject *bp, uint32_t width, uint32_t height, uint32_t nslices)
+{
+    const size_t quad = (size_t)16 * width * height, tile = 2 * quad;
+    const uint32_t most = (uint32_t)std::min<size_t>(32, (2ull << 30) / std::max<size_t>(tile, 1) * 8);
+    if (!most) return 0;
+    if (bp->cells.grow((std::min(most, nslices) + 3) / 4 * quad)) return most;
+    return (uint32_t)std::min<size_t>(32, bp->cells.bytes / tile * 8);
+}
+
 // A single sinogram is split into 2, 4 or 8 equal angle groups (at least 32 angles each) whose
 // partial images are summed, when that spreads its 32x96 tiles more evenly over the SMs: the
 // busiest SM's share of tiles over the average one drops by more than 5%; 1 = no split.
@@ -652,12 +677,12 @@ extern "C" ufob_status ufob_backproject_run(ufob_backproject *bp, const void *d_
     }
     const bool kahan = want_kahan(bp->props, kind, height);
     if (kind == SINO_F32 && cells_apply(bp->props, g)) {
-        // slice cells by groups of 32 slices; without the memory for them the row kernel does it
-        // (nor do captured graphs use them, which would keep the address of a buffer that may grow)
+        // slice cells by groups of slices (not in captured graphs, which would keep the address of a
+        // buffer that may grow)
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
-        const uint32_t G = std::min(nslices, 32u);
-        if (cap == cudaStreamCaptureStatusNone && bp->cells.ensure((size_t)((G + 3) / 4) * 16 * width * height) == UFOB_OK) {
+        const uint32_t G = cap == cudaStreamCaptureStatusNone ? cells_group(bp, width, height, nslices) : 0;
+        if (G) {
             if (bp->cells_free)
                 UFOB_CUDA_TRY(cudaStreamWaitEvent(s, bp->cells_free, 0));
             else

@@ -64,6 +64,7 @@ struct DevBuf {
         bytes = 0;
     }
     ufob_status ensure(size_t n);  // grow to at least n bytes (contents not kept)
+    bool grow(size_t n);           // the same, but without the memory for it the buffer stays as it is
     template <typename T> T *as() const { return reinterpret_cast<T *>(ptr); }
 };
 
