@@ -230,7 +230,10 @@ void ufob_stacked_bp_destroy(ufob_stacked_bp *sb);
  * variant: inputs/outputs in host memory (pinned or pageable), copies are
  * overlapped with compute on internal streams, in chunks of slices_per_chunk
  * slices (0 = 32).  F16 chunks of 17 slices and more (tensor cores) are
- * downloaded in bands of rows as they are made; otherwise, from 32 up, the
+ * downloaded in bands of rows as they are made, and a remainder of fewer than
+ * 17 slices is shared among the other chunks; with an even slices_per_chunk
+ * the results are those of one call of all slices, bit for bit.  Smaller F16 chunks run as calls of so few
+ * slices do and differ from that in the FP16 rounding.  Otherwise, from 32 up, the
  * first and the last chunk are 16 slices, so the first compute waits for a
  * short upload and little download trails the last one.
  */

@@ -198,15 +198,29 @@ def test_dead_slice_is_cheap(cuda):
     assert torch.isnan(outs[1][17, W // 4:3 * W // 4, W // 4:3 * W // 4]).all()
 
 
-# the host pipeline makes large images in bands of rows: the same bits as one launch, whole chunks
-# and a last chunk of few slices (which the slice-quad kernel takes)
-@pytest.mark.parametrize("nz,chunk", [(20, 32), (70, 32), (64, 64)])
+# the host pipeline makes large images in bands of rows, and shares a remainder of few slices among the
+# other chunks: the same bits as one call of all slices, whatever the chunks (70 slices in chunks of 32
+# were once 32 + 32 on the tensor cores and 6 on the slice-quad kernel)
+@pytest.mark.parametrize("nz,chunk", [(20, 32), (70, 32), (64, 64), (33, 32), (49, 32), (18, 17), (52, 17)])
 def test_host_bands(cuda, nz, chunk):
     P, W = 20, 1030
     raw = torch.randn(nz, P, W)
     f = ufob.FBP(filter_props={"size_x": 2048, "crop_width": W}, storage=ufob.F16)
     got = f.process_host(raw.pin_memory(), out=torch.empty(nz, W, W).pin_memory(), slices_per_chunk=chunk)
-    dev = raw.cuda()
-    parts = [f.process(dev[z:z + chunk].contiguous()).cpu() for z in range(0, nz, chunk)]
+    want = f.process(raw.cuda()).cpu()
     ufob.device_status()
-    assert torch.equal(got, torch.cat(parts))
+    assert torch.equal(got, want)
+    ref = _ref(raw[nz - 1:].numpy(), 2048)  # a slice of the last chunk
+    assert oracle.rel_l2(got[nz - 1:].numpy(), ref) < TOL
+
+
+ROI = dict(roi_x=900, roi_y=1100, roi_width=64, roi_height=48)
+
+
+# 260 slices of 1500 x 2048 are more than one group: the four left over take the kernel of the call
+def test_remainder_of_groups(cuda):
+    sino = torch.randn(260, 1500, 2048, device="cuda")
+    f = ufob.FBP(bp_props=ROI, storage=ufob.F16)
+    whole, tail = f.process(sino), f.process(sino[200:].contiguous())
+    ufob.device_status()
+    assert torch.equal(whole[200:], tail)

@@ -898,20 +898,20 @@ extern "C" void ufob_stacked_bp_destroy(ufob_stacked_bp *sb)
 }
 
 // Filter + backproject `nz` slices already on the device; logical row
-// slice * height + angle of `src` is sinogram row `angle` of slice `slice`.
+// slice * height + angle of `src` is sinogram row `angle` of slice `slice`.  `umma`: FP16 on the tensor
+// cores, as decided for the whole call.
 // With `bands`, the image is made in up to `bands` bands of rows (where the backprojector can write
 // them in place) and done(first row, rows) is called after each band's work is on the stream.
 static ufob_status fbp_group(ufob_fbp *x, const RowSource &src, uint32_t width, uint32_t height, uint32_t nz,
-                             float *d_out, cudaStream_t s, uint32_t bands = 1,
+                             bool umma, float *d_out, cudaStream_t s, uint32_t bands = 1,
                              const std::function<ufob_status(uint32_t, uint32_t)> &done = nullptr)
 {
     uint32_t nfft, fw;
     UFOB_TRY(filter_sizes(x->f->props, width, &nfft, &fw));
     UFOB_TRY(filter_plan_build(x->f->props, nfft, x->f->plan, s));
-    // F16: slice octets for the tensor cores (16 B per detector position and eight slices) or, for
+    // F16: slice octets for the tensor cores (16 B per detector position and eight slices) or, in calls of
     // few slices, slice-quad cells (16 B per detector position and four slices), or pairs for a single
     // slice (a quad cell would carry three empty slices); BF16: pairs; F32: rows
-    const bool umma = x->storage == UFOB_F16 && umma_applies(x->bp->props, nz);
     const bool quads = x->storage == UFOB_F16 && nz > 1 && !umma;
     const bool pairs = x->storage == UFOB_BF16 || (x->storage == UFOB_F16 && nz == 1);
     const uint32_t pitch = umma ? fw : quads ? fw + 1 : pairs ? round_up(fw + 1, 4) : round_up(fw, 4);
@@ -999,16 +999,29 @@ extern "C" ufob_status ufob_fbp_kernel_times(ufob_fbp *x, double *filter_ms, uin
     return UFOB_OK;
 }
 
-static uint32_t group_slices(const ufob_fbp *x, uint32_t width, uint32_t height, uint32_t nslices)
+// Slices whose octets fit 2 GiB.
+static uint64_t octet_slices(uint32_t width, uint32_t height)
+{
+    return (2ull << 30) / std::max<uint64_t>((uint64_t)(width + 4) * 2 * height, 1);
+}
+
+// Whether a call's FP16 slices run on the tensor cores.  Decided once per call and not per group, so that
+// a remainder has the values it would have in another grouping.
+static bool fbp_umma(const ufob_fbp *x, uint32_t, uint32_t, uint32_t nslices)
+{
+    return x->storage == UFOB_F16 && umma_applies(x->bp->props, nslices);
+}
+
+static uint32_t group_slices(uint32_t width, uint32_t height, uint32_t nslices, bool umma)
 {
     // bound the filtered workspace to ~2 GiB, in multiples of 32 slices (whole slice tiles of
     // the backprojectors, which run 4 to 32 slices per CTA) or, for very large slices, of 8
-    uint64_t per_slice = (uint64_t)(width + 4) * 4 * height;
+    const uint64_t per_slice = (uint64_t)(width + 4) * 4 * height;
     uint64_t g = (2ull << 30) / std::max<uint64_t>(per_slice, 1);
     g = g >= 32 ? g / 32 * 32 : std::max<uint64_t>(8, g / 8 * 8);
-    if (x->storage == UFOB_F16 && umma_applies(x->bp->props, nslices)) {
+    if (umma) {
         // slice octets take 2 bytes a value, and the tensor-core kernel up to 128 slices per CTA
-        const uint64_t g2 = (2ull << 30) / std::max<uint64_t>((uint64_t)(width + 4) * 2 * height, 1);
+        const uint64_t g2 = octet_slices(width, height);
         if (g2 >= 128) g = g2 / 128 * 128;
     }
     return (uint32_t)std::min<uint64_t>(g, nslices);
@@ -1022,10 +1035,11 @@ extern "C" ufob_status ufob_fbp_run(ufob_fbp *x, const float *d_sino, uint32_t w
     uint32_t ow, oh;
     UFOB_TRY(ufob_fbp_get_requisition(x, width, height, &ow, &oh));
     cudaStream_t s = (cudaStream_t)stream;
-    const uint32_t G = group_slices(x, width, height, nslices);
+    const bool umma = fbp_umma(x, width, height, nslices);
+    const uint32_t G = group_slices(width, height, nslices, umma);
     for (uint32_t z = 0; z < nslices; z += G) {
         const uint32_t nz = std::min(G, nslices - z);
-        UFOB_TRY(fbp_group(x, plain_rows(d_sino + (size_t)z * width * height, width), width, height, nz,
+        UFOB_TRY(fbp_group(x, plain_rows(d_sino + (size_t)z * width * height, width), width, height, nz, umma,
                            d_out + (size_t)z * ow * oh, s));
     }
     return UFOB_OK;
@@ -1044,13 +1058,14 @@ extern "C" ufob_status ufob_fbp_run_projections(ufob_fbp *x, const ufob_preproce
     cudaStream_t s = (cudaStream_t)stream;
     // every slice group reads the same projections: a cone weight restarts at its count each time
     const uint32_t count0 = pre && pre->cone ? ufob_cone_weight_get_count(pre->cone) : 0;
-    const uint32_t G = group_slices(x, width, n_projections, n_rows);
+    const bool umma = fbp_umma(x, width, n_projections, n_rows);
+    const uint32_t G = group_slices(width, n_projections, n_rows, umma);
     for (uint32_t z = 0; z < n_rows; z += G) {
         const uint32_t nz = std::min(G, n_rows - z);
         if (pre && pre->cone) UFOB_TRY(ufob_cone_weight_set_count(pre->cone, count0));
         RowSource src;
         UFOB_TRY(projection_source(pre, d_proj, width, height, n_projections, width, true, first_row + z, nz, src, s));
-        UFOB_TRY(fbp_group(x, src, width, n_projections, nz, d_out + (size_t)z * ow * oh, s));
+        UFOB_TRY(fbp_group(x, src, width, n_projections, nz, umma, d_out + (size_t)z * ow * oh, s));
     }
     if (pre && pre->cone) UFOB_TRY(ufob_cone_weight_set_count(pre->cone, count0 + n_projections));
     return UFOB_OK;
@@ -1076,19 +1091,31 @@ extern "C" ufob_status ufob_fbp_run_host(ufob_fbp *x, const float *h_sino, uint3
             UFOB_CUDA_TRY(cudaEventCreateWithFlags(&x->ev_out[i], cudaEventDisableTiming));
         }
     }
-    const size_t in_bytes = (size_t)chunk * width * height * 4, out_bytes = (size_t)chunk * ow * oh * 4;
-    for (int i = 0; i < 2; i++) {
-        UFOB_TRY(x->hin[i].ensure(in_bytes));
-        UFOB_TRY(x->hout[i].ensure(out_bytes));
+    const bool umma = fbp_umma(x, width, height, chunk);
+    auto staging = [&](uint32_t slices) -> ufob_status {
+        for (int i = 0; i < (umma && nslices <= slices ? 1 : 2); i++) {  // (row chunks below have edges)
+            UFOB_TRY(x->hin[i].ensure((size_t)slices * width * height * 4));
+            UFOB_TRY(x->hout[i].ensure((size_t)slices * ow * oh * 4));
+        }
+        return UFOB_OK;
+    };
+    if (umma && nslices % chunk && nslices % chunk < kUmmaMinSlices) {
+        // a small last chunk would take as long as a whole one: share it among the others (up to 16 slices
+        // more in a single chunk, which then needs no second pair of buffers) or, without the
+        // memory for that, make one chunk more of equal ones.  Even numbers: the filter transforms slices
+        // in pairs, which keep their partners.
+        const uint32_t n = nslices / chunk;
+        const uint32_t larger = round_up((nslices + n - 1) / n, 2);
+        chunk = staging(larger) == UFOB_OK ? larger : round_up((nslices + n) / (n + 1), 2);
     }
+    UFOB_TRY(staging(chunk));
     // Pipeline: H2D(c) on the upload stream -> filter+BP(c) on the compute stream -> D2H(c) on the download
     // stream, double-buffered so chunk c+1's upload and chunk c-1's download overlap chunk c's compute.
     // Chunk sizes: a short first chunk (compute starts after a small upload) and a short last one
     // (little download left after the last compute), `chunk` slices in between.  On the tensor cores
-    // 16 slices take as long as 32 (and 64 hardly longer), so there all chunks are whole, and a chunk's
+    // 16 slices take as long as 32 (and 64 hardly longer), so there chunks have no edges, and a chunk's
     // image is downloaded in four bands of rows while the next band is computed: 32 slices of
     // 2048^2 x 1500 angles 40.0 -> 25.6 ms.
-    const bool umma = x->storage == UFOB_F16 && umma_applies(x->bp->props, chunk);
     const uint32_t edge = chunk >= 32 && !umma ? 16 : 0;
     // at least two waves of CTAs (four per SM) in every band
     const uint32_t bands = std::max(1u, std::min(4u, (ow / 11) * (oh / kUmmaTileRows) / (8 * (uint32_t)num_sms())));
@@ -1110,7 +1137,7 @@ extern "C" ufob_status ufob_fbp_run_host(ufob_fbp *x, const float *h_sino, uint3
         UFOB_CUDA_TRY(cudaStreamWaitEvent(x->s_comp, x->ev_in[b], 0));
         if (c >= 2) UFOB_CUDA_TRY(cudaStreamWaitEvent(x->s_comp, x->ev_out[b], 0));  // hout[b] downloaded
         const size_t plane = (size_t)ow * oh * 4;
-        UFOB_TRY(fbp_group(x, plain_rows(x->hin[b].as<float>(), width), width, height, nz, x->hout[b].as<float>(),
+        UFOB_TRY(fbp_group(x, plain_rows(x->hin[b].as<float>(), width), width, height, nz, umma, x->hout[b].as<float>(),
                            x->s_comp, bands, [&](uint32_t y, uint32_t rows) -> ufob_status {
                                // a wait takes the event as recorded last, so one event serves all bands
                                UFOB_CUDA_TRY(cudaEventRecord(x->ev_band, x->s_comp));
