@@ -224,3 +224,14 @@ def test_remainder_of_groups(cuda):
     whole, tail = f.process(sino), f.process(sino[200:].contiguous())
     ufob.device_status()
     assert torch.equal(whole[200:], tail)
+
+
+# slices so large that fewer than 17 of them would fit a group at four bytes a value
+def test_large_slices(cuda):
+    nz, P, W = 20, 4500, 5000
+    raw = torch.randn(nz, P, W).pin_memory()
+    f = ufob.FBP(filter_props={"size_x": 8192, "crop_width": W}, bp_props=ROI, storage=ufob.F16)
+    host = f.process_host(raw, out=torch.empty(nz, 48, 64).pin_memory())
+    assert torch.equal(f.process(raw.cuda()).cpu(), host)
+    ufob.device_status()
+    assert oracle.rel_l2(host[7:8].numpy(), _ref(raw[7:8].numpy(), 8192, **ROI)) < TOL

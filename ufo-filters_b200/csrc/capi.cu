@@ -1007,9 +1007,9 @@ static uint64_t octet_slices(uint32_t width, uint32_t height)
 
 // Whether a call's FP16 slices run on the tensor cores.  Decided once per call and not per group, so that
 // a remainder has the values it would have in another grouping.
-static bool fbp_umma(const ufob_fbp *x, uint32_t, uint32_t, uint32_t nslices)
+static bool fbp_umma(const ufob_fbp *x, uint32_t width, uint32_t height, uint32_t nslices)
 {
-    return x->storage == UFOB_F16 && umma_applies(x->bp->props, nslices);
+    return x->storage == UFOB_F16 && umma_applies(x->bp->props, nslices) && octet_slices(width, height) >= 16;
 }
 
 static uint32_t group_slices(uint32_t width, uint32_t height, uint32_t nslices, bool umma)
@@ -1020,9 +1020,10 @@ static uint32_t group_slices(uint32_t width, uint32_t height, uint32_t nslices, 
     uint64_t g = (2ull << 30) / std::max<uint64_t>(per_slice, 1);
     g = g >= 32 ? g / 32 * 32 : std::max<uint64_t>(8, g / 8 * 8);
     if (umma) {
-        // slice octets take 2 bytes a value, and the tensor-core kernel up to 128 slices per CTA
+        // slice octets take 2 bytes a value, and the tensor-core kernel up to 128 slices per CTA in shares
+        // of about 32
         const uint64_t g2 = octet_slices(width, height);
-        if (g2 >= 128) g = g2 / 128 * 128;
+        g = g2 >= 128 ? g2 / 128 * 128 : g2 >= 32 ? g2 / 32 * 32 : g2 / 8 * 8;
     }
     return (uint32_t)std::min<uint64_t>(g, nslices);
 }
