@@ -23,8 +23,7 @@ def _both(sino, **props):
     return a.cpu().numpy(), b.cpu().numpy()
 
 
-# (slices, angles, width, properties); the launches are large enough for the cell kernel (two CTAs
-# per SM: ceil(w / 32) * ceil(h / 64) * ceil(nz / 8) >= 296)
+# (slices, angles, width, properties): both sides of the rule that picks the kernel
 CASES = [
     (64, 40, 250, {}),
     (5, 33, 1100, {}),
@@ -109,3 +108,25 @@ def test_large_sinograms_take_no_cells(cuda):
     assert before - torch.cuda.mem_get_info()[0] < 64 << 20
     want = ufob.BackprojectTask(tile=2, **roi).process(sino)
     assert torch.equal(out, want)
+
+
+# ---- launches that have to be the cell kernel: a packing and a backprojection per 32 slices
+
+def _launches(f):
+    n = ufob.launch_count()
+    out = f()
+    return out, ufob.launch_count() - n
+
+
+# launches whose last waves are nearly empty stay with the row kernel, the others take the cells
+@pytest.mark.parametrize("nz,W,cells", [(64, 288, False), (64, 320, False), (40, 416, False), (24, 480, True),
+                                        (32, 512, True), (12, 1001, True)])
+def test_filled_waves(cuda, nz, W, cells):
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("sizes chosen for 148 SMs")
+    t = torch.randn(nz, 3, W, device="cuda")
+    task = ufob.BackprojectTask()
+    task.process(t)
+    got, n = _launches(lambda: task.process(t))
+    assert n == (2 * ((nz + 31) // 32) if cells else 1)
+    assert torch.equal(got, ufob.BackprojectTask(tile=2).process(t))

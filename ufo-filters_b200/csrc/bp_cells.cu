@@ -298,8 +298,22 @@ bool bp_cells_applies(const BPGeometry &g)
 {
     // two CTAs on every SM; below that the row kernel's smaller tiles spread better.  One to four
     // slices would leave half of the CTA's slices empty.
-    return g.nz > 4 && (uint64_t)((g.roi_w + TX - 1) / TX) * ((g.roi_h + TY - 1) / TY) * ((g.nz + ZT - 1) / ZT) >=
-                           2 * (uint64_t)num_sms();
+    const uint64_t sms = (uint64_t)num_sms(), tx = (g.roi_w + TX - 1) / TX;
+    const uint64_t tiles = tx * ((g.roi_h + TY - 1) / TY);
+    if (g.nz <= 4 || tiles * ((g.nz + ZT - 1) / ZT) < 2 * sms) return false;
+    // Every launch of up to kCellsGroup slices ends in a partly filled wave of two CTAs per SM, which takes
+    // 0.55 of a full one with a CTA per SM; the row kernel's 32 x 32 x 4 tiles (padded to whole ones, too)
+    // take 1.45 times as long per tile volume and even out.  us of rows / cells (waves, volume): 64 x 201
+    // x 288^2 326 / 409 (2, 1.10), 64 x 224 x 320^2 431 / 450 (2, 1.35), 40 x 291 x 416^2 605 / 631 (2.1, 1.43),
+    // 24 x 336 x 480^2 582 / 514 (1.55, 1.14), 12 x 700 x 1001^2 2462 / 2313 (3.55, 2.60).
+    auto waves = [&](uint32_t nz) {
+        const uint64_t ctas = tiles * ((nz + ZT - 1) / ZT), rest = ctas % (2 * sms);
+        return (double)(ctas / (2 * sms)) + (rest == 0 ? 0.0 : rest <= sms ? 0.55 : 1.0);
+    };
+    const double cells = g.nz / kCellsGroup * waves(kCellsGroup) + waves(g.nz % kCellsGroup);
+    const double volume = (double)(tx * ((g.roi_h + 31) / 32) * ((g.nz + 3) / 4)) * (32 * 32 * 4) /
+                          (2.0 * (double)sms * TX * TY * ZT);
+    return cells <= 1.45 * volume;
 }
 
 ufob_status pack_cells_launch(const float *d_in, uint32_t pitch, uint64_t slice_pitch, uint32_t W, uint32_t P,

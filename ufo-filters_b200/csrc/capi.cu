@@ -586,10 +586,10 @@ static bool cells_apply(const ufob_bp_props &p, const BPGeometry &g)
 static uint32_t cells_group(ufob_backproject *bp, uint32_t width, uint32_t height, uint32_t nslices)
 {
     const size_t quad = (size_t)16 * width * height, tile = 2 * quad;
-    const uint32_t most = (uint32_t)std::min<size_t>(32, (2ull << 30) / std::max<size_t>(tile, 1) * 8);
+    const uint32_t most = (uint32_t)std::min<size_t>(kCellsGroup, (2ull << 30) / std::max<size_t>(tile, 1) * 8);
     if (!most) return 0;
     if (bp->cells.grow((std::min(most, nslices) + 3) / 4 * quad)) return most;
-    return (uint32_t)std::min<size_t>(32, bp->cells.bytes / tile * 8);
+    return (uint32_t)std::min<size_t>(kCellsGroup, bp->cells.bytes / tile * 8);
 }
 
 // A single sinogram is split into 2, 4 or 8 equal angle groups (at least 32 angles each) whose

@@ -271,6 +271,7 @@ ufob_status make_quad_map(CUtensorMap *map, const void *base, uint32_t cells, ui
                           uint32_t pitch, uint64_t group_pitch, uint32_t box_cells, uint32_t box_groups);
 // FP32 stacks from slice cells [ceil(nz/4)][P][W] of four floats: the row kernel's image, bit for
 // bit.  pack_cells_launch makes the cells from rows.
+constexpr uint32_t kCellsGroup = 32;  // slices packed and backprojected at a time
 bool bp_cells_applies(const BPGeometry &g);
 ufob_status bp_cells_launch(const BPGeometry &g, const void *d_cells, float *d_out, cudaStream_t stream);
 ufob_status pack_cells_launch(const float *d_in, uint32_t pitch, uint64_t slice_pitch, uint32_t W, uint32_t P,
