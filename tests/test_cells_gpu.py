@@ -118,6 +118,63 @@ def _launches(f):
     return out, ufob.launch_count() - n
 
 
+def _cells(task, run):
+    run(task)  # builds the angle table
+    out, n = _launches(lambda: run(task))
+    assert n == 2 * ((out.shape[0] + 31) // 32), "not the cell kernel"
+    return out
+
+
+# odd widths and heights, odd regions inside and across the detector's edge, two to four groups with a
+# remainder of few slices, angle counts around stages and sum blocks, steep and exact angles
+CELL_CASES = [
+    (96, 40, 250, {}),
+    (5, 33, 1100, {}),
+    (37, 7, 353, dict(axis_pos=150.25)),
+    (32, 8, 385, dict(angle_offset=math.pi / 2)),
+    (61, 17, 417, dict(angle_step=math.pi / 2)),
+    (64, 24, 416, dict(axis_pos=207.5, angle_step=math.pi / 4, angle_offset=5.5)),
+    (101, 31, 400, dict(roi_x=3, roi_y=17, roi_width=383, roi_height=371)),
+    (32, 64, 320, dict(roi_x=250, roi_y=100, roi_width=320, roi_height=500)),
+]
+
+
+@pytest.mark.parametrize("nz,P,W,props", CELL_CASES)
+def test_cells_give_the_rows_bits(cuda, nz, P, W, props):
+    t = torch.randn(nz, P, W, device="cuda")
+    got = _cells(ufob.BackprojectTask(**props), lambda task: task.process(t))
+    assert torch.equal(got, ufob.BackprojectTask(tile=2, **props).process(t))
+    ufob.device_status()
+    z = nz - 1
+    ref = oracle.backproject(t[z].cpu().numpy(), **props)
+    # rows of noise: 32-bit detector coordinates (2^-14 of a bin at 1100) times the step to the next bin
+    assert oracle.rel_l2(got[z].cpu().numpy(), ref) < 1e-4
+
+
+def test_cells_nonfinite(cuda):
+    t = torch.randn(61, 30, 417, device="cuda")
+    t[3, 4, 100], t[60, 29, 0], t[35, 7, 416] = math.inf, math.nan, -math.inf
+    got = _cells(ufob.BackprojectTask(), lambda task: task.process(t)).cpu().numpy()
+    np.testing.assert_array_equal(got, ufob.BackprojectTask(tile=2).process(t).cpu().numpy())
+
+
+def test_cells_from_unaligned_rows(cuda):
+    """An odd pitch and base: the packing reads them in place, the row kernel restages."""
+    nz, P, W = 56, 20, 321
+    buf = torch.randn(nz, P, W + 2, device="cuda")
+    out = [torch.empty(nz, W, W, device="cuda") for _ in range(2)]
+
+    def run(task, o):
+        ufob.check(ufob.lib().ufob_backproject_run(task._h, buf.data_ptr() + 4, ufob.F32, ufob.ROWS, W, P, nz, W + 2,
+                                                   (W + 2) * P, o.data_ptr(), torch.cuda.current_stream().cuda_stream))
+        return o
+
+    _cells(ufob.BackprojectTask(), lambda task: run(task, out[0]))
+    run(ufob.BackprojectTask(tile=2), out[1])
+    torch.cuda.synchronize()
+    assert torch.equal(out[0], out[1])
+
+
 # launches whose last waves are nearly empty stay with the row kernel, the others take the cells
 @pytest.mark.parametrize("nz,W,cells", [(64, 288, False), (64, 320, False), (40, 416, False), (24, 480, True),
                                         (32, 512, True), (12, 1001, True)])
