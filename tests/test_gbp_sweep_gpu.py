@@ -92,3 +92,21 @@ def test_column_walks(cuda, props):
     got = _run(proj, props)
     assert oracle.rel_l2(got, ref) < 2e-5
     assert oracle.rel_l2(got, _run(proj, props, staging="texture")) < 2e-5
+
+
+# steps too coarse to stage: the texture gathers do it, and no copy of the projections is made for it
+def test_unstaged_sweep_takes_no_memory(cuda):
+    proj = torch.randn(64, 512, 1024, device="cuda")
+    t = ufob.GeneralBackprojectTask(num_projections=64)
+    for k, v in {**BASE, "center-position-x": 512.0, "center-position-z": 256.0, "parameter": "center-position-x",
+                 "z": 3.0, "region": (200.0, 800.0, 30.0)}.items():
+        t.set_property(k, v)
+    out = torch.empty(20, 37, 41, device="cuda")
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    t.process(proj, out=out)
+    torch.cuda.synchronize()
+    assert before - torch.cuda.mem_get_info()[0] < proj.numel()  # a quarter of the copy
+    t.set_property("staging", "texture")
+    assert torch.equal(out, t.process(proj))
+    ufob.device_status()

@@ -1462,6 +1462,8 @@ static ufob_status gbp_staged(ufob_gbp *g, const float *d_proj, uint32_t W, uint
     c.bh = g->col_plan.bh;
     c.walk = g->col_plan.walk;
     if (!gbp_col_fits(c)) return UFOB_OK;
+    // only a sweep that will be staged takes the memory for its transposed projections; without it, gathers
+    if (turned && !g->d_proj_h.grow((size_t)n * W * pitch * sizeof(float))) return UFOB_OK;
     UFOB_TRY(g->d_geom.ensure(table.size() * sizeof(double) + nz * sizeof(double)));
     UFOB_TRY(g->d_zvals.ensure(nz * sizeof(double) * 2));
     UFOB_TRY(g->d_tab_f.ensure((size_t)n * kTab * sizeof(float)));
@@ -1570,14 +1572,11 @@ static ufob_status gbp_compute(ufob_gbp *g, const float *d_proj, uint32_t W, uin
     const bool paramz = pcol == -1;
     // sweeps of a parallel-beam centre run as columns of the staged kernel (which they share with
     // parameter z), from 9 slices: a column has 16, and half-empty ones still match the gathers
-    // (360 x 512^2 -> 40 x 512^2: 6.74 -> 4.46 ms); the transposed projections of the horizontal one need their memory
+    // (360 x 512^2 -> 40 x 512^2: 6.74 -> 4.46 ms)
     const bool stageable = (g->compute_type == 0 || g->compute_type == 2) && !g->interpolation && g->staging &&
                            g->result_type == RT_FLOAT && g->store_type == ST_FLOAT && g->addressing_mode == AD_CLAMP;
-    const uint32_t tpitch = round_up(H, 4);
     int sweep = SWEEP_NONE;
-    if (stageable && parallel && nz > 8 && n <= 65535 && pcol == GC_CENTER_X &&
-        g->d_proj_h.ensure((size_t)n * W * tpitch * sizeof(float)) == UFOB_OK)
-        sweep = SWEEP_CENTER_X;
+    if (stageable && parallel && nz > 8 && n <= 65535 && pcol == GC_CENTER_X) sweep = SWEEP_CENTER_X;
     if (stageable && parallel && nz > 8 && pcol == GC_CENTER_Z && W % 4 == 0 && !((uintptr_t)d_proj & 15))
         sweep = SWEEP_CENTER_Z;
     if (sweep) {
