@@ -586,16 +586,6 @@ __global__ void __launch_bounds__(256, 2) k_gbp_col(const __grid_constant__ CUte
     for (int j = 0; j < ZP; j++)
         zz[j] = f2pack((float)c.zvals[min(z0 + Z0 * j, (int)c.nz - 1)],
                        (float)c.zvals[min(z0 + Z0 * j + Z1, (int)c.nz - 1)]);
-    float zstep = 0.f;  // largest step of a walk, with the sign of all of them (z values are equally spaced)
-    if constexpr (WALK) {
-        float last = (float)c.zvals[min(z0, (int)c.nz - 1)];
-#pragma unroll
-        for (int k = 1; k < ZT; k++) {
-            const float z = (float)c.zvals[min(z0 + k, (int)c.nz - 1)];
-            if (fabsf(z - last) > fabsf(zstep)) zstep = z - last;
-            last = z;
-        }
-    }
     float zlo, zhi, zdummy;
     f2unpack(zz[0], zlo, zdummy);
     f2unpack(zz[ZP - 1], zdummy, zhi);
@@ -759,76 +749,46 @@ __global__ void __launch_bounds__(256, 2) k_gbp_col(const __grid_constant__ CUte
                             bsum[j] = CONE ? f2fma(val, WG, bsum[j]) : f2add(bsum[j], val);
                         }
                     } else {
-                    // row i's two texels of one lane's voxel, interpolated along u
-                    auto rows = [&](const float *base, uint32_t i0, uint32_t i1) {
-                        const float *p0 = base + i0 * (uint32_t)bw, *p1 = base + i1 * (uint32_t)bw;
-                        const uint64_t t0 = f2pack(p0[0], p1[0]), t1 = f2pack(p0[1], p1[1]);
-                        return f2fma(AA, f2sub(t1, t0), t0);
-                    };
-                    // fraction along v of pair j, and its rows; one unsigned clamp keeps every read
-                    // inside the window (the plan's guard texels already do for every in-range footprint)
-                    auto locate = [&](int j, uint32_t &i0, uint32_t &i1) {
-                        const uint64_t vp = f2fma(AV, zz[j], BV);
-                        const uint64_t rv = f2add_rd(vp, MM);
-                        float r0, r1;
-                        f2unpack(rv, r0, r1);
-                        i0 = min((uint32_t)(__float_as_int(r0) - vbase), c.bh - 2u);
-                        i1 = min((uint32_t)(__float_as_int(r1) - vbase), c.bh - 2u);
-                        return f2sub(vp, f2sub(rv, MM));
-                    };
-                    auto add = [&](int j, uint64_t bb, uint64_t top, uint64_t bot) {
-                        const uint64_t val = f2fma(bb, f2sub(bot, top), top);
-                        bsum[j] = f2add(bsum[j], val);
-                    };
-                    // Where v moves by less than a row from voxel to voxel (0.99: rounding), a walk in
-                    // the direction of growing v reads one new row per voxel: its upper row is the
-                    // upper or the lower one of the voxel before.
-                    auto walk = [&](auto down) {
-                        uint64_t top = 0, bot = 0;
-                        uint32_t l0 = 0, l1 = 0;
+                        // row i's two texels of one lane's voxel, interpolated along u
+                        auto rows = [&](const float *base, uint32_t i0, uint32_t i1) {
+                            const float *p0 = base + i0 * (uint32_t)bw, *p1 = base + i1 * (uint32_t)bw;
+                            const uint64_t t0 = f2pack(p0[0], p1[0]), t1 = f2pack(p0[1], p1[1]);
+                            return f2fma(AA, f2sub(t1, t0), t0);
+                        };
+                        // v moves by less than 0.99 rows from voxel to voxel (the plan saw to it, with this
+                        // table's and these z values), so a walk in the direction of growing v reads one new
+                        // row per voxel: its upper row is the upper or the lower one of the voxel before
+                        auto walk = [&](auto down) {
+                            uint64_t top = 0, bot = 0;
+                            uint32_t l0 = 0, l1 = 0;
 #pragma unroll
-                        for (int i = 0; i < ZP; i++) {
-                            const int j = decltype(down)::value ? ZP - 1 - i : i;
-                            uint32_t i0, i1;
-                            const uint64_t bb = locate(j, i0, i1);
-                            if (i == 0) {
-                                top = rows(col, i0, i1);
-                            } else {
-                                float t0, t1, b0, b1;
-                                f2unpack(top, t0, t1);
-                                f2unpack(bot, b0, b1);
-                                top = f2pack(i0 != l0 ? b0 : t0, i1 != l1 ? b1 : t1);
+                            for (int i = 0; i < ZP; i++) {
+                                const int j = decltype(down)::value ? ZP - 1 - i : i;
+                                const uint64_t vp = f2fma(AV, zz[j], BV);
+                                const uint64_t rv = f2add_rd(vp, MM);
+                                const uint64_t bb = f2sub(vp, f2sub(rv, MM));
+                                float r0, r1;
+                                f2unpack(rv, r0, r1);
+                                const uint32_t i0 = min((uint32_t)(__float_as_int(r0) - vbase), c.bh - 2u);
+                                const uint32_t i1 = min((uint32_t)(__float_as_int(r1) - vbase), c.bh - 2u);
+                                if (i == 0) {
+                                    top = rows(col, i0, i1);
+                                } else {
+                                    float t0, t1, b0, b1;
+                                    f2unpack(top, t0, t1);
+                                    f2unpack(bot, b0, b1);
+                                    top = f2pack(i0 != l0 ? b0 : t0, i1 != l1 ? b1 : t1);
+                                }
+                                bot = rows(col + bw, i0, i1);
+                                l0 = i0;
+                                l1 = i1;
+                                bsum[j] = f2add(bsum[j], f2fma(bb, f2sub(bot, top), top));
                             }
-                            bot = rows(col + bw, i0, i1);
-                            l0 = i0;
-                            l1 = i1;
-                            add(j, bb, top, bot);
-                        }
-                    };
-                    const float vstep = Av * zstep;
-                    if (__all_sync(__activemask(), vstep >= 0.f && vstep < 0.99f)) {
-                        walk(std::false_type());
-                    } else if (__all_sync(__activemask(), vstep <= 0.f && vstep > -0.99f)) {
-                        walk(std::true_type());
-                    } else {
-                        // a projection past the plan's rows per voxel
-#pragma unroll
-                        for (int j = 0; j < ZP; j++) {
-                            const uint64_t vp = f2fma(AV, zz[j], BV);
-                            const uint64_t rv = f2add_rd(vp, MM);
-                            const uint64_t bb = f2sub(vp, f2sub(rv, MM));
-                            float r0, r1;
-                            f2unpack(rv, r0, r1);
-                            const uint32_t i0 = min((uint32_t)(__float_as_int(r0) - vbase), c.bh - 2u);
-                            const uint32_t i1 = min((uint32_t)(__float_as_int(r1) - vbase), c.bh - 2u);
-                            const float *p0 = col + i0 * (uint32_t)bw, *p1 = col + i1 * (uint32_t)bw;
-                            const uint64_t t00 = f2pack(p0[0], p1[0]), t10 = f2pack(p0[1], p1[1]);
-                            const uint64_t t01 = f2pack(p0[bw], p1[bw]), t11 = f2pack(p0[bw + 1], p1[bw + 1]);
-                            const uint64_t top = f2fma(AA, f2sub(t10, t00), t00), bot = f2fma(AA, f2sub(t11, t01), t01);
-                            const uint64_t val = f2fma(bb, f2sub(bot, top), top);
-                            bsum[j] = f2add(bsum[j], val);
-                        }
-                    }
+                        };
+                        if (Av * (zhi - zlo) >= 0.f)
+                            walk(std::false_type());
+                        else
+                            walk(std::true_type());
                     }
                 } else {
                     // window not staged: the same footprints and weights from global memory
@@ -961,11 +921,12 @@ static GBPColPlan gbp_col_plan(const std::vector<double> &tabs, uint32_t n, bool
     const double bw = std::ceil((wmax + 2.0) / 4.0) * 4.0, bh = hmax + 2.0;
     if (!(bw >= 4 && bw <= 256 && bh >= 2 && bh <= 256)) return plan;
     plan.ok = true;
-    double step = 0.0;
-    for (uint32_t k = 1; k < nz; k++) step = std::max(step, std::fabs(zvals[k] - zvals[k - 1]));
+    // in FP32, as the kernel has the table and the z values (whose rounding can widen a small step)
+    float step = 0.f;
+    for (uint32_t k = 1; k < nz; k++) step = std::max(step, std::fabs((float)zvals[k] - (float)zvals[k - 1]));
     plan.walk = !cone;
     for (uint32_t p = 0; p < n; p++)
-        plan.walk = plan.walk && std::fabs(tabs[(size_t)p * kTab + 6]) * step < 0.99;
+        plan.walk = plan.walk && std::fabs((float)tabs[(size_t)p * kTab + 6] * step) < 0.99f;
     plan.bw = (uint32_t)bw;
     plan.bh = (uint32_t)bh;
     return plan;
