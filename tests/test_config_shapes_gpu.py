@@ -1,8 +1,8 @@
 """The benchmarked workloads at their own shapes.
 
 * One 32-slice group of the batched FBP (2048 detector bins x 1500 angles,
-  noisy ellipsoid phantom) in plain FP32 and in FP16 slice-quad storage with
-  blocked Kahan sums, against the FP64 oracle on a 256^2 region of four of its
+  noisy ellipsoid phantom) in plain FP32, in FP16 storage on the tensor cores and
+  in FP16 slice-quad storage with blocked Kahan sums, against the FP64 oracle on a 256^2 region of four of its
   slices and, for the plain form, against the reference's own filter and
   backproject code compiled for the CPU (src/ufo-filter-task.c,
   src/ufo-backproject-task.c, src/kernels/backproject.cl) on the same region:
@@ -54,7 +54,7 @@ def c1_group(cuda):
 
 
 # FP32 bound: 1500 uncompensated FP32 sums per pixel of a noisy phantom (the plain form, as the
-# reference sums); the FP16 forms (the default FP32 block sums, and blocked Kahan sums on request)
+# reference sums); the FP16 forms (tensor cores, and slice quads with blocked Kahan sums)
 # are bounded by the FP16 rounding of the filtered cells
 @pytest.mark.parametrize("storage,compensated,tol", [(ufob.F32, 0, 3e-5), (ufob.F16, 0, 1e-3), (ufob.F16, 1, 1e-3)])
 def test_c1_group_vs_oracle(c1_group, storage, compensated, tol):

@@ -235,3 +235,46 @@ def test_large_slices(cuda):
     assert torch.equal(f.process(raw.cuda()).cpu(), host)
     ufob.device_status()
     assert oracle.rel_l2(host[7:8].numpy(), _ref(raw[7:8].numpy(), 8192, **ROI)) < TOL
+
+
+# every FFT size of the register-radix filter (its teams meet as half warps at 256, on named barriers, or
+# one team fills a CTA at 4096, which stores octets another way) and the shared-memory filter on both sides
+SIZES = [(60, 64), (250, 256), (500, 512), (1000, 1024), (2000, 2048), (4000, 4096), (5000, 8192)]
+
+
+# One angle of 0 degrees puts pixel x of any row on bin x with weight 1, so the image is the octet's halves
+# times pi: the FP16 rounding of the rows form up to one step of a value whose FP32 round-off differs (the FFT
+# pairs other rows), for small values one step of the row's largest.
+@pytest.mark.parametrize("W,N", SIZES)
+@pytest.mark.parametrize("nz", [17, 23])
+def test_octet_cells(cuda, W, N, nz):
+    raw = _raw(nz, 1, W, N)
+    got = _fbp(raw, N, roi_x=0, roi_y=1, roi_width=W, roi_height=2) / np.float32(math.pi)
+    ref = oracle.fft_filter_ifft(raw.reshape(-1, W), size_x=N, crop_width=W)
+    f = ufob.FilterTask(size_x=N, crop_width=W)
+    for z in range(nz):
+        rows = f.process(torch.from_numpy(raw[z]).cuda(), dtype=ufob.F16).float().cpu().numpy()[0]
+        scale = float(np.abs(rows).max())
+        for y in range(2):
+            assert oracle.rel_l2(got[z, y], ref[z]) < 2e-3
+            assert np.all(np.abs(got[z, y] - rows) <= 2.0 ** -10 * np.abs(rows) + 2.0 ** -11 * scale)
+
+
+# raw projections through the preprocessing fused into the filter
+@pytest.mark.parametrize("W,N", SIZES)
+def test_octets_from_projections(cuda, W, N):
+    nz, P = 19, 6
+    rng = np.random.default_rng(W)
+    dark = rng.uniform(90, 110, (nz, W)).astype(np.float32)
+    flat = (dark + rng.uniform(800, 1200, (nz, W))).astype(np.float32)
+    data = (dark + rng.uniform(50, 1000, (P, nz, W))).astype(np.float32)
+    roi = dict(roi_x=W // 3, roi_y=W // 4, roi_width=40, roi_height=23)
+    f = ufob.FBP(filter_props={"size_x": N, "crop_width": W}, bp_props=roi, storage=ufob.F16)
+    dev = [torch.from_numpy(a).cuda() for a in (data, dark, flat)]
+    got = f.process_projections(dev[0], ffc=ufob.FlatFieldCorrectTask(absorption_correct=1), dark=dev[1],
+                                flat=dev[2]).cpu().numpy()
+    ufob.device_status()
+    sinos = oracle.transpose_projections(oracle.flat_field_correct(data, dark, flat, absorption_correct=True))
+    ref = _ref(np.ascontiguousarray(sinos, dtype=np.float32), N, **roi)
+    for z in range(nz):
+        assert oracle.rel_l2(got[z], ref[z]) < TOL, z
