@@ -56,7 +56,7 @@
 #include <algorithm>
 #include <climits>
 
-#include "tma.cuh"
+#include "tcgen05.cuh"
 #include "ufob_internal.h"
 
 namespace ufob {
@@ -89,41 +89,6 @@ struct UmmaShape {
     static constexpr uint32_t smem(uint32_t ns) { return SB * KA * window_bytes(ns) + totals_bytes(ns) + 128; }
 };
 
-__device__ __forceinline__ void tmem_alloc(uint32_t *slot, uint32_t ncols)
-{
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(ncols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols)
-{
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-
-// Shared-memory matrix descriptor (version 1), no swizzle.
-__device__ __forceinline__ uint64_t desc_plain(uint32_t saddr, uint32_t lbo, uint32_t sbo)
-{
-    return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)((lbo >> 4) & 0x3FFF) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | ((uint64_t)1 << 46);
-}
-
-// A from tensor memory, B from shared memory
-__device__ __forceinline__ void mma_f16(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t acc)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
-        "r"(a), "l"(b), "r"(idesc), "r"(acc)
-        : "memory");
-}
-
-__device__ __forceinline__ void mma_commit(uint64_t *bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-                 : "memory");
-}
-
 // Sixteen columns of a warp's lanes; the registers hold them after tmem_wait16.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16])
 {
@@ -149,28 +114,6 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr),
                  "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                  : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-// Bounded wait that also gives up once another role raised the abort flag.
-__device__ __forceinline__ bool wait_or_abort(uint64_t *bar, uint32_t parity, volatile int *abort_flag)
-{
-    uint64_t t0 = 0;
-    for (uint32_t i = 1;; i++) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((i & 255u) == 0) {
-            if (*abort_flag) return false;
-            const uint64_t t = global_timer_ns();
-            if (!t0) {
-                t0 = t;
-            } else if (t - t0 > kWaitLimitNs) {
-                *abort_flag = 1;
-                return false;
-            }
-        }
-    }
 }
 
 struct UmmaArgs {
@@ -360,7 +303,8 @@ __global__ void __launch_bounds__(1024) k_octs_finite(uint4 *__restrict__ cells,
                 uint2 f = make_uint2(0, 0);
                 for (int k = 0; k < 8; k++) {
                     const uint32_t n = (nan >> k) & 1u, a = (pos >> k) & 1u, b = (neg >> k) & 1u;
-                    (k < 4 ? f.x : f.y) |= (n || (a && b) ? CLASS_NAN : a ? CLASS_POS : b ? CLASS_NEG : 0) << (8 * (k & 3));
+                    const uint32_t cls = n || (a && b) ? CLASS_NAN : a ? CLASS_POS : b ? CLASS_NEG : 0;
+                    (k < 4 ? f.x : f.y) |= cls << (8 * (k & 3));
                 }
                 flags[r] = f;
                 ranges[r] = make_int2(lo, hi);
@@ -460,9 +404,9 @@ __global__ void __launch_bounds__(kThreads, Sh::CTAS)
             if (row < MX * MY)
 #pragma unroll
                 for (int i = 0; i < 4; i++)
-                    t[i * (MX * MY)] = make_float4(v[i].x + __uint_as_float(r[4 * i]), v[i].y + __uint_as_float(r[4 * i + 1]),
-                                                   v[i].z + __uint_as_float(r[4 * i + 2]),
-                                                   v[i].w + __uint_as_float(r[4 * i + 3]));
+                    t[i * (MX * MY)] =
+                        make_float4(v[i].x + __uint_as_float(r[4 * i]), v[i].y + __uint_as_float(r[4 * i + 1]),
+                                    v[i].z + __uint_as_float(r[4 * i + 2]), v[i].w + __uint_as_float(r[4 * i + 3]));
             __syncwarp();
         }
         tc_fence_before();
@@ -536,7 +480,7 @@ __global__ void __launch_bounds__(kThreads, Sh::CTAS)
         const int m = warp - kBuildWarps - 1;  // accumulator of an MMA warp
         // D = F32, A = B = F16, B N-major
         const uint32_t idesc = (1u << 4) | (1u << 16) | ((args.ns >> 3) << 17) | ((128u >> 4) << 24);
-        const uint64_t desc0 = desc_plain(base, 128, KW * 16);
+        const uint64_t desc0 = plain_desc(base, 128, KW * 16);
         const uint32_t dcol = tmem + (uint32_t)m * args.ns;
         const uint32_t acol = tmem + MT * args.ns + (uint32_t)m * (KT / 2);
         uint32_t acc = 0;
@@ -585,13 +529,13 @@ __global__ void __launch_bounds__(kThreads, Sh::CTAS)
                         if (nval == KA) {
 #pragma unroll
                             for (int a = 0; a < KA; a++)
-                                mma_f16(dcol, acol + (sa * KA + a) * (MT * (KT / 2)),
+                                mma_ts(dcol, acol + (sa * KA + a) * (MT * (KT / 2)),
                                         desc0 + (uint64_t)((sb * KA + a) * (bbytes >> 4) + off[a]), idesc,
                                         a > 0 ? 1u : acc);
                         } else {
 #pragma unroll 1
                             for (uint32_t a = 0; a < nval; a++)
-                                mma_f16(dcol, acol + (sa * KA + a) * (MT * (KT / 2)),
+                                mma_ts(dcol, acol + (sa * KA + a) * (MT * (KT / 2)),
                                         desc0 + (uint64_t)((sb * KA + a) * (bbytes >> 4) + s_off[m][j + a]), idesc,
                                         a > 0 ? 1u : acc);
                         }

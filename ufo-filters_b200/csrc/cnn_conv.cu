@@ -28,87 +28,16 @@
 // version 1, no swizzle; c=F32, a=b=BF16, N>>3, M>>4, K- or MN-major bits).
 #include <cuda_bf16.h>
 
+#include "tcgen05.cuh"
 #include "ufob_internal.h"
 
 namespace ufob {
-
-// ------------------------------------------------------------------ tcgen05 / mbarrier helpers
-
-__device__ __forceinline__ uint32_t cvta_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void cnn_mbar_init(uint64_t *bar)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(cvta_smem(bar)) : "memory");
-}
-
-// Bounded wait (2 s); the timer is read only every 256 polls so that its
-// latency does not delay noticing the phase flip.
-__device__ __forceinline__ bool cnn_mbar_wait(uint64_t *bar, uint32_t parity)
-{
-    uint64_t t0 = 0;
-    for (uint32_t i = 1;; i++) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(cvta_smem(bar)), "r"(parity)
-            : "memory");
-        if (ok) return true;
-        if ((i & 255u) == 0) {
-            uint64_t t;
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-            if (!t0)
-                t0 = t;
-            else if (t - t0 > 2000000000ull)
-                return false;
-        }
-    }
-}
-
-__device__ __forceinline__ void tmem_alloc(uint32_t *slot, uint32_t ncols)
-{
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(cvta_smem(slot)), "r"(ncols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols)
-{
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-
-// Shared-memory matrix descriptor, no swizzle (layout type 0), version 1.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo)
-{
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr >> 4) & 0x3FFF);
-    d |= (uint64_t)((lbo >> 4) & 0x3FFF) << 16;
-    d |= (uint64_t)((sbo >> 4) & 0x3FFF) << 32;
-    d |= (uint64_t)1 << 46;  // version
-    return d;
-}
 
 // Instruction descriptor of kind::f16: D = F32, A = B = BF16, M x N, majorness bits.
 __host__ __device__ constexpr uint32_t idesc_bf16(uint32_t M, uint32_t N, uint32_t a_mn_major, uint32_t b_mn_major)
 {
     return (1u << 4) | (1u << 7) | (1u << 10) | (a_mn_major << 15) | (b_mn_major << 16) | ((N >> 3) << 17) |
            ((M >> 4) << 24);
-}
-
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
-__device__ __forceinline__ void umma_commit(uint64_t *bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cvta_smem(bar))
-                 : "memory");
 }
 
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8])
@@ -121,10 +50,6 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8])
 #pragma unroll
     for (int i = 0; i < 8; i++) v[i] = __uint_as_float(r[i]);
 }
-
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
 static constexpr int kErrConvTimeout = 0x2001;
 
@@ -174,9 +99,9 @@ __global__ void __launch_bounds__(128) k_conv3x3(const ConvArgs a)
 
     if (warp == 0) tmem_alloc(&tslot, ncols);
     if (tid == 0) {
-        cnn_mbar_init(&bars[0]);
-        cnn_mbar_init(&bars[1]);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        mbar_init(&bars[0], 1);
+        mbar_init(&bars[1], 1);
+        fence_barrier_init();
     }
     tc_fence_before();
     __syncthreads();
@@ -232,7 +157,8 @@ __global__ void __launch_bounds__(128) k_conv3x3(const ConvArgs a)
     load(0);
     for (int i = 0; i < nk && ok; i++) {
         const int st = i & 1;
-        if (i >= 2) ok = cnn_mbar_wait(&bars[st], (uint32_t)(((i - 2) >> 1) & 1));  // MMAs of chunk i-2 done
+        // MMAs of chunk i-2 done
+        if (i >= 2) ok = mbar_wait_bounded(&bars[st], (uint32_t)(((i - 2) >> 1) & 1), kWaitLimitNs);
 #pragma unroll
         for (int k = 0; k < kchunks; k++)
             *reinterpret_cast<uint4 *>(sA[st] + k * lboA + (tid >> 3) * 128 + (tid & 7) * 16) = ra[k];
@@ -248,16 +174,16 @@ __global__ void __launch_bounds__(128) k_conv3x3(const ConvArgs a)
         __syncthreads();
         if (tid == 0) {
             tc_fence_after();
-            const uint32_t a0 = cvta_smem(sA[st]), b0 = cvta_smem(sB[st]);
+            const uint32_t a0 = smem_u32(sA[st]), b0 = smem_u32(sB[st]);
             const int steps = min(kConvBK, K - i * kConvBK) / 16;
             for (int s = 0; s < steps; s++)
-                umma_bf16(tmem, smem_desc(a0 + s * 2 * lboA, lboA, 128), smem_desc(b0 + s * 2 * lboB, lboB, 128),
+                mma_ss(tmem, plain_desc(a0 + s * 2 * lboA, lboA, 128), plain_desc(b0 + s * 2 * lboB, lboB, 128),
                           idesc, (i > 0 || s > 0) ? 1u : 0u);
-            umma_commit(&bars[st]);
+            mma_commit(&bars[st]);
         }
     }
     // the last chunk's commit covers every earlier MMA of this thread
-    if (ok) ok = cnn_mbar_wait(&bars[(nk - 1) & 1], (uint32_t)(((nk - 1) >> 1) & 1));
+    if (ok) ok = mbar_wait_bounded(&bars[(nk - 1) & 1], (uint32_t)(((nk - 1) >> 1) & 1), kWaitLimitNs);
     tc_fence_after();
     if (!ok) {
         if (tid == 0) atomicExch(a.err, kErrConvTimeout);
@@ -326,9 +252,9 @@ __device__ __forceinline__ void red_add4(float *dst, float x, float y, float z, 
 // behind (inside the CTA's shared memory) and are not used.
 //
 // As the forward kernel, bound by the latency of a chunk: next chunk's loads in registers, several
-// taps of a small layer along N (nine CTAs per pixel range before), shared memory by the channels, 32-bit pixel arithmetic in the loads (64-bit divisions per 16 bytes had been
-// most of a chunk's instructions), at least 512 pixels per CTA and 16-byte reductions into the
-// gradient.  Training step of 16 x 512^2 (us, before -> after): 165 -> 38..89 for the layers up to 128
+// taps of a small layer along N (nine CTAs per pixel range before), shared memory by the channels, 32-bit
+// pixel arithmetic in the loads (64-bit divisions per 16 bytes had been most of a chunk's instructions),
+// at least 512 pixels per CTA and 16-byte reductions into the gradient.  Training step of 16 x 512^2 (us, before -> after): 165 -> 38..89 for the layers up to 128
 // channels, 107..165 -> 36 for 128<->256.
 constexpr int kWgradCols = 128;  // channels of either operand per CTA at most
 
@@ -354,9 +280,9 @@ __global__ void __launch_bounds__(128) k_conv3x3_wgrad(const WgradArgs a)
 
     if (warp == 0) tmem_alloc(&tslot, ncols);
     if (tid == 0) {
-        cnn_mbar_init(&bars[0]);
-        cnn_mbar_init(&bars[1]);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        mbar_init(&bars[0], 1);
+        mbar_init(&bars[1], 1);
+        fence_barrier_init();
     }
     tc_fence_before();
     __syncthreads();
@@ -403,7 +329,7 @@ __global__ void __launch_bounds__(128) k_conv3x3_wgrad(const WgradArgs a)
     if (nk > 0) load(0);
     for (int i = 0; i < nk && ok; i++) {
         const int st = i & 1;
-        if (i >= 2) ok = cnn_mbar_wait(&bars[st], (uint32_t)(((i - 2) >> 1) & 1));
+        if (i >= 2) ok = mbar_wait_bounded(&bars[st], (uint32_t)(((i - 2) >> 1) & 1), kWaitLimitNs);
 #pragma unroll
         for (int q = 0; q < NR; q++) {
             const uint32_t idx = tid + 128 * q, k = idx / ca, g = idx - k * ca;
@@ -422,15 +348,15 @@ __global__ void __launch_bounds__(128) k_conv3x3_wgrad(const WgradArgs a)
         __syncthreads();
         if (tid == 0) {
             tc_fence_after();
-            const uint32_t a0 = cvta_smem(sA[st]), b0 = cvta_smem(sB[st]);
+            const uint32_t a0 = smem_u32(sA[st]), b0 = smem_u32(sB[st]);
             // MN-major: leading offset = K-group stride, stride offset = 8-row group stride
             for (int s = 0; s < BK / 16; s++)
-                umma_bf16(tmem, smem_desc(a0 + s * 2 * lboA, lboA, 128), smem_desc(b0 + s * 2 * lboB, lboB, 128),
+                mma_ss(tmem, plain_desc(a0 + s * 2 * lboA, lboA, 128), plain_desc(b0 + s * 2 * lboB, lboB, 128),
                           idesc, (i > 0 || s > 0) ? 1u : 0u);
-            umma_commit(&bars[st]);
+            mma_commit(&bars[st]);
         }
     }
-    if (nk > 0 && ok) ok = cnn_mbar_wait(&bars[(nk - 1) & 1], (uint32_t)(((nk - 1) >> 1) & 1));
+    if (nk > 0 && ok) ok = mbar_wait_bounded(&bars[(nk - 1) & 1], (uint32_t)(((nk - 1) >> 1) & 1), kWaitLimitNs);
     tc_fence_after();
     if (!ok) {
         if (tid == 0) atomicExch(a.err, kErrConvTimeout);

@@ -30,6 +30,7 @@
 
 #include <algorithm>
 
+#include "tcgen05.cuh"
 #include "ufob_internal.h"
 
 namespace ufob {
@@ -44,54 +45,6 @@ constexpr int kAStages = 2;
 constexpr int kMaxBStages = 16;
 constexpr int kErrFastTimeout = 0x2101;
 constexpr size_t kMaxSmem = 220 * 1024;
-constexpr uint64_t kLimitNs = 2000000000ull;
-
-__device__ __forceinline__ uint32_t sa(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void bar_init(uint64_t *b, uint32_t count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sa(b)), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ bool bar_try(uint64_t *b, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(sa(b)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-__device__ __forceinline__ uint64_t now_ns()
-{
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// Bounded wait that also gives up as soon as another role raised the abort flag.
-// The timer and the flag are checked only every 256 polls: a %globaltimer read
-// per poll delays noticing the phase flip by the read's latency.
-__device__ __forceinline__ bool bar_wait(uint64_t *b, uint32_t parity, volatile int *abort_flag)
-{
-    uint64_t t0 = 0;
-    for (uint32_t i = 1;; i++) {
-        if (bar_try(b, parity)) return true;
-        if ((i & 255u) == 0) {
-            if (*abort_flag) return false;
-            const uint64_t t = now_ns();
-            if (!t0) {
-                t0 = t;
-            } else if (t - t0 > kLimitNs) {
-                *abort_flag = 1;
-                return false;
-            }
-        }
-    }
-}
-
 // Programmatic dependent launch: the next kernel of the forward pass may be scheduled as soon as
 // every CTA of this one has started (launch_dependents); a kernel launched that way waits for its
 // predecessor, and hence for every earlier kernel of the stream, to complete and become visible
@@ -99,48 +52,9 @@ __device__ __forceinline__ bool bar_wait(uint64_t *b, uint32_t parity, volatile 
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-__device__ __forceinline__ void bar_arrive(uint64_t *b)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sa(b)) : "memory");
-}
-
-__device__ __forceinline__ void bar_expect(uint64_t *b, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sa(b)), "r"(bytes) : "memory");
-}
-
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *b)
-{
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     sa(dst)),
-                 "l"(src), "r"(bytes), "r"(sa(b))
-                 : "memory");
-}
-
-__device__ __forceinline__ uint64_t desc_kmajor(uint32_t saddr, uint32_t lbo, uint32_t sbo)
-{
-    return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)((lbo >> 4) & 0x3FFF) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | ((uint64_t)1 << 46);
-}
-
 __host__ __device__ constexpr uint32_t idesc_f16_bf16(uint32_t M, uint32_t N)
 {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
-}
-
-__device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
-        "l"(a), "l"(b), "r"(idesc), "r"(acc)
-        : "memory");
-}
-
-__device__ __forceinline__ void commit(uint64_t *b)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(sa(b))
-                 : "memory");
 }
 
 // tcgen05.ld of N consecutive 32-bit columns (32 lanes x 32 bit), no wait
@@ -186,9 +100,6 @@ __device__ __forceinline__ void tld<32>(uint32_t taddr, float (&v)[32])
 __device__ __forceinline__ int ilog2_dev(int v) { return 31 - __clz(v); }
 
 __device__ __forceinline__ void tld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
 __device__ __forceinline__ uint4 pack8(const float (&v)[8])
 {
@@ -252,7 +163,7 @@ __device__ __forceinline__ void issue_tap(uint32_t dcol, uint32_t Cout, uint64_t
     for (int m = 0; m < MT; m++)
 #pragma unroll
         for (int k = 0; k < KS; k++)
-            mma(dcol + (uint32_t)m * Cout, dA + (uint64_t)(m * 128) + (uint64_t)(2 * k) * a16,
+            mma_ss(dcol + (uint32_t)m * Cout, dA + (uint64_t)(m * 128) + (uint64_t)(2 * k) * a16,
                 dB + (uint64_t)(2 * k) * b16, idesc, (first && k == 0) ? 0u : 1u);
 }
 
@@ -287,29 +198,29 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv_cg(const FastConvArgs a)
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < kAStages; i++) {
-            bar_init(&a_full[i], 1);
-            bar_init(&a_empty[i], 1);
+            mbar_init(&a_full[i], 1);
+            mbar_init(&a_empty[i], 1);
         }
         for (int i = 0; i < nbs; i++) {
-            bar_init(&b_full[i], 1);
-            bar_init(&b_empty[i], 1);
+            mbar_init(&b_full[i], 1);
+            mbar_init(&b_empty[i], 1);
         }
         for (int i = 0; i < 2; i++) {
-            bar_init(&t_full[i], 1);
-            bar_init(&t_empty[i], kEpiWarps);
+            mbar_init(&t_full[i], 1);
+            mbar_init(&t_empty[i], kEpiWarps);
         }
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     for (int i = threadIdx.x; i < Cout; i += blockDim.x) s_bias[i] = a.bias[i];
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sa(&tslot)), "r"(ncols)
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tslot)), "r"(ncols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    fence_before();
+    tc_fence_before();
     __syncthreads();
-    fence_after();
+    tc_fence_after();
     const uint32_t tmem = tslot;
     volatile int *abort_p = &abort_flag;
 
@@ -328,9 +239,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv_cg(const FastConvArgs a)
                 for (int kc = 0; kc < nchunks; kc++)
                     for (int t = 0; t < 9; t++) {
                         const int sb = kc * 9 + t;
-                        bar_expect(&b_full[sb], b_stage);
+                        mbar_arrive_expect_tx(&b_full[sb], b_stage);
                         const bf16 *src = a.wt + ((size_t)t * (Cin / 8) + (size_t)kc * cgc) * Cout * 8;
-                        bulk_g2s(sB + (size_t)sb * b_stage, src, b_stage, &b_full[sb]);
+                        bulk_load_1d(sB + (size_t)sb * b_stage, src, b_stage, &b_full[sb]);
                         last_b[sb] = 0;
                     }
             }
@@ -339,23 +250,23 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv_cg(const FastConvArgs a)
                 const long long q0 = tile * (long long)(MT * 128);
                 for (int kc = 0; kc < nchunks && ok; kc++) {
                     const int s = (int)(ka % kAStages);
-                    ok = bar_wait(&a_empty[s], ((ka / kAStages) & 1u) ^ 1u, abort_p);
+                    ok = wait_or_abort(&a_empty[s], ((ka / kAStages) & 1u) ^ 1u, abort_p);
                     if (!ok) break;
-                    bar_expect(&a_full[s], a_stage);
+                    mbar_arrive_expect_tx(&a_full[s], a_stage);
                     for (int g = 0; g < cgc; g++) {
                         const bf16 *src = a.in + (size_t)(kc * cgc + g) * plane_elems +
                                           (size_t)(a.gi.guard + q0 - halo) * 8;
-                        bulk_g2s(sA + (size_t)s * a_stage + (size_t)g * a_plane, src, a_plane, &a_full[s]);
+                        bulk_load_1d(sA + (size_t)s * a_stage + (size_t)g * a_plane, src, a_plane, &a_full[s]);
                     }
                     last_a[s] = (int)ka;
                     ka++;
                     for (int t = 0; t < 9 && ok && !resident; t++) {
                         const int sb = (int)(kb % nbs);
-                        ok = bar_wait(&b_empty[sb], ((kb / nbs) & 1u) ^ 1u, abort_p);
+                        ok = wait_or_abort(&b_empty[sb], ((kb / nbs) & 1u) ^ 1u, abort_p);
                         if (!ok) break;
-                        bar_expect(&b_full[sb], b_stage);
+                        mbar_arrive_expect_tx(&b_full[sb], b_stage);
                         const bf16 *src = a.wt + ((size_t)t * (Cin / 8) + (size_t)kc * cgc) * Cout * 8;
-                        bulk_g2s(sB + (size_t)sb * b_stage, src, b_stage, &b_full[sb]);
+                        bulk_load_1d(sB + (size_t)sb * b_stage, src, b_stage, &b_full[sb]);
                         last_b[sb] = (int)kb;
                         kb++;
                     }
@@ -365,17 +276,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv_cg(const FastConvArgs a)
                 atomicExch(a.err, kErrFastTimeout);
                 // let copies already in flight land before the CTA can exit (bounded)
                 for (int s = 0; s < kAStages; s++) {
-                    const uint64_t t0 = now_ns();
+                    const uint64_t t0 = global_timer_ns();
                     if (last_a[s] >= 0)
-                        while (!bar_try(&a_full[s], ((uint32_t)last_a[s] / kAStages) & 1u) &&
-                               now_ns() - t0 < kLimitNs / 8) {
+                        while (!mbar_try_wait(&a_full[s], ((uint32_t)last_a[s] / kAStages) & 1u) &&
+                               global_timer_ns() - t0 < kWaitLimitNs / 8) {
                         }
                 }
                 for (int s = 0; s < nbs; s++) {
-                    const uint64_t t0 = now_ns();
+                    const uint64_t t0 = global_timer_ns();
                     if (last_b[s] >= 0)
-                        while (!bar_try(&b_full[s], ((uint32_t)last_b[s] / nbs) & 1u) &&
-                               now_ns() - t0 < kLimitNs / 8) {
+                        while (!mbar_try_wait(&b_full[s], ((uint32_t)last_b[s] / nbs) & 1u) &&
+                               global_timer_ns() - t0 < kWaitLimitNs / 8) {
                         }
                 }
             }
@@ -387,35 +298,35 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv_cg(const FastConvArgs a)
             bool ok = true;
             for (long long tile = blockIdx.x; tile < a.ntiles && ok; tile += gridDim.x, it++) {
                 const uint32_t ab = it & 1u;
-                ok = bar_wait(&t_empty[ab], ((it >> 1) & 1u) ^ 1u, abort_p);
+                ok = wait_or_abort(&t_empty[ab], ((it >> 1) & 1u) ^ 1u, abort_p);
                 if (!ok) break;
-                fence_after();
+                tc_fence_after();
                 const uint32_t dcol = tmem + ab * acc_cols;
                 for (int kc = 0; kc < nchunks && ok; kc++) {
                     const int s = (int)(ka % kAStages);
-                    ok = bar_wait(&a_full[s], (ka / kAStages) & 1u, abort_p);
+                    ok = wait_or_abort(&a_full[s], (ka / kAStages) & 1u, abort_p);
                     if (!ok) break;
-                    fence_after();
-                    const uint32_t abase = sa(sA + (size_t)s * a_stage);
+                    tc_fence_after();
+                    const uint32_t abase = smem_u32(sA + (size_t)s * a_stage);
                     for (int t = 0; t < 9 && ok; t++) {
                         const int sb = resident ? kc * 9 + t : (int)(kb % nbs);
                         if (!resident || it == 0) {
-                            ok = bar_wait(&b_full[sb], resident ? 0u : (kb / nbs) & 1u, abort_p);
+                            ok = wait_or_abort(&b_full[sb], resident ? 0u : (kb / nbs) & 1u, abort_p);
                             if (!ok) break;
-                            fence_after();
+                            tc_fence_after();
                         }
-                        const uint32_t bbase = sa(sB + (size_t)sb * b_stage);
+                        const uint32_t bbase = smem_u32(sB + (size_t)sb * b_stage);
                         const int off = halo + (t / 3 - 1) * Wp + (t % 3 - 1);
-                        issue_tap<MT, KS>(dcol, (uint32_t)Cout, desc_kmajor(abase + (uint32_t)off * 16, a_plane, 128),
-                                          desc_kmajor(bbase, (uint32_t)Cout * 16, 128), a_plane >> 4, (uint32_t)Cout,
+                        issue_tap<MT, KS>(dcol, (uint32_t)Cout, plain_desc(abase + (uint32_t)off * 16, a_plane, 128),
+                                          plain_desc(bbase, (uint32_t)Cout * 16, 128), a_plane >> 4, (uint32_t)Cout,
                                           idesc, kc == 0 && t == 0);
-                        if (!resident) commit(&b_empty[sb]);  // frees the weight stage once these MMAs finish
+                        if (!resident) mma_commit(&b_empty[sb]);  // frees the weight stage once these MMAs finish
                         kb++;
                     }
-                    commit(&a_empty[s]);
+                    mma_commit(&a_empty[s]);
                     ka++;
                 }
-                commit(&t_full[ab]);
+                mma_commit(&t_full[ab]);
             }
             if (!ok) atomicExch(a.err, kErrFastTimeout);
         }
@@ -430,11 +341,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv_cg(const FastConvArgs a)
         pdl_wait();  // skip tensors and the FBP image come from earlier kernels
         for (long long tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x, it++) {
             const uint32_t ab = it & 1u;
-            if (!bar_wait(&t_full[ab], (it >> 1) & 1u, abort_p)) {
+            if (!wait_or_abort(&t_full[ab], (it >> 1) & 1u, abort_p)) {
                 if (lane == 0) atomicExch(a.err, kErrFastTimeout);
                 break;
             }
-            fence_after();
+            tc_fence_after();
             const uint32_t q0 = (uint32_t)tile * (uint32_t)(MT * 128) + (uint32_t)(quarter * 32 + lane);
             const uint32_t tb = tmem + ((uint32_t)(quarter * 32) << 16) + ab * acc_cols + (uint32_t)(half * ch);
             // pixel of row q of the padded grid: (b, y, x), inside = interior pixel
@@ -583,12 +494,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv_cg(const FastConvArgs a)
                     }
                 }
             }
-            fence_before();
+            tc_fence_before();
             __syncwarp();
-            if (lane == 0) bar_arrive(&t_empty[ab]);
+            if (lane == 0) mbar_arrive(&t_empty[ab]);
         }
     }
-    fence_before();
+    tc_fence_before();
     __syncthreads();
     if (warp == 1) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
