@@ -181,39 +181,48 @@ __device__ __forceinline__ uint32_t nonfinite_slices(const UmmaArgs &a, float cx
     const uint32_t lane = threadIdx.x & 31;
     const size_t row0 = (size_t)g * a.P;
     uint32_t nan = 0, pos = 0, neg = 0;
-    for (uint32_t p0 = 0; p0 < a.P; p0 += 32) {
-        const uint32_t pl = min(p0 + lane, a.P - 1);
-        const int2 r = __ldg(a.ranges + row0 + pl);
-        const float2 sl = __ldg(&a.sincos[pl]);
-        const int w0 = min(window_start(cx, cy, sl, a.axis), window_start(cx, cy + MY, sl, a.axis));
-        uint32_t hits = __ballot_sync(0xffffffffu, p0 + lane < a.P && r.x <= w0 + KW && r.y >= w0 - 1);
-        for (; hits && __any_sync(0xffffffffu, in && (bad & ~nan)); hits &= hits - 1) {
-            const uint32_t q = __ffs(hits) - 1, p = p0 + q;
-            const float s = __shfl_sync(0xffffffffu, sl.x, q), c = __shfl_sync(0xffffffffu, sl.y, q);
-            const int first = __shfl_sync(0xffffffffu, r.x, q), last = __shfl_sync(0xffffffffu, r.y, q);
-            const float h = fmaf(by, s, fmaf(bx, c, a.axis)) - 0.5f;
-            const float e = floorf(h), f = h - e;
-            if (!in || !(e >= -1.0f && e < (float)a.W)) continue;
-            const int j = (int)e;
-            if (j + 1 < first || j > last) continue;
-            const uint2 cls = __ldg(a.flags + row0 + p);
-            const uint4 *row = a.sino + (size_t)g * a.group_pitch + (size_t)p * a.pitch;
-            const uint4 zero = make_uint4(0, 0, 0, 0);
-            const uint4 lo = j >= 0 ? __ldg(row + j) : zero, hi = j + 1 < (int)a.W ? __ldg(row + j + 1) : zero;
-            const uint32_t l[4] = {lo.x, lo.y, lo.z, lo.w}, u[4] = {hi.x, hi.y, hi.z, hi.w};
+    constexpr int N = 4;  // groups of 32 angles tested together: one latency for their tables
+    for (uint32_t p0 = 0; p0 < a.P; p0 += 32 * N) {
+        int2 r[N];
+        float2 sl[N];
 #pragma unroll
-            for (int k = 0; k < 8; k++) {
-                const uint32_t b = ((k < 4 ? cls.x : cls.y) >> (8 * (k & 3))) & 0xffu;
-                const float s0 = octet_value((l[k / 2] >> (16 * (k & 1))) & 0xffffu, b);
-                const float s1 = octet_value((u[k / 2] >> (16 * (k & 1))) & 0xffffu, b);
-                const float v = (1.0f - f) * s0 + f * s1;
-                if (v != v) nan |= 1u << k;
-                if (v == INFINITY) pos |= 1u << k;
-                if (v == -INFINITY) neg |= 1u << k;
-            }
-            nan |= pos & neg;
+        for (int k = 0; k < N; k++) {
+            const uint32_t p = p0 + 32 * k + lane;
+            r[k] = p < a.P ? __ldg(a.ranges + row0 + p) : make_int2(INT_MAX, -1);
+            sl[k] = __ldg(&a.sincos[min(p, a.P - 1)]);
         }
-        if (hits) break;
+#pragma unroll
+        for (int k = 0; k < N; k++) {
+            const int w0 = min(window_start(cx, cy, sl[k], a.axis), window_start(cx, cy + MY, sl[k], a.axis));
+            uint32_t hits = __ballot_sync(0xffffffffu, r[k].x <= w0 + KW && r[k].y >= w0 - 1);
+            for (; hits && __any_sync(0xffffffffu, in && (bad & ~nan)); hits &= hits - 1) {
+                const uint32_t q = __ffs(hits) - 1, p = p0 + 32 * k + q;
+                const float s = __shfl_sync(0xffffffffu, sl[k].x, q), c = __shfl_sync(0xffffffffu, sl[k].y, q);
+                const int first = __shfl_sync(0xffffffffu, r[k].x, q), last = __shfl_sync(0xffffffffu, r[k].y, q);
+                const float h = fmaf(by, s, fmaf(bx, c, a.axis)) - 0.5f;
+                const float e = floorf(h), f = h - e;
+                if (!in || !(e >= -1.0f && e < (float)a.W)) continue;
+                const int j = (int)e;
+                if (j + 1 < first || j > last) continue;
+                const uint2 cls = __ldg(a.flags + row0 + p);
+                const uint4 *row = a.sino + (size_t)g * a.group_pitch + (size_t)p * a.pitch;
+                const uint4 zero = make_uint4(0, 0, 0, 0);
+                const uint4 lo = j >= 0 ? __ldg(row + j) : zero, hi = j + 1 < (int)a.W ? __ldg(row + j + 1) : zero;
+                const uint32_t l[4] = {lo.x, lo.y, lo.z, lo.w}, u[4] = {hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const uint32_t b = ((i < 4 ? cls.x : cls.y) >> (8 * (i & 3))) & 0xffu;
+                    const float s0 = octet_value((l[i / 2] >> (16 * (i & 1))) & 0xffffu, b);
+                    const float s1 = octet_value((u[i / 2] >> (16 * (i & 1))) & 0xffffu, b);
+                    const float v = (1.0f - f) * s0 + f * s1;
+                    if (v != v) nan |= 1u << i;
+                    if (v == INFINITY) pos |= 1u << i;
+                    if (v == -INFINITY) neg |= 1u << i;
+                }
+                nan |= pos & neg;
+            }
+        }
+        if (!__any_sync(0xffffffffu, in && (bad & ~nan))) break;
     }
     return nan | (pos & ~nan) << 8 | (neg & ~nan) << 16;
 }

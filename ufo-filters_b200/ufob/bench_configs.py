@@ -140,7 +140,7 @@ def bench_pre(reps=3, n_proj=1500, rows=256, width=2048, seed=7):
     g = torch.Generator(device="cuda").manual_seed(seed)
     dark = 100 + torch.rand(rows, width, device="cuda", generator=g)
     flat = dark + 1000
-    proj = dark + 900 * torch.rand(n_proj, rows, width, device="cuda", generator=g)
+    proj = dark + 50 + 900 * torch.rand(n_proj, rows, width, device="cuda", generator=g)  # no zero counts
     ffc = FlatFieldCorrectTask(absorption_correct=1)
     f = FilterTask()
     tr = TransposeProjectionsTask(num_projections=n_proj)
