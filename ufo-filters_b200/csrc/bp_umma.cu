@@ -39,8 +39,8 @@
 // arrive on one barrier that frees its weights and its windows.  What bounds it is the fixed cost
 // of a stage (barriers, issue latencies), so up to 64 slices two CTAs share an SM (KA = 4); above,
 // tensor memory holds one CTA, whose stages are longer (KA = 8) and whose totals are mostly registers.
-// 2048^2 x 1500 angles, ms per pass: ns <= 32 16.2, 64 17.6, 96 23.6, 128 28.9 (12.4, 22.9, 25.6,
-// 27.9 TGUPS; slice quads 6.6).  Four CTAs per SM with KA = 2 up to 32 slices: 16.2 (2% faster without the
+// 2048^2 x 1500 angles, ms per pass: ns <= 32 16.0, 64 17.4, 96 23.4, 128 28.5 (12.6, 23.1, 25.8,
+// 28.3 TGUPS; slice quads 6.6).  Four CTAs per SM with KA = 2 up to 32 slices: 16.2 (2% faster without the
 // totals, which then are all in shared memory); two with KA = 2 for 96: 26.4.
 //
 // A non-finite value of a window would reach every pixel of its tile (0 * inf).  The filter flags
@@ -76,7 +76,7 @@ enum { CLASS_NAN = 1, CLASS_POS = 2, CLASS_NEG = 4 };  // flag bytes: what the -
 constexpr int kErrUmmaTimeout = 0x1003;
 
 // KA angles per stage, SB stages of windows, CTAs per SM, and how many 16-column chunks of a builder
-// thread's totals are in registers (the others in shared memory).
+// thread's totals are in registers (the others in shared memory; the CTA's slices fill at least RC chunks).
 template <int KA_, int SB_, int CTAS_, int RC_>
 struct UmmaShape {
     static constexpr int KA = KA_, SB = SB_, CTAS = CTAS_, RC = RC_;
@@ -592,7 +592,7 @@ __global__ void __launch_bounds__(kThreads, Sh::CTAS)
                 float v[16];
 #pragma unroll
                 for (int i = 0; i < 16; i++) v[i] = tot[16 * q + i];
-                if (q < (int)chunks) store(q, v);
+                store(q, v);
             }
 #pragma unroll 1
             for (uint32_t q = RC; q < chunks; q++) {
@@ -666,11 +666,12 @@ uint32_t bp_umma_slices(uint32_t nz)
     static const struct {
         uint32_t ns;
         float ms;
-    } kPass[] = {{32, 16.2f}, {64, 17.6f}, {96, 23.6f}, {128, 28.9f}};
+    } kPass[] = {{32, 16.0f}, {64, 17.4f}, {96, 23.4f}, {128, 28.5f}};
     uint32_t best = 128;
     float best_t = 1e30f;
     for (uint32_t chunks = (nz + 127) / 128; chunks <= (nz + 31) / 32; chunks++) {
-        const uint32_t ns = round_up((nz + chunks - 1) / chunks, 16);
+        uint32_t ns = std::max(32u, round_up((nz + chunks - 1) / chunks, 16));
+        if (ns > 64) ns = std::max(ns, 96u);  // as many columns as the shape's totals in registers
         float ms = kPass[3].ms;
         for (int i = 3; i >= 0; i--)
             if (ns <= kPass[i].ns) ms = kPass[i].ms;
@@ -736,8 +737,11 @@ ufob_status bp_umma_launch(const BPGeometry &g, const void *d_sino, uint32_t pit
     CUtensorMap map;
     UFOB_TRY(make_octet_map(&map, d_sino, g.W, g.P, (g.nz + 7) / 8, pitch, group_pitch, a.ns / 8));
     // two CTAs per SM while the accumulators and four angles' weights of both fit in tensor memory
-    if (a.ns <= 64) return launch<UmmaShape<4, 4, 2, 4>>(map, a, 64, stream);
-    return launch<UmmaShape<8, 3, 1, 12>>(map, a, 128, stream);
+    using Small = UmmaShape<4, 4, 2, 4>;
+    using Large = UmmaShape<8, 3, 1, 12>;
+    static_assert(MT * 32 >= 16 * Small::RC && MT * 96 >= 16 * Large::RC, "see bp_umma_slices");
+    if (a.ns <= 64) return launch<Small>(map, a, 64, stream);
+    return launch<Large>(map, a, 128, stream);
 }
 
 }  // namespace ufob

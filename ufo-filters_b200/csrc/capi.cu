@@ -555,7 +555,7 @@ static ufob_status bp_prepare(ufob_backproject *bp, uint32_t width, uint32_t hei
 
 // Whether a stack of FP16 sinograms runs on the tensor cores: the default form of the linear mode
 // (no compensated or half sums, no pinned tile), and enough slices.  A pass takes the same time for
-// any number of slices up to 32 (its weights): 16.2 ms at 2048^2 x 1500, against 7.3 / 10.7 / 15.7 /
+// any number of slices up to 32 (its weights): 16.0 ms at 2048^2 x 1500, against 7.3 / 10.7 / 15.7 /
 // 30 ms of the slice-quad kernel for up to 4 / 8 / 16 / 32 slices (721 x 1001^2: 2.0 against 1.92 for
 // 16), so it starts where that kernel would take its 32-slice tile.
 static constexpr uint32_t kUmmaMinSlices = 17;
@@ -897,6 +897,13 @@ extern "C" void ufob_stacked_bp_destroy(ufob_stacked_bp *sb)
     delete sb;
 }
 
+// Workspace of a group of slices on the tensor cores: octets and their flags.
+static ufob_status umma_workspace(ufob_fbp *x, uint32_t fw, uint32_t height, uint32_t nz)
+{
+    UFOB_TRY(x->work.ensure((size_t)fw * 16 * height * ((nz + 7) / 8)));
+    return x->flags.ensure(umma_flag_bytes(height, nz));
+}
+
 // Filter + backproject `nz` slices already on the device; logical row
 // slice * height + angle of `src` is sinogram row `angle` of slice `slice`.  `umma`: FP16 on the tensor
 // cores, as decided for the whole call.
@@ -915,10 +922,9 @@ static ufob_status fbp_group(ufob_fbp *x, const RowSource &src, uint32_t width, 
     const bool quads = x->storage == UFOB_F16 && nz > 1 && !umma;
     const bool pairs = x->storage == UFOB_BF16 || (x->storage == UFOB_F16 && nz == 1);
     const uint32_t pitch = umma ? fw : quads ? fw + 1 : pairs ? round_up(fw + 1, 4) : round_up(fw, 4);
-    const size_t work_bytes = umma    ? (size_t)pitch * 16 * height * ((nz + 7) / 8)
-                              : quads ? (size_t)pitch * 16 * height * ((nz + 3) / 4) : (size_t)pitch * 4 * height * nz;
-    UFOB_TRY(x->work.ensure(work_bytes));
-    if (umma) UFOB_TRY(x->flags.ensure(umma_flag_bytes(height, nz)));
+    const size_t work_bytes =
+        quads ? (size_t)pitch * 16 * height * ((nz + 3) / 4) : (size_t)pitch * 4 * height * nz;
+    UFOB_TRY(umma ? umma_workspace(x, fw, height, nz) : x->work.ensure(work_bytes));
     cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr;
     if (x->timing) {
         e0 = x->next_event();
@@ -1093,12 +1099,14 @@ extern "C" ufob_status ufob_fbp_run_host(ufob_fbp *x, const float *h_sino, uint3
         }
     }
     const bool umma = fbp_umma(x, width, height, chunk);
-    auto staging = [&](uint32_t slices) -> ufob_status {
+    uint32_t nfft, fw;
+    UFOB_TRY(filter_sizes(x->f->props, width, &nfft, &fw));
+    auto buffers = [&](uint32_t slices) -> ufob_status {
         for (int i = 0; i < (umma && nslices <= slices ? 1 : 2); i++) {  // (row chunks below have edges)
             UFOB_TRY(x->hin[i].ensure((size_t)slices * width * height * 4));
             UFOB_TRY(x->hout[i].ensure((size_t)slices * ow * oh * 4));
         }
-        return UFOB_OK;
+        return umma ? umma_workspace(x, fw, height, slices) : UFOB_OK;
     };
     if (umma && nslices % chunk && nslices % chunk < kUmmaMinSlices) {
         // a small last chunk would take as long as a whole one: share it among the others (up to 16 slices
@@ -1107,9 +1115,9 @@ extern "C" ufob_status ufob_fbp_run_host(ufob_fbp *x, const float *h_sino, uint3
         // in pairs, which keep their partners.
         const uint32_t n = nslices / chunk;
         const uint32_t larger = round_up((nslices + n - 1) / n, 2);
-        chunk = staging(larger) == UFOB_OK ? larger : round_up((nslices + n) / (n + 1), 2);
+        chunk = buffers(larger) == UFOB_OK ? larger : round_up((nslices + n) / (n + 1), 2);
     }
-    UFOB_TRY(staging(chunk));
+    UFOB_TRY(buffers(chunk));
     // Pipeline: H2D(c) on the upload stream -> filter+BP(c) on the compute stream -> D2H(c) on the download
     // stream, double-buffered so chunk c+1's upload and chunk c-1's download overlap chunk c's compute.
     // Chunk sizes: a short first chunk (compute starts after a small upload) and a short last one
