@@ -30,7 +30,7 @@
 //     builders add to totals in registers and shared memory.  The tensor cores cut an addition off at the
 //     accumulator's last bit: one sum over 1500 angles of rows in [1, 2) is 3.9e-5 too small, 6000 angles
 //     1.6e-4, with blocks 1.1e-6 for any number (the slice-quad kernel's error, rounding of the rows
-//     included, 4.6e-6 and 2.3e-6; this one's 4.3e-6 and 2.4e-6).  Costs 1.1 of 15.1 ms for 32 slices, 0.9 of
+//     included, 4.6e-6 and 2.3e-6; this one's 4.3e-6 and 2.4e-6).  Costs 0.9 of 15.1 ms for 32 slices, 0.6 of
 //     16.8 for 64; blocks of 32 angles 0.5 to 1 ms more, of 128 a bias of 2.2e-6.
 //
 // Roles of a CTA: four builder warps, a producer warp (one TMA per angle), an MMA warp per

@@ -1005,17 +1005,11 @@ extern "C" ufob_status ufob_fbp_kernel_times(ufob_fbp *x, double *filter_ms, uin
     return UFOB_OK;
 }
 
-// Slices whose octets fit 2 GiB.
-static uint64_t octet_slices(uint32_t width, uint32_t height)
-{
-    return (2ull << 30) / std::max<uint64_t>((uint64_t)(width + 4) * 2 * height, 1);
-}
-
 // Whether a call's FP16 slices run on the tensor cores.  Decided once per call and not per group, so that
 // a remainder has the values it would have in another grouping.
-static bool fbp_umma(const ufob_fbp *x, uint32_t width, uint32_t height, uint32_t nslices)
+static bool fbp_umma(const ufob_fbp *x, uint32_t nslices)
 {
-    return x->storage == UFOB_F16 && umma_applies(x->bp->props, nslices) && octet_slices(width, height) >= 16;
+    return x->storage == UFOB_F16 && umma_applies(x->bp->props, nslices);
 }
 
 static uint32_t group_slices(uint32_t width, uint32_t height, uint32_t nslices, bool umma)
@@ -1027,9 +1021,9 @@ static uint32_t group_slices(uint32_t width, uint32_t height, uint32_t nslices, 
     g = g >= 32 ? g / 32 * 32 : std::max<uint64_t>(8, g / 8 * 8);
     if (umma) {
         // slice octets take 2 bytes a value, and the tensor-core kernel up to 128 slices per CTA in shares
-        // of about 32
-        const uint64_t g2 = octet_slices(width, height);
-        g = g2 >= 128 ? g2 / 128 * 128 : g2 >= 32 ? g2 / 32 * 32 : g2 / 8 * 8;
+        // of about 32; 16 very large slices take what 8 do as quad cells
+        const uint64_t g2 = (2ull << 30) / std::max<uint64_t>((uint64_t)(width + 4) * 2 * height, 1);
+        g = g2 >= 128 ? g2 / 128 * 128 : g2 >= 32 ? g2 / 32 * 32 : std::max<uint64_t>(16, g2 / 8 * 8);
     }
     return (uint32_t)std::min<uint64_t>(g, nslices);
 }
@@ -1042,7 +1036,7 @@ extern "C" ufob_status ufob_fbp_run(ufob_fbp *x, const float *d_sino, uint32_t w
     uint32_t ow, oh;
     UFOB_TRY(ufob_fbp_get_requisition(x, width, height, &ow, &oh));
     cudaStream_t s = (cudaStream_t)stream;
-    const bool umma = fbp_umma(x, width, height, nslices);
+    const bool umma = fbp_umma(x, nslices);
     const uint32_t G = group_slices(width, height, nslices, umma);
     for (uint32_t z = 0; z < nslices; z += G) {
         const uint32_t nz = std::min(G, nslices - z);
@@ -1065,7 +1059,7 @@ extern "C" ufob_status ufob_fbp_run_projections(ufob_fbp *x, const ufob_preproce
     cudaStream_t s = (cudaStream_t)stream;
     // every slice group reads the same projections: a cone weight restarts at its count each time
     const uint32_t count0 = pre && pre->cone ? ufob_cone_weight_get_count(pre->cone) : 0;
-    const bool umma = fbp_umma(x, width, n_projections, n_rows);
+    const bool umma = fbp_umma(x, n_rows);
     const uint32_t G = group_slices(width, n_projections, n_rows, umma);
     for (uint32_t z = 0; z < n_rows; z += G) {
         const uint32_t nz = std::min(G, n_rows - z);
@@ -1098,7 +1092,7 @@ extern "C" ufob_status ufob_fbp_run_host(ufob_fbp *x, const float *h_sino, uint3
             UFOB_CUDA_TRY(cudaEventCreateWithFlags(&x->ev_out[i], cudaEventDisableTiming));
         }
     }
-    const bool umma = fbp_umma(x, width, height, chunk);
+    const bool umma = fbp_umma(x, chunk);
     uint32_t nfft, fw;
     UFOB_TRY(filter_sizes(x->f->props, width, &nfft, &fw));
     auto buffers = [&](uint32_t slices) -> ufob_status {
