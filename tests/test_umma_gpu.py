@@ -62,7 +62,7 @@ def test_angle_counts(cuda, nz, P):
 # blocks of 64 angles whose sums are added to the totals: block ends, for either split of the totals
 # between registers and shared memory (up to 32, 64, 96 and 128 slices)
 @pytest.mark.parametrize("nz", [17, 33, 65, 128])
-@pytest.mark.parametrize("P", [63, 64, 65, 127, 128, 129, 200])
+@pytest.mark.parametrize("P", [63, 64, 65, 95, 96, 97, 127, 128, 129, 160, 161, 200, 320])
 def test_angle_blocks(cuda, nz, P):
     raw = _raw(nz, P, 40, P)
     got, ref = _fbp(raw, 64), _ref(raw, 64)

@@ -30,8 +30,10 @@
 //     builders add to totals in registers and shared memory.  The tensor cores cut an addition off at the
 //     accumulator's last bit: one sum over 1500 angles of rows in [1, 2) is 3.9e-5 too small, 6000 angles
 //     1.6e-4, with blocks 1.1e-6 for any number (the slice-quad kernel's error, rounding of the rows
-//     included, 4.6e-6 and 2.3e-6; this one's 4.3e-6 and 2.4e-6).  Costs 0.9 of 15.1 ms for 32 slices, 0.6 of
-//     16.8 for 64; blocks of 32 angles 0.5 to 1 ms more, of 128 a bias of 2.2e-6.
+//     included, 4.6e-6 and 2.3e-6; this one's 4.3e-6 and 2.4e-6).  Up to 32 slices the blocks
+//     use two sets of accumulators in turn, so nobody waits for the adding (one set: 16.0 against
+//     15.7 ms).  Costs 0.6 of 15.1 ms for 32 slices, 0.7 of 16.8 for 64; blocks of 32 angles 0.5 to 1 ms
+//     more, of 128 a bias of 2.2e-6.
 //
 // Roles of a CTA: four builder warps, a producer warp (one TMA per angle), an MMA warp per
 // accumulator (the issuing lane's instructions, not the tensor pipe, limit one warp for both: 29
@@ -39,8 +41,8 @@
 // arrive on one barrier that frees its weights and its windows.  What bounds it is the fixed cost
 // of a stage (barriers, issue latencies), so up to 64 slices two CTAs share an SM (KA = 4); above,
 // tensor memory holds one CTA, whose stages are longer (KA = 8) and whose totals are mostly registers.
-// 2048^2 x 1500 angles, ms per pass: ns <= 32 16.0, 64 17.4, 96 23.4, 128 28.5 (12.6, 23.1, 25.8,
-// 28.3 TGUPS; slice quads 6.6).  Four CTAs per SM with KA = 2 up to 32 slices: 16.2 (2% faster without the
+// 2048^2 x 1500 angles, ms per pass: ns <= 32 15.7, 64 17.5, 96 23.7, 128 28.4 (12.8, 23.0, 25.5,
+// 28.4 TGUPS; slice quads 6.6).  Four CTAs per SM with KA = 2 up to 32 slices: 16.2 (2% faster without the
 // totals, which then are all in shared memory); two with KA = 2 for 96: 26.4.
 //
 // A non-finite value of a window would reach every pixel of its tile (0 * inf).  The filter flags
@@ -131,6 +133,7 @@ struct UmmaArgs {
     uint64_t plane;  // output floats between slices
     int *err;
     uint32_t tiles_x, tiles_y, tmem_cols;
+    uint32_t sets;  // of accumulators, used in turn by the blocks of angles
     uint32_t one;  // 1, not known to the compiler: keeps the weights' sums off the busier ALU pipe
 };
 
@@ -391,13 +394,17 @@ __global__ void __launch_bounds__(kThreads, Sh::CTAS)
     float4 *totals = reinterpret_cast<float4 *>(gbase + SB * KA * bbytes) + row;
     float tot[RC > 0 ? 16 * RC : 1];
     const uint32_t tlane = tmem + ((uint32_t)(warp & 3) << 21);
-    // adds the accumulators' sums, whose products are done, and lets the next block's begin
-    auto add_block = [&](bool first) {
+    // (one CTA's tensor memory has no room for two sets)
+    const uint32_t sets = Sh::CTAS > 1 ? args.sets : 1, set_cols = MT * args.ns;
+    // adds the sums of block b, whose products are done, and lets a later block's begin in their place
+    auto add_block = [&](uint32_t b) {
+        const bool first = b == 0;
+        const uint32_t tcol = tlane + (b % sets) * set_cols;
         tc_fence_after();
         uint32_t r[16];
 #pragma unroll
         for (int q = 0; q < RC; q++) {
-            tmem_ld16(tlane + 16 * q, r);
+            tmem_ld16(tcol + 16 * q, r);
             tmem_wait16(r);
 #pragma unroll
             for (int i = 0; i < 16; i++) tot[16 * q + i] = __uint_as_float(r[i]) + (first ? 0.0f : tot[16 * q + i]);
@@ -405,7 +412,7 @@ __global__ void __launch_bounds__(kThreads, Sh::CTAS)
 #pragma unroll 1
         for (uint32_t q = RC; q < chunks; q++) {
             float4 *t = totals + (q - RC) * 4 * (MX * MY), v[4];
-            tmem_ld16(tlane + 16 * q, r);
+            tmem_ld16(tcol + 16 * q, r);
 #pragma unroll
             for (int i = 0; i < 4; i++)
                 v[i] = first || row >= MX * MY ? make_float4(0.f, 0.f, 0.f, 0.f) : t[i * (MX * MY)];
@@ -425,18 +432,21 @@ __global__ void __launch_bounds__(kThreads, Sh::CTAS)
 
     if (warp < kBuildWarps) {
         const float kFix = 6144.0f;  // 1.5 * 2^12: 11 fractional bits left in the mantissa
-        const uint32_t ta = tmem + MT * args.ns + ((uint32_t)warp << 21);
+        const uint32_t ta = tmem + sets * set_cols + ((uint32_t)warp << 21);
+        uint32_t added_blocks = 0;
         const uint32_t one = args.one;
         float4 *tab = s_tab[warp];
         bool ok = true;
         for (uint32_t p0 = 0; p0 < P && ok; p0 += 32) {
-            if (p0 && p0 % kBlock == 0) {
-                // the sums of the block that ended with the group before, once its products are done
-                const uint32_t prev = p0 / KA - 1;
-                ok = wait_or_abort(&empty[prev % SB], (prev / SB) & 1u, abort_flag);
+            // the sums of a block once its products are done: with one set of accumulators at its end, with
+            // two half a block later, when there is nothing to wait for
+            const uint32_t late = (sets - 1) * (kBlock / 2);
+            if (p0 >= kBlock && p0 % kBlock == late) {
+                const uint32_t prev = (p0 - late) / KA - 1;  // its last stage
+                ok = late != 0 || wait_or_abort(&empty[prev % SB], (prev / SB) & 1u, abort_flag);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
-                add_block(p0 == kBlock);
+                add_block(added_blocks++);
             }
             {
                 const float2 sc = __ldg(&args.sincos[min(p0 + lane, P - 1)]);
@@ -484,14 +494,19 @@ __global__ void __launch_bounds__(kThreads, Sh::CTAS)
                 if (lane == 0) mbar_arrive(&full_a[s]);
             }
         }
+        // a block before a last one too short for that: with all products done
+        if (ok && (added_blocks + 1) * kBlock < P) {
+            ok = wait_or_abort(&done, 0, abort_flag);
+            if (__all_sync(0xffffffffu, ok)) add_block(added_blocks);
+        }
     } else {
         const bool produce = warp == kBuildWarps;
         const int m = warp - kBuildWarps - 1;  // accumulator of an MMA warp
         // D = F32, A = B = F16, B N-major
         const uint32_t idesc = (1u << 4) | (1u << 16) | ((args.ns >> 3) << 17) | ((128u >> 4) << 24);
         const uint64_t desc0 = plain_desc(base, 128, KW * 16);
-        const uint32_t dcol = tmem + (uint32_t)m * args.ns;
-        const uint32_t acol = tmem + MT * args.ns + (uint32_t)m * (KT / 2);
+        uint32_t dcol = tmem + (uint32_t)m * args.ns;
+        const uint32_t acol = tmem + sets * set_cols + (uint32_t)m * (KT / 2);
         uint32_t acc = 0;
         bool ok = true;
         for (uint32_t p0 = 0; p0 < P; p0 += 32) {
@@ -510,9 +525,11 @@ __global__ void __launch_bounds__(kThreads, Sh::CTAS)
             }
             const uint32_t n = min(32u, P - p0);
             if (!produce && p0 % kBlock == 0) {
-                // a block's first products overwrite the sums of the one before, once these are added
+                // a block's first products overwrite the sums of an earlier one, once these are added
+                const uint32_t b = p0 / kBlock;
                 acc = 0;
-                if (p0 && lane == 0) ok = wait_or_abort(&added, (p0 / kBlock - 1) & 1u, abort_flag);
+                dcol = tmem + (b % sets) * set_cols + (uint32_t)m * args.ns;
+                if (b >= sets && lane == 0) ok = wait_or_abort(&added, (b - sets) & 1u, abort_flag);
             }
             if (lane == 0 && ok) {
                 for (uint32_t j = 0; j < n; j += KA) {
@@ -569,13 +586,14 @@ __global__ void __launch_bounds__(kThreads, Sh::CTAS)
             const size_t plane = args.plane;
             const uint32_t nz = min(args.ns, args.nz - z0);
             const bool added_some = P > kBlock;
+            const uint32_t tlast = tlane + ((P - 1) / kBlock % sets) * set_cols;
             // chunk q, with the totals so far in v
             auto store = [&](uint32_t q, float (&v)[16]) {
                 const uint32_t h = 16 * q >= args.ns, c = 16 * q - h * args.ns;
                 const int y = py + (int)h * MY;
                 if (c >= nz) return;
                 uint32_t r[16];
-                tmem_ld16(tlane + 16 * q, r);
+                tmem_ld16(tlast + 16 * q, r);
                 tmem_wait16(r);
                 if (row < MX * MY && px < (int)args.roi_w && y < (int)args.roi_h) {
                     float *o = args.out + (size_t)(z0 + c) * plane + (size_t)y * args.roi_w + px;
@@ -646,8 +664,11 @@ ufob_status make_octet_map(CUtensorMap *map, const void *base, uint32_t W, uint3
 template <typename Sh>
 ufob_status launch(const CUtensorMap &map, UmmaArgs a, uint32_t most_slices, cudaStream_t stream)
 {
+    // two sets of accumulators where that does not cost tensor memory for another CTA
+    const uint32_t cols = MT * a.ns + Sh::kACols;
     a.tmem_cols = 32;
-    while (a.tmem_cols < MT * a.ns + Sh::kACols) a.tmem_cols *= 2;
+    while (a.tmem_cols < cols) a.tmem_cols *= 2;
+    a.sets = Sh::CTAS > 1 && cols + MT * a.ns <= a.tmem_cols ? 2 : 1;
     static std::atomic<uint64_t> attr_devs{0};
     UFOB_CUDA_TRY(smem_limit_per_device(k_bp_umma<Sh>, (int)Sh::smem(most_slices), attr_devs));
     dim3 grid(a.tiles_x * a.tiles_y, (a.nz + a.ns - 1) / a.ns);
@@ -666,7 +687,7 @@ uint32_t bp_umma_slices(uint32_t nz)
     static const struct {
         uint32_t ns;
         float ms;
-    } kPass[] = {{32, 16.0f}, {64, 17.4f}, {96, 23.4f}, {128, 28.5f}};
+    } kPass[] = {{32, 15.7f}, {64, 17.5f}, {96, 23.7f}, {128, 28.4f}};
     uint32_t best = 128;
     float best_t = 1e30f;
     for (uint32_t chunks = (nz + 127) / 128; chunks <= (nz + 31) / 32; chunks++) {

@@ -555,7 +555,7 @@ static ufob_status bp_prepare(ufob_backproject *bp, uint32_t width, uint32_t hei
 
 // Whether a stack of FP16 sinograms runs on the tensor cores: the default form of the linear mode
 // (no compensated or half sums, no pinned tile), and enough slices.  A pass takes the same time for
-// any number of slices up to 32 (its weights): 16.0 ms at 2048^2 x 1500, against 7.3 / 10.7 / 15.7 /
+// any number of slices up to 32 (its weights): 15.7 ms at 2048^2 x 1500, against 7.3 / 10.7 / 15.7 /
 // 30 ms of the slice-quad kernel for up to 4 / 8 / 16 / 32 slices (721 x 1001^2: 2.0 against 1.92 for
 // 16), so it starts where that kernel would take its 32-slice tile.
 static constexpr uint32_t kUmmaMinSlices = 17;
